@@ -421,6 +421,22 @@ int32_t ojx_e8t_gemm_lowbit(int32_t bits, const void* x, int32_t x_dtype, int64_
                             void* workspace, size_t workspace_bytes, void* stream);
 
 /*
+ * The packed linear of any format and any batch: y[M, N] = x[M, K] . W^T (+ bias), routed to the decode-shape kernels or the
+ * tcgen05 kernel by the library's own rule.  `format`: 0 ternary (1.5 bits), 2 or 1 the sibling formats.  Scratch:
+ * ojx_e8t_linear_workspace_bytes(...) bytes, 256-byte aligned (0 bytes: none needed); its contents never have to be
+ * initialised and may be reused once the call's kernels have finished.  `flags`: 0, or OJX_LINEAR_DECODE / OJX_LINEAR_GEMM to
+ * force a route (tests).
+ */
+#define OJX_LINEAR_DECODE 1
+#define OJX_LINEAR_GEMM   2
+size_t  ojx_e8t_linear_workspace_bytes(int32_t format, int32_t x_dtype, int64_t M, int64_t N, int64_t K, int32_t group, int32_t flags);
+int32_t ojx_e8t_linear(int32_t format, const void* x, int32_t x_dtype, int64_t M,
+                       const uint8_t* packed, const uint16_t* scales, const void* bias,
+                       int64_t N, int64_t K, int32_t group,
+                       void* y, int32_t y_dtype,
+                       void* workspace, size_t workspace_bytes, int32_t flags, void* stream);
+
+/*
  * Backward of the packed linear with respect to its input: dX[M, K] = dY[M, N] . W[N, K], W given packed, on the
  * same tcgen05 pipeline (the contraction runs over the weight rows; the decoded weights enter the MMAs as an
  * MN-major operand, so no dense or transposed copy of W ever exists).  Replaces the decode-then-matmul of

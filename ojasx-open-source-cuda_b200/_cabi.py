@@ -8,6 +8,8 @@ a ``RuntimeError`` carrying the status name is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import shutil
 import subprocess
@@ -18,11 +20,13 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libojx_e8t.so")
+GLUE_PATH = os.path.join(LIB_DIR, "_ojx_torch.so")       # CPython extension: the hot entry points on torch tensors
 
 OJX_F32, OJX_F16, OJX_BF16 = 0, 1, 2
 OJX_GEMV_STATIC_WEIGHTS, OJX_GEMV_SIGNAL_PEERS, OJX_GEMV_WAIT_PEERS, OJX_GEMV_TEST_LOSE_COPY = 1, 2, 4, 8
 OJX_GEMV_INDEPENDENT = 16
 OJX_ENCODE_HADAMARD = 1
+OJX_LINEAR_DECODE, OJX_LINEAR_GEMM = 1, 2
 PEER_SYNC_BYTES = 48        # sizeof(ojx_e8t_peer_sync): epoch, arrived, status, spin_limit, flag[8]
 
 EXPORTED_SYMBOLS = (
@@ -30,7 +34,7 @@ EXPORTED_SYMBOLS = (
     "ojx_e8t_gemv_workspace_bytes", "ojx_e8t_gemv", "ojx_e8t_gemv_lora", "ojx_e8t_gemv_tiles", "ojx_e8t_gemv_kchunks",
     "ojx_e8t_gemv_grouped", "ojx_e8t_gemv_grouped_peers", "ojx_e8t_gemv_grouped_ex", "ojx_e8t_peer_wait", "ojx_e8t_enable_peer_access", "ojx_e8t_gemm_workspace_bytes", "ojx_e8t_gemm", "ojx_e8t_gemm_lowbit", "ojx_e8t_gemm_status", "ojx_e8t_gemm_dx", "ojx_e8t_gemm_dx_lowbit", "ojx_e8t_gemm_dx_workspace_bytes",
     "ojx_e8t_generate", "ojx_e8t_last_cuda_error", "ojx_e8t_device_status", "ojx_e8t_poll_status", "ojx_e8t_set_wait_limit",
-    "ojx_e8t_gemv_static_scratch", "ojx_e8t_gemv_static_scratch_capacity",
+    "ojx_e8t_gemv_static_scratch", "ojx_e8t_gemv_static_scratch_capacity", "ojx_e8t_linear", "ojx_e8t_linear_workspace_bytes",
 )
 
 NVCC_FLAGS = [
@@ -51,30 +55,52 @@ def sources():
         os.path.join(os.path.dirname(HERE), "include", "ojx_e8t.h")]
 
 
+def _stale(path: str, srcs) -> bool:
+    return not os.path.exists(path) or any(os.path.getmtime(f) > os.path.getmtime(path) for f in srcs)
+
+
 def needs_build() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    built = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(s) > built for s in sources())
+    return _stale(LIB_PATH, sources())
+
+
+def _compile(cmd, out: str) -> str:
+    tmp = out + ".tmp.%d" % os.getpid()
+    proc = subprocess.run(cmd + ["-o", tmp], capture_output=True, text=True)
+    if proc.returncode != 0:
+        raise RuntimeError(f"{cmd[0]} failed:\n" + proc.stdout + proc.stderr)
+    os.replace(tmp, out)
+    return proc.stderr
+
+
+def _build_glue() -> None:
+    """``csrc/torch_glue.cpp`` -> ``lib/_ojx_torch.so`` against the installed torch's headers and libraries."""
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"))
+    includes = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+                sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    _compile(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
+              f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f"-I{d}" for d in includes] +
+             [os.path.join(CSRC, "torch_glue.cpp"), f"-L{os.path.join(root, 'lib')}", f"-L{LIB_DIR}", "-l:libojx_e8t.so",
+              "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], GLUE_PATH)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile ``csrc/ojx_e8t.cu`` for sm_100a into ``lib/libojx_e8t.so`` (nvcc cross-compiles
-    without a GPU).  Returns the library path."""
-    if not force and not needs_build():
-        return LIB_PATH
-    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
-    if not os.path.exists(nvcc):
-        raise RuntimeError("nvcc not found: cannot build libojx_e8t.so")
-    os.makedirs(LIB_DIR, exist_ok=True)
-    tmp = LIB_PATH + ".tmp.%d" % os.getpid()
-    cmd = [nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", tmp, os.path.join(CSRC, "ojx_e8t.cu")]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if proc.returncode != 0:
-        raise RuntimeError("nvcc failed:\n" + proc.stdout + proc.stderr)
-    os.replace(tmp, LIB_PATH)
-    if verbose:
-        print(proc.stderr)
+    """Compile ``csrc/ojx_e8t.cu`` for sm_100a into ``lib/libojx_e8t.so`` (nvcc cross-compiles without a GPU) and the
+    torch module beside it.  Returns the library path."""
+    if force or needs_build():
+        nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+        if not os.path.exists(nvcc):
+            raise RuntimeError("nvcc not found: cannot build libojx_e8t.so")
+        os.makedirs(LIB_DIR, exist_ok=True)
+        log = _compile([nvcc] + NVCC_FLAGS + (["-Xptxas", "-v"] if verbose else []) + [os.path.join(CSRC, "ojx_e8t.cu")], LIB_PATH)
+        if verbose:
+            print(log)
+    header = os.path.join(os.path.dirname(HERE), "include", "ojx_e8t.h")
+    if force or _stale(GLUE_PATH, [os.path.join(CSRC, "torch_glue.cpp"), header]):
+        _build_glue()
     return LIB_PATH
 
 
@@ -156,6 +182,10 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.ojx_e8t_gemm_dx.argtypes = [vp, i32, i64, vp, vp, i64, i64, i32, vp, i32, vp, sz, vp]
     lib.ojx_e8t_gemm_dx_lowbit.restype = i32
     lib.ojx_e8t_gemm_dx_lowbit.argtypes = [i32] + [vp, i32, i64, vp, vp, i64, i64, i32, vp, i32, vp, sz, vp]
+    lib.ojx_e8t_linear_workspace_bytes.restype = sz
+    lib.ojx_e8t_linear_workspace_bytes.argtypes = [i32, i32, i64, i64, i64, i32, i32]
+    lib.ojx_e8t_linear.restype = i32
+    lib.ojx_e8t_linear.argtypes = [i32, vp, i32, i64, vp, vp, vp, i64, i64, i32, vp, i32, vp, sz, i32, vp]
     lib.ojx_e8t_gemm_status.restype = i32
     lib.ojx_e8t_gemm_status.argtypes = [vp, vp]
     lib.ojx_e8t_last_cuda_error.restype = ctypes.c_char_p
@@ -186,6 +216,24 @@ def lib() -> ctypes.CDLL:
     return _lib
 
 
+_glue = None
+
+
+def glue():
+    """The torch extension module (see ``csrc/torch_glue.cpp``); raises if it has not been built."""
+    global _glue
+    if _glue is None:
+        lib()                                            # the library it links against, with its own error message
+        import torch                                     # noqa: F401  (its libraries have to be loaded first)
+        if not os.path.exists(GLUE_PATH):
+            raise RuntimeError(f"{GLUE_PATH} is missing. Build it with this module's build().")
+        loader = importlib.machinery.ExtensionFileLoader("_ojx_torch", GLUE_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ojx_torch", loader))
+        loader.exec_module(module)
+        _glue = module
+    return _glue
+
+
 def status_name(code: int) -> str:
     return lib().ojx_e8t_status_string(int(code)).decode()
 
@@ -194,10 +242,16 @@ def raise_pending() -> None:
     """Raises if a kernel launched earlier ran into the limit of one of its bounded waits (read from the library's
     pinned status word: no synchronisation).  Called by the wrappers at the start of every decode-shape call."""
     if lib().ojx_e8t_poll_status() != 0:
-        raise OjxError("an earlier launch gave up on a bounded device-side wait (OJX_ERR_TIMEOUT): its outputs are invalid")
+        _raise_pending()
+
+
+def _raise_pending() -> None:
+    raise OjxError("an earlier launch gave up on a bounded device-side wait (OJX_ERR_TIMEOUT): its outputs are invalid")
 
 
 def check(code: int, what: str) -> None:
+    if code == 1:                                        # torch_glue: a failure of an earlier launch is pending
+        _raise_pending()
     if code != 0:
         detail = ""
         if code == -6:

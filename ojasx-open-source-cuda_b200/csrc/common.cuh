@@ -115,7 +115,7 @@ static __device__ int g_device_status = 0;
 // library image, pinned and mapped on first use, into which a kernel that gave up on a wait writes its code.
 // Kernels receive its device address as an argument (null when the mapping failed: then only
 // g_device_status is written).
-int* host_status_device_ptr();
+int* host_status_device_ptr(cudaStream_t stream);
 int  host_status_take();                       // returns the recorded code (0: none) and clears it
 uint32_t& wait_limit_override();               // 0: the built-in limit; set by ojx_e8t_set_wait_limit (tests)
 

@@ -58,6 +58,8 @@ struct GemmParams {
     const void* bias;
     void* y;
     int32_t* status;
+    int* host_status;              // mapped host word for the same event (may be null)
+    int clear_status;              // this launch clears the status word (no wait can have given up yet)
     int M, N, K;
     int y_stride;                  // elements between consecutive token rows of y (N of the whole matrix)
     int tile_limit;                // process only the first tile_limit tiles of the enumeration
@@ -73,16 +75,15 @@ struct GemmParams {
 // takes one token row, finds its largest magnitude, then writes the row as fp16 scaled by the power of two
 // that brings that magnitude into [2^14, 2^15), and the inverse factor for the epilogue.  Rows of up to
 // TPR * 8 * VECS elements stay in registers between the two steps (one global read); longer rows are read
-// twice.  The first thread also clears the status word the GEMM kernel reports through.
+// twice.
 template <int TPR, int VECS>
 __global__ void __launch_bounds__(256) normalize_rows_bf16_to_f16_kernel(const __nv_bfloat16* __restrict__ x,
                                                                           __half* __restrict__ out, float* __restrict__ up,
-                                                                          int64_t M, int64_t K, int32_t* __restrict__ status) {
+                                                                          int64_t M, int64_t K) {
     __shared__ uint32_t warp_max[8];
     constexpr int kRowsPerCta = 256 / TPR;
     const int t = threadIdx.x % TPR;
     const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + threadIdx.x / TPR;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && status != nullptr) *status = 0;
     const bool live = row < M;                                            // whole warps share `live`
     const uint4* src = reinterpret_cast<const uint4*>(x + (live ? row : 0) * K);   // K % 256 == 0: rows are 16-byte aligned
     uint4* dst = reinterpret_cast<uint4*>(out + (live ? row : 0) * K);
@@ -352,6 +353,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             mbar_init(tempty_bar(a), 4);            // one arrive per epilogue warp
         }
         *abort_flag = 0;
+        if (p.clear_status && blockIdx.x == 0) *p.status = 0;      // a wait gives up millions of polls later
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 13) {
@@ -683,7 +685,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
 
     tc_fence_before();
     __syncthreads();
-    if (tid == 0 && *abort_flag != 0 && p.status != nullptr) atomicCAS(p.status, 0, *abort_flag);
+    if (tid == 0 && *abort_flag != 0) {
+        if (p.status != nullptr) atomicCAS(p.status, 0, *abort_flag);
+        atomicCAS(&g_device_status, 0, *abort_flag);
+        if (p.host_status != nullptr) *reinterpret_cast<volatile int*>(p.host_status) = *abort_flag;
+    }
     if (warp == 13) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem_base) : "memory");
@@ -784,13 +790,11 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
     if (convert) {
         if (K <= 4096)
             normalize_rows_bf16_to_f16_kernel<32, 16><<<(unsigned)((M + 7) / 8), 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K, static_cast<int32_t*>(workspace));
+                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K);
         else
             normalize_rows_bf16_to_f16_kernel<256, 8><<<(unsigned)M, 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K, static_cast<int32_t*>(workspace));
+                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K);
         if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
-    } else if (cudaMemsetAsync(workspace, 0, 4, s) != cudaSuccess) {
-        return OJX_ERR_LAUNCH;
     }
 
     // One launch over the rectangle of weight rows [n0, N) x tokens [m0, M) of the problem, in tiles of
@@ -813,6 +817,8 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
         prm.bias = bias ? static_cast<const uint8_t*>(bias) + (size_t)n0 * dtype_size(x_dtype) : nullptr;
         prm.y = static_cast<uint8_t*>(y) + ((size_t)m0 * (size_t)N + (size_t)n0) * dtype_size(y_dtype);
         prm.status = static_cast<int32_t*>(workspace);
+        prm.host_status = host_status_device_ptr(s);
+        prm.clear_status = (n0 == 0 && m0 == 0) ? 1 : 0;
         prm.M = (int)Ms; prm.N = (int)Ns; prm.K = (int)K;
         prm.y_stride = (int)N;
         prm.y_dtype = y_dtype; prm.bias_dtype = x_dtype;
@@ -905,13 +911,11 @@ int32_t gemm_dx_fmt_impl(int fmt, const void* gy, int gy_dtype, int64_t M, const
         // per-token power-of-two factors exactly as in the forward launch; rows here are N long (any multiple of 8)
         if (N <= 4096)
             normalize_rows_bf16_to_f16_kernel<32, 16><<<(unsigned)((M + 7) / 8), 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N, static_cast<int32_t*>(workspace));
+                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N);
         else
             normalize_rows_bf16_to_f16_kernel<256, 8><<<(unsigned)M, 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N, static_cast<int32_t*>(workspace));
+                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N);
         if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
-    } else if (cudaMemsetAsync(workspace, 0, 4, s) != cudaSuccess) {
-        return OJX_ERR_LAUNCH;
     }
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
@@ -925,6 +929,8 @@ int32_t gemm_dx_fmt_impl(int fmt, const void* gy, int gy_dtype, int64_t M, const
     prm.packed = packed; prm.scales = scales; prm.bias = nullptr;
     prm.y = dx;
     prm.status = static_cast<int32_t*>(workspace);
+    prm.host_status = host_status_device_ptr(s);
+    prm.clear_status = 1;
     prm.M = (int)M;
     prm.N = (int)K;                    // roles swapped: the output's feature dimension is the weight columns ...
     prm.K = (int)N;                    // ... and the contraction runs over the weight rows

@@ -70,7 +70,7 @@ template <int NB, bool kXF16, bool kI8 = false>
 static int32_t launch_gemv_a16(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count, int total,
                                int M, int y_dtype, const PeerMap& peers_in, int overlap, cudaStream_t s) {
     PeerMap peers = peers_in;
-    peers.host_status = host_status_device_ptr();
+    peers.host_status = host_status_device_ptr(s);
     peers.wait_limit = wait_limit_override() != 0 ? wait_limit_override() : kSpinLimit;
     static std::atomic<uint64_t> configured{0};
     using Cfg = A16Cfg<NB>;
@@ -148,7 +148,7 @@ int32_t peer_wait_impl(ojx_e8t_peer_sync* peer_sync, int world, cudaStream_t s) 
     peers.world = world;
     peers.sync = peer_sync;
     peers.mode = OJX_GEMV_WAIT_PEERS;
-    peers.host_status = host_status_device_ptr();
+    peers.host_status = host_status_device_ptr(s);
     peer_wait_kernel<<<1, 32, 0, s>>>(peers);
     return launch_status();
 }

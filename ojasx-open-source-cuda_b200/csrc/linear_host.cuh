@@ -1,0 +1,52 @@
+// One entry for the packed linear of every format: which kernel serves a call is decided here, once, for the C ABI, the
+// torch module (torch_glue.cpp) and the ctypes wrappers alike.
+#pragma once
+
+#include "gemv_host.cuh"
+#include "gemm_tcgen05.cuh"
+
+namespace ojx {
+
+constexpr int kForceDecode = 1, kForceGemm = 2;        // flags of ojx_e8t_linear (tests)
+
+// Batches of tokens run the tcgen05 kernel, decode shapes the GEMV kernels.  Where the line lies (14336 x 4096):
+//   * ternary, groups of 32: the decode kernel takes up to 16 rows (its two column blocks);
+//   * ternary, groups of 16: no tensor-core decode kernel, the shared-memory fp32 kernel wins for one or two rows only
+//     (35 against 54 us at one row, 82 against 54 us at four);
+//   * 2.0 / 1.0 bits: groups of 32 with K % 2048 == 0 have int8 decode kernels for up to eight rows; elsewhere the fp32
+//     decode kernel loses from four rows on (59 against 50 us at four rows, groups of 8).
+inline bool linear_uses_gemm(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, bool aligned, int flags) {
+    if (flags & kForceDecode) return false;
+    const bool able = (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && K % 256 == 0 && aligned &&
+                      (group == 32 || group == 16 || (fmt != 0 && group == 8));
+    if (flags & kForceGemm) return true;               // the kernel's own checks report what it cannot take
+    if (!able) return false;
+    if (fmt == 0) return M > 16 || (group == 16 && M > 2);
+    const bool decode_tc = group == 32 && K % 2048 == 0;
+    return M > 8 || (M >= 4 && !decode_tc);
+}
+
+inline int linear_group(int fmt, int group) { return fmt == 0 ? effective_group(group) : group; }
+
+size_t linear_workspace_bytes_impl(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, int flags) {
+    group = linear_group(fmt, group);
+    if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, true, flags))
+        return x_dtype == OJX_BF16 ? gemm_workspace_bytes_impl(M, N, K) : 256;
+    return fmt == 0 ? gemv_workspace_bytes_impl(M, N, K) : 0;
+}
+
+int32_t linear_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
+                    const void* bias, int64_t N, int64_t K, int group, void* y, int y_dtype, void* ws, size_t ws_bytes,
+                    int flags, cudaStream_t s) {
+    OJX_RETURN_IF(fmt != 0 && fmt != 1 && fmt != 2, OJX_ERR_UNSUPPORTED);
+    OJX_RETURN_IF((flags & ~(kForceDecode | kForceGemm)) != 0, OJX_ERR_UNSUPPORTED);
+    group = linear_group(fmt, group);
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) |
+                           reinterpret_cast<uintptr_t>(scales)) & 15) == 0;
+    if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, aligned, flags))
+        return gemm_fmt_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, ws, ws_bytes, s);
+    if (fmt == 0) return gemv_impl(x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, ws, ws_bytes, s);
+    return linear_lowbit_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, s, nullptr, nullptr, 0);
+}
+
+}  // namespace ojx

@@ -1,5 +1,6 @@
 // The whole library is this one translation unit: C ABI entry points (declared in
 // include/ojx_e8t.h) in front of the kernel files included below.  Built for sm_100a only.
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -11,6 +12,7 @@
 #include "gemv_a16.cuh"
 #include "gemv_host.cuh"
 #include "gemm_tcgen05.cuh"
+#include "linear_host.cuh"
 
 namespace ojx {
 
@@ -29,15 +31,21 @@ int check_arch() {
 
 alignas(4096) static volatile int g_host_status_page[1024];
 
-int* host_status_device_ptr() {
-    static std::once_flag once;
-    static bool registered = false;
-    std::call_once(once, [] {
-        const cudaError_t e = cudaHostRegister(const_cast<int*>(g_host_status_page), sizeof(g_host_status_page), cudaHostRegisterMapped);
-        registered = (e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered);
-        (void)cudaGetLastError();
-    });
-    if (!registered) return nullptr;
+int* host_status_device_ptr(cudaStream_t stream) {
+    static std::mutex mtx;
+    static std::atomic<int> state{0};               // 0 not tried, 1 registered, -1 failed
+    if (state.load(std::memory_order_acquire) == 0) {
+        // pinning is not allowed while the stream is being captured: that launch goes without the word
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return nullptr; }
+        std::lock_guard<std::mutex> lock(mtx);
+        if (state.load(std::memory_order_relaxed) == 0) {
+            const cudaError_t e = cudaHostRegister(const_cast<int*>(g_host_status_page), sizeof(g_host_status_page), cudaHostRegisterMapped);
+            (void)cudaGetLastError();
+            state.store((e == cudaSuccess || e == cudaErrorHostMemoryAlreadyRegistered) ? 1 : -1, std::memory_order_release);
+        }
+    }
+    if (state.load(std::memory_order_acquire) < 0) return nullptr;
     static int* cached[64] = {nullptr};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
@@ -264,6 +272,17 @@ int32_t ojx_e8t_gemm_dx_lowbit(int32_t bits, const void* grad_y, int32_t gy_dtyp
     if (bits != 1 && bits != 2) return OJX_ERR_UNSUPPORTED;
     return ojx::gemm_dx_fmt_impl(bits, grad_y, gy_dtype, M, packed, scales, N, K, group, dx, dx_dtype, workspace, workspace_bytes,
                                  (cudaStream_t)stream);
+}
+
+size_t ojx_e8t_linear_workspace_bytes(int32_t format, int32_t x_dtype, int64_t M, int64_t N, int64_t K, int32_t group, int32_t flags) {
+    return ojx::linear_workspace_bytes_impl(format, x_dtype, M, N, K, group, flags);
+}
+
+int32_t ojx_e8t_linear(int32_t format, const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
+                       const void* bias, int64_t N, int64_t K, int32_t group, void* y, int32_t y_dtype,
+                       void* workspace, size_t workspace_bytes, int32_t flags, void* stream) {
+    return ojx::linear_impl(format, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, workspace, workspace_bytes,
+                            flags, (cudaStream_t)stream);
 }
 
 int32_t ojx_e8t_gemm_status(const void* workspace, void* stream) {

@@ -211,6 +211,9 @@ def _get_packer_for_bitrate(bitrate: float):
     return E8LatticePacker                      # the reference's default branch (lattice.py:536-541)
 
 
+_FORMATS = {1.0: 1, 1.5: 0, 2.0: 2}               # bit-rate -> format code of the C ABI
+
+
 def _lowbit(bitrate: float) -> int:
     return 1 if float(bitrate) == 1.0 else 2
 
@@ -373,6 +376,15 @@ class E8LatticeLinear(nn.Module):
         return y.reshape(*x.shape[:-1], self.out_features)
 
     def forward_fused(self, x: torch.Tensor) -> torch.Tensor:
+        if self.rank == 0 and not torch.compiler.is_compiling():
+            bias = self._parameters["bias"]
+            if not torch.is_grad_enabled() or not (x.requires_grad or (bias is not None and bias.requires_grad)):
+                # nothing to differentiate: one native call, no autograd node
+                b = self._buffers
+                y = ops.layer_forward(_FORMATS[self.bitrate], x, b["packed_weight"], b["block_scales"], bias, self.out_features,
+                                      self.in_features, self.group_size, self.use_hadamard)
+                if y is not None:
+                    return y
         fused = self._forward_decode_with_adapter(x)
         if fused is not None:
             return fused

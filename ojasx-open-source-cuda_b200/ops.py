@@ -16,7 +16,7 @@ from . import _cabi
 
 _DT = {torch.float32: _cabi.OJX_F32, torch.float16: _cabi.OJX_F16, torch.bfloat16: _cabi.OJX_BF16}
 
-# Largest M handled by the decode-shape kernel; larger batches go to the tensor-core GEMM.
+# Largest M of a grouped decode-shape launch.
 GEMV_MAX_M = 16
 
 _scratch: Dict[Tuple[int, int, str], torch.Tensor] = {}
@@ -48,6 +48,13 @@ def _stream_ptr(device: torch.device) -> int:
     return int(torch.cuda.current_stream(device).cuda_stream)
 
 
+def _result(r, what: str):
+    """What a function of the torch module returned: its result, or a status that raises."""
+    if type(r) is int:
+        _cabi.check(r, what)
+    return r
+
+
 def scratch(device: torch.device, nbytes: int, tag: str = "ws") -> torch.Tensor:
     """Grow-only scratch buffer per (device, stream, tag) - the counterpart of the reference's
     ``_get_ephemeral_workspace`` (ojasx2/math/lattice.py:62-84), but only a few KB..MB of fp32
@@ -76,6 +83,10 @@ def packed_sizes(rows: int, cols: int, group_size: int) -> Tuple[int, int]:
 def fwht32(x: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Normalised 32-point Walsh-Hadamard transform of consecutive blocks of the last dimension, one kernel,
     bit-identical to the reference's ``fwht_block32`` (``ojasx2/math/lattice.py:91-102``)."""
+    if out is None:
+        y = _cabi.glue().fwht32(x)
+        if y is not None:
+            return _result(y, "ojx_e8t_fwht32")
     dev = _require_cuda(x)
     if x.shape[-1] % 32 != 0 or x.numel() == 0:
         raise ValueError("the last dimension must be a positive multiple of 32")
@@ -125,7 +136,11 @@ def _encode_lowbit(bits: int, w: torch.Tensor, group_size: int, out, hadamard: b
     wc = w.detach().contiguous()
     if hadamard and cols % 32 == 0:
         wc = fwht32(wc)
+    name = "ojx_e8t_encode_2bit" if bits == 2 else "ojx_e8t_encode_1bit"
     if out is None:
+        pair = _cabi.glue().encode(bits, wc, g, nbytes, nscales, 0)
+        if pair is not None:
+            return _result(pair, name)
         packed = torch.empty(nbytes, dtype=torch.uint8, device=dev)
         scales = torch.empty(nscales, dtype=torch.float16, device=dev)
     else:
@@ -133,7 +148,6 @@ def _encode_lowbit(bits: int, w: torch.Tensor, group_size: int, out, hadamard: b
         if packed.numel() != nbytes or scales.numel() != nscales or packed.dtype != torch.uint8 \
                 or scales.dtype != torch.float16 or not packed.is_contiguous() or not scales.is_contiguous():
             raise ValueError("output buffers have the wrong size, dtype or layout")
-    name = "ojx_e8t_encode_2bit" if bits == 2 else "ojx_e8t_encode_1bit"
     with torch.cuda.device(dev):
         st = getattr(_cabi.lib(), name)(wc.data_ptr(), _dtype_code(wc.dtype), rows, cols, g, packed.data_ptr(),
                                         scales.data_ptr(), _stream_ptr(dev))
@@ -145,8 +159,11 @@ def _decode_lowbit(bits: int, packed: torch.Tensor, scales: torch.Tensor, shape:
     dev = _require_cuda(packed, scales)
     rows, cols = int(shape[0]), int(shape[1])
     group = (packed.numel() * (4 if bits == 2 else 8)) // max(1, scales.numel())
-    out = torch.empty((rows, cols), dtype=dtype, device=dev)
     name = "ojx_e8t_decode_2bit" if bits == 2 else "ojx_e8t_decode_1bit"
+    w = _cabi.glue().decode(bits, packed, scales, rows, cols, group, _dtype_code(dtype))
+    if w is not None:
+        return _result(w, name)
+    out = torch.empty((rows, cols), dtype=dtype, device=dev)
     with torch.cuda.device(dev):
         st = getattr(_cabi.lib(), name)(packed.contiguous().data_ptr(), scales.contiguous().data_ptr(), rows, cols, group,
                                         _dtype_code(dtype), out.data_ptr(), _stream_ptr(dev))
@@ -154,42 +171,36 @@ def _decode_lowbit(bits: int, packed: torch.Tensor, scales: torch.Tensor, shape:
     return out
 
 
-LOWBIT_GEMV_MAX_M = 8      # rows of x the decode kernels of the 2.0-bit / 1.0-bit formats take
-
-
-def _linear_lowbit(bits: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor],
-                   n: int, k: int, group_size: int, out_dtype: Optional[torch.dtype]) -> torch.Tensor:
-    dev = _require_cuda(x, packed, scales)
-    x2 = x.detach().reshape(-1, k).contiguous()
-    m = int(x2.shape[0])
-    y = torch.empty((m, n), dtype=out_dtype or x2.dtype, device=dev)
+def _linear(fmt: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor],
+            n: int, k: int, group_size: int, out_dtype: Optional[torch.dtype], flags: int = 0) -> torch.Tensor:
+    """``y[M, N]`` of any format through ``ojx_e8t_linear`` (the library decides which kernel serves the call):
+    operands of the plain form go through the torch module, everything else is checked and converted here first."""
+    y = _cabi.glue().linear(fmt, x, packed, scales, bias, n, k, group_size, -1 if out_dtype is None else _dtype_code(out_dtype), flags, False)
+    if y is not None:
+        return _result(y, "ojx_e8t_linear")
+    dev, x2d, pk, sc, b = _prep_linear(x, packed, scales, bias, n, k)
+    _cabi.raise_pending()
+    m = int(x2d.shape[0])
+    y = torch.empty((m, n), dtype=out_dtype or x2d.dtype, device=dev)
     if m == 0:
         return y
-    b = None if bias is None else bias.detach().to(x2.dtype).contiguous()
     lib = _cabi.lib()
-    # the decode kernels on int8 tensor cores take groups of 32 with K % 2048 == 0; where only the fp32 decode kernel is
-    # left, the prefill kernel is already the faster one from four rows on (measured on 14336 x 4096, groups of 8:
-    # 59 against 50 us at four rows)
-    decode_tc = int(group_size) == 32 and k % 2048 == 0
-    if ((m > LOWBIT_GEMV_MAX_M or (m >= 4 and not decode_tc)) and int(group_size) in (8, 16, 32) and k % 256 == 0
-            and x2.dtype in (torch.bfloat16, torch.float16)
-            and packed.numel() * (4 if bits == 2 else 8) == n * k
-            and (x2.data_ptr() | packed.data_ptr() | scales.data_ptr()) % 16 == 0):
-        # batches of tokens: the tcgen05 prefill kernel with this format's decoder
-        with torch.cuda.device(dev):
-            ws = _gemm_scratch(dev, lib.ojx_e8t_gemm_workspace_bytes(m, n, k))
-            st = lib.ojx_e8t_gemm_lowbit(bits, x2.data_ptr(), _dtype_code(x2.dtype), m, packed.data_ptr(), scales.data_ptr(),
-                                         None if b is None else b.data_ptr(), n, k, int(group_size), y.data_ptr(), _dtype_code(y.dtype),
-                                         ws.data_ptr(), ws.numel(), _stream_ptr(dev))
-        _cabi.check(st, "ojx_e8t_gemm_lowbit")
-        return y
-    name = "ojx_e8t_linear_2bit" if bits == 2 else "ojx_e8t_linear_1bit"
     with torch.cuda.device(dev):
-        st = getattr(_cabi.lib(), name)(x2.data_ptr(), _dtype_code(x2.dtype), m, packed.data_ptr(), scales.data_ptr(),
-                                        None if b is None else b.data_ptr(), n, k, int(group_size), y.data_ptr(),
-                                        _dtype_code(y.dtype), _stream_ptr(dev))
-    _cabi.check(st, name)
+        need = lib.ojx_e8t_linear_workspace_bytes(fmt, _dtype_code(x2d.dtype), m, n, k, group_size, flags)
+        ws = torch.empty(need, dtype=torch.uint8, device=dev) if need else None
+        st = lib.ojx_e8t_linear(fmt, x2d.data_ptr(), _dtype_code(x2d.dtype), m, pk.data_ptr(), sc.data_ptr(),
+                                b.data_ptr() if b is not None else None, n, k, group_size, y.data_ptr(), _dtype_code(y.dtype),
+                                ws.data_ptr() if ws is not None else None, need, flags, _stream_ptr(dev))
+    _cabi.check(st, "ojx_e8t_linear")
     return y
+
+
+def layer_forward(fmt: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor], n: int, k: int,
+                  group_size: int, hadamard: bool) -> Optional[torch.Tensor]:
+    """A layer's forward without gradients, ``[..., K] -> [..., N]`` in ONE native call (rotation of x included); ``None``
+    when the operands are not of the plain form."""
+    y = _cabi.glue().linear(fmt, x, packed, scales, bias, n, k, group_size, -1, 0, hadamard)
+    return _result(y, "ojx_e8t_linear")
 
 
 def lowbit_lora_fusable(m: int, k: int, group_size: int, rank: int) -> bool:
@@ -242,7 +253,7 @@ def linear_2bit(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bia
     groups of 32 and K % 2048 == 0), more rows with 16-bit activations, groups of 8, 16 or 32 and K % 256 == 0 the tcgen05
     prefill kernel (weights rounded to fp16 once, as ``decode_2bit(..., torch.float16)`` gives them), anything else
     a scalar fp32 kernel."""
-    return _linear_lowbit(2, x, packed, scales, bias, n, k, group_size, out_dtype)
+    return _linear(2, x.reshape(-1, k), packed, scales, bias, int(n), int(k), int(group_size), out_dtype)
 
 
 def encode_1bit(w: torch.Tensor, group_size: int = 32, out: Optional[Tuple[torch.Tensor, torch.Tensor]] = None,
@@ -262,7 +273,7 @@ def linear_1bit(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bia
                 group_size: int, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
     """``y = x . W^T (+ bias)`` from root codes; routed as :func:`linear_2bit` (here the fp16 weights of the
     prefill kernel are exact)."""
-    return _linear_lowbit(1, x, packed, scales, bias, n, k, group_size, out_dtype)
+    return _linear(1, x.reshape(-1, k), packed, scales, bias, int(n), int(k), int(group_size), out_dtype)
 
 
 def _fp32_pass(x: torch.Tensor, name: str, vectors: bool) -> torch.Tensor:
@@ -317,6 +328,9 @@ def encode(w: torch.Tensor, group_size: int = 32, out: Optional[Tuple[torch.Tens
             wc = fwht32(wc)
     nbytes, nscales = packed_sizes(rows, cols, group_size)
     if out is None:
+        pair = _cabi.glue().encode(0, wc, int(group_size), nbytes, nscales, flags)
+        if pair is not None:
+            return _result(pair, "ojx_e8t_encode_ex")
         packed = torch.empty(nbytes, dtype=torch.uint8, device=dev)
         scales = torch.empty(nscales, dtype=torch.float16, device=dev)
     else:
@@ -345,6 +359,10 @@ def decode(packed: torch.Tensor, scales: torch.Tensor, shape: Tuple[int, int], d
     group = padded // max(1, scales.numel())
     if rows * cols > padded or group % 16 != 0 or group * scales.numel() != padded:
         raise ValueError("packed/scales sizes are inconsistent with the requested shape")
+    if out is None:
+        w = _cabi.glue().decode(0, packed, scales, rows, cols, group, _dtype_code(dtype))
+        if w is not None:
+            return _result(w, "ojx_e8t_decode")
     pk, sc = packed.contiguous(), scales.contiguous()
     if out is None:
         out = torch.empty((rows, cols), dtype=dtype, device=dev)
@@ -424,47 +442,15 @@ def linear(x2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: 
            out_dtype: Optional[torch.dtype] = None, force: Optional[str] = None) -> torch.Tensor:
     """y[M, N] = x[M, K] . dequant(W)^T (+ bias), output in x's dtype unless ``out_dtype`` is given.
 
-    Routing: M <= 16 -> decode-shape kernel (``ojx_e8t_gemv``); larger M with K % 256 == 0, 16-bit
-    activations and groups of 32 or 16 -> tcgen05 kernel (``ojx_e8t_gemm``; groups of 16 take it from three rows on);
-    everything else -> inside ``ojx_e8t_gemv`` the shared-memory fp32 kernel (up to eight rows, K % 64 == 0, groups
-    of 16, 32, 64, ...; any activation dtype) or the scalar kernel.  ``force`` ("gemv" or "gemm") overrides the routing for tests.
+    The library routes the call (``csrc/linear_host.cuh``): decode-shape kernels for small batches, the tcgen05 kernel for
+    batches of tokens, shared-memory or scalar fp32 kernels for what those do not take.  ``force`` ("gemv" or "gemm")
+    overrides the routing for tests.
     """
     n, k = int(out_features), int(in_features)
-    dev, x2d, pk, sc, b = _prep_linear(x2d, packed, scales, bias, n, k)
-    _cabi.raise_pending()
-    m = int(x2d.shape[0])
-    ydt = out_dtype or x2d.dtype
-    y = torch.empty((m, n), dtype=ydt, device=dev)
-    if m == 0:
-        return y
-    g = effective_group(group_size)
-    lib = _cabi.lib()
-    # groups of 16 (what the reference layer's default group size of 8 becomes for this format) have no tensor-core
-    # decode kernel: one or two rows run the shared-memory fp32 kernel inside ojx_e8t_gemv, more rows the prefill kernel
-    # (measured on 14336 x 4096 with the wrapper: 35 against 54 us at one row, 82 against 54 us at four)
-    use_gemm = ((m > GEMV_MAX_M or (g == 16 and m > 2)) and k % 256 == 0 and g in (16, 32) and x2d.dtype in (torch.bfloat16, torch.float16)
-                and (k * 3 // 16) * n == pk.numel())
-    if force == "gemm":
-        use_gemm = True
-    elif force == "gemv":
-        use_gemm = False
-    with torch.cuda.device(dev):
-        if use_gemm:
-            need = lib.ojx_e8t_gemm_workspace_bytes(m, n, k)
-            ws = _gemm_scratch(dev, need)
-            st = lib.ojx_e8t_gemm(x2d.data_ptr(), _dtype_code(x2d.dtype), m, pk.data_ptr(), sc.data_ptr(),
-                                  b.data_ptr() if b is not None else None, n, k, g, y.data_ptr(), _dtype_code(ydt),
-                                  ws.data_ptr(), ws.numel(), _stream_ptr(dev))
-            _cabi.check(st, "ojx_e8t_gemm")
-        else:
-            need = lib.ojx_e8t_gemv_workspace_bytes(m, n, k)
-            ws = scratch(dev, need, "gemv") if need else None
-            st = lib.ojx_e8t_gemv(x2d.data_ptr(), _dtype_code(x2d.dtype), m, pk.data_ptr(), sc.data_ptr(),
-                                  b.data_ptr() if b is not None else None, n, k, g, y.data_ptr(), _dtype_code(ydt),
-                                  ws.data_ptr() if ws is not None else None, ws.numel() if ws is not None else 0,
-                                  _stream_ptr(dev))
-            _cabi.check(st, "ojx_e8t_gemv")
-    return y
+    if x2d.dim() != 2:
+        raise ValueError(f"x must be [M, {k}], got {tuple(x2d.shape)}")
+    flags = 0 if force is None else {"gemv": _cabi.OJX_LINEAR_DECODE, "gemm": _cabi.OJX_LINEAR_GEMM}[force]
+    return _linear(0, x2d, packed, scales, bias, n, k, int(group_size), out_dtype, flags)
 
 
 def linear_dx(grad_y2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, out_features: int, in_features: int,
@@ -473,6 +459,11 @@ def linear_dx(grad_y2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor
     :func:`linear` with respect to its input, without a decoded copy of W.  Shapes the tensor-core kernel does not
     take (fp32 gradients, K % 256 != 0, N % 8 != 0, another group size) decode W with the decode kernel and multiply."""
     n, k = int(out_features), int(in_features)
+    g = effective_group(group_size)
+    if k % 256 == 0 and n % 8 == 0 and g in (16, 32) and (k * 3 // 16) * n == packed.numel():
+        dx = _cabi.glue().linear_dx(0, grad_y2d, packed, scales, n, k, g, -1 if out_dtype is None else _dtype_code(out_dtype))
+        if dx is not None:
+            return _result(dx, "ojx_e8t_gemm_dx")
     dev = _require_cuda(grad_y2d, packed, scales)
     if grad_y2d.dim() != 2 or grad_y2d.shape[1] != n:
         raise ValueError(f"grad_y must be [M, {n}], got {tuple(grad_y2d.shape)}")
@@ -481,7 +472,6 @@ def linear_dx(grad_y2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor
     gy = grad_y2d.contiguous()
     m = int(gy.shape[0])
     ydt = out_dtype or gy.dtype
-    g = effective_group(group_size)
     if m == 0:
         return torch.empty((0, k), dtype=ydt, device=dev)
     fast = (gy.dtype in (torch.bfloat16, torch.float16) and k % 256 == 0 and n % 8 == 0 and g in (16, 32)
@@ -507,6 +497,11 @@ def linear_dx_lowbit(bits: int, grad_y2d: torch.Tensor, packed: torch.Tensor, sc
     packed codes (``ojx_e8t_gemm_dx_lowbit``; the weights enter the tensor cores as fp16).  Shapes the kernel does not
     take (fp32 gradients, K % 256 != 0, N % 8 != 0, groups other than 8, 16 and 32) decode W and multiply."""
     n, k = int(out_features), int(in_features)
+    if (k % 256 == 0 and n % 8 == 0 and int(group_size) in (8, 16, 32) and packed.numel() * (4 if bits == 2 else 8) == n * k
+            and (grad_y2d.data_ptr() | packed.data_ptr() | scales.data_ptr()) % 16 == 0):
+        dx = _cabi.glue().linear_dx(bits, grad_y2d, packed, scales, n, k, int(group_size), -1 if out_dtype is None else _dtype_code(out_dtype))
+        if dx is not None:
+            return _result(dx, "ojx_e8t_gemm_dx_lowbit")
     dev = _require_cuda(grad_y2d, packed, scales)
     if grad_y2d.dim() != 2 or grad_y2d.shape[1] != n:
         raise ValueError(f"grad_y must be [M, {n}], got {tuple(grad_y2d.shape)}")
@@ -540,10 +535,9 @@ def _gemm_scratch(device: torch.device, nbytes: int) -> torch.Tensor:
 
 
 def gemm_status(device: torch.device) -> None:
-    """Raise if a bounded wait inside the last prefill GEMM on this device/stream expired."""
-    ws = _gemm_scratch(device, 256)
+    """Raise if a bounded wait inside a launch on this device expired since the last check (synchronises)."""
     with torch.cuda.device(device):
-        st = _cabi.lib().ojx_e8t_gemm_status(ws.data_ptr(), _stream_ptr(device))
+        st = _cabi.lib().ojx_e8t_device_status()
     _cabi.check(st, "ojx_e8t_gemm (device status)")
 
 
@@ -633,17 +627,18 @@ class GroupedGemv:
             if not (1 <= len(peer_delta) <= 8):
                 raise ValueError("peer_delta needs one entry per rank, at most 8")
             self._peers = (ctypes.c_int64 * len(peer_delta))(*[int(d) for d in peer_delta])
+        index = self.device.index if self.device.index is not None else torch.cuda.current_device()
+        self._args = (index, self.table.data_ptr(), self.count, self.total_tiles, self.M, _dtype_code(self.x_dtype),
+                      _dtype_code(self.y_dtype), self.needs_reduce,
+                      ctypes.addressof(self._peers) if self._peers is not None else 0,
+                      len(self._peers) if self._peers is not None else 1, self.peer_sync or 0)
 
     def __call__(self, independent: Optional[bool] = None) -> None:
         """Launches the group; ``independent`` overrides the constructor's choice for this call."""
         flags = self.flags
         if independent is not None:
             flags = (flags | _cabi.OJX_GEMV_INDEPENDENT) if independent else (flags & ~_cabi.OJX_GEMV_INDEPENDENT)
-        _cabi.raise_pending()
-        with torch.cuda.device(self.device):
-            st = _cabi.lib().ojx_e8t_gemv_grouped_ex(
-                self.table.data_ptr(), self.count, self.total_tiles, self.M, _dtype_code(self.x_dtype),
-                _dtype_code(self.y_dtype), self.needs_reduce,
-                ctypes.addressof(self._peers) if self._peers is not None else None,
-                len(self._peers) if self._peers is not None else 1, self.peer_sync, flags, _stream_ptr(self.device))
-        _cabi.check(st, "ojx_e8t_gemv_grouped_ex")
+        a = self._args
+        st = _cabi.glue().grouped(a[0], a[1], a[2], a[3], a[4], a[5], a[6], a[7], a[8], a[9], a[10], flags)
+        if st != 0:
+            _cabi.check(st, "ojx_e8t_gemv_grouped_ex")

@@ -1,0 +1,49 @@
+"""Kernel and dispatch variants at the sizes where they can go wrong, against the dense product of the decoded weights."""
+
+import pytest
+
+from conftest import have_cuda, load_pkg
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def P():
+    if not have_cuda():
+        pytest.skip("no CUDA device")
+    return load_pkg()
+
+
+def _packer(P, bits):
+    return {1.0: P.RootE8LatticePacker, 1.5: P.TernaryE8LatticePacker, 2.0: P.E8LatticePacker}[bits]
+
+
+def _problem(P, bits, n, k, group, seed=7):
+    w = P.ops.generate(n * k, seed, 0.02, torch.float16, torch.device(DEV)).view(n, k)
+    packed, scales, shape = _packer(P, bits).pack(w, group)
+    return packed, scales, _packer(P, bits).unpack(packed, scales, shape, torch.float32)
+
+
+@pytest.mark.parametrize("bits", [1.0, 1.5, 2.0])
+def test_operands_of_any_form_give_the_plain_call_s_result(P, bits):
+    """Non-contiguous x, a bias of another dtype, leading dimensions: the general path equals the native call."""
+    n, k, m = 96, 2048, 3
+    packed, scales, wd = _problem(P, bits, n, k, 32)
+    fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    x = P.ops.generate(m * k, 8, 1.0, torch.bfloat16, torch.device(DEV)).view(m, k)
+    bias = P.ops.generate(n, 9, 0.5, torch.bfloat16, torch.device(DEV))
+    plain = fn(x, packed, scales, bias, n, k, 32)
+    ref = x.float() @ wd.t() + bias.float()
+    assert float((plain.float() - ref).norm() / ref.norm()) <= 4e-3
+    assert torch.equal(plain, fn(x.t().contiguous().t(), packed, scales, bias.float(), n, k, 32))
+    layer = P.E8LatticeLinear(k, n, bias=True, group_size=32, bitrate=bits, device=DEV, dtype=torch.bfloat16)
+    layer.packed_weight.copy_(packed)
+    layer.block_scales.copy_(scales)
+    with torch.no_grad():
+        layer.bias.copy_(bias)
+        assert torch.equal(layer(x.view(m, 1, k)), plain.view(m, 1, n))          # native call
+    y = layer(x.clone().requires_grad_(True))                                    # autograd node
+    assert y.requires_grad and torch.equal(y.detach(), plain)
