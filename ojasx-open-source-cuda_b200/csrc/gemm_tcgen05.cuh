@@ -61,6 +61,7 @@ struct GemmParams {
     int* host_status;              // mapped host word for the same event (may be null)
     int clear_status;              // this launch clears the status word (no wait can have given up yet)
     int M, N, K;
+    int k_len;                     // contraction length that matters (K, or less where K is a padded row length)
     int y_stride;                  // elements between consecutive token rows of y (N of the whole matrix)
     int tile_limit;                // process only the first tile_limit tiles of the enumeration
     int y_dtype;
@@ -370,7 +371,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
     const int m_blocks = (p.M + p.bn - 1) / p.bn;
     const uint32_t x_bytes = (uint32_t)p.bn * kGemmBK * 2;
     const int tiles = min(n_blocks * m_blocks, p.tile_limit);
-    const int k_blocks = (p.K + kGemmBK - 1) / kGemmBK;
+    const int k_blocks = (p.k_len + kGemmBK - 1) / kGemmBK;
 
     if (warp == 12) {
         // ---------------- TMA producer ----------------
@@ -560,6 +561,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q, ++it) {
+                    if (ch * 4 + q >= k_blocks) break;                             // padded rows: the last chunk may be cut short
                     const int s = it % kGemmStages;
                     const uint32_t ph = (it / kGemmStages) & 1u;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, 4)) { ok = false; break; }
@@ -626,6 +628,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q, ++it) {
+                    if (ch * 4 + q >= k_blocks) break;                             // padded rows: the last chunk may be cut short
                     const int s = it % kGemmStages;
                     const uint32_t ph = (it / kGemmStages) & 1u;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, 4)) { ok = false; break; }
@@ -728,18 +731,43 @@ inline GemmKernelFn gemm_kernel_for(int fmt, int group, int* slot) {
     return nullptr;
 }
 
-inline bool gemm_fast_ok(int64_t M, int64_t N, int64_t K, int group, int x_dtype) {
-    return M >= 1 && N >= 1 && K >= 256 && K % 256 == 0 && group == 32 &&
+inline bool gemm_fast_ok(int64_t M, int64_t N, int64_t K, int x_dtype) {
+    return M >= 1 && N >= 1 && K >= 32 && K % 32 == 0 &&
            (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && M < (1 << 30) && N < (1 << 30) && K < (1 << 30);
 }
 
 // Scratch: a 256-byte status block (word 0: give-up code of a bounded wait; zeroed by every call), the
-// per-token output factors (M floats, padded to 256 bytes), then room for an fp16 copy of the activations.
-inline size_t gemm_up_bytes(int64_t M) { return (((size_t)M * 4) + 255) & ~(size_t)255; }
+// per-token output factors (M floats, padded to 256 bytes), room for an fp16 copy of the activations and, when K is not
+// a multiple of 256, the weights with every row padded to one (sized for the largest format, 2 bits with groups of 8).
+inline size_t pad256(size_t n) { return (n + 255) & ~(size_t)255; }
+inline size_t gemm_up_bytes(int64_t M) { return pad256((size_t)M * 4); }
+inline int64_t gemm_padded_k(int64_t K) { return (K + 255) / 256 * 256; }
 size_t gemm_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
-    (void)N;
     if (M <= 0 || K <= 0) return 256;
-    return 256 + gemm_up_bytes(M) + (size_t)M * (size_t)K * 2;
+    size_t need = 256 + gemm_up_bytes(M) + (size_t)M * (size_t)K * 2;
+    if (K % 256 != 0 && N > 0) need = pad256(need) + 2 * (size_t)N * (size_t)(gemm_padded_k(K) / 4);
+    return need;
+}
+
+// Copies rows of `src_bytes` (even) to rows of `dst_bytes` (a multiple of 16), the rest of a row zero: codes or scales of
+// a matrix whose K is not a multiple of 256, whose rows start at any even address, for the 16-byte loads of the decoders.
+// Thread = one 16-byte destination vector.  It costs about the packed bytes twice (2000 x 2912: 2 us), once per call,
+// instead of 2-byte accesses in the decoders' inner loop; a batch of tokens hides it.
+__global__ void __launch_bounds__(256) pad_rows_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst, int64_t rows,
+                                                        int src_bytes, int dst_bytes) {
+    const int vecs = dst_bytes / 16;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < rows * vecs; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t row = i / vecs;
+        const int at = (int)(i - row * vecs) * 16;
+        const uint16_t* s = reinterpret_cast<const uint16_t*>(src + row * src_bytes + at);
+        uint32_t w[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const uint32_t lo = at + 4 * j < src_bytes ? __ldg(s + 2 * j) : 0u, hi = at + 4 * j + 2 < src_bytes ? __ldg(s + 2 * j + 1) : 0u;
+            w[j] = lo | (hi << 16);
+        }
+        *reinterpret_cast<uint4*>(dst + row * dst_bytes + at) = make_uint4(w[0], w[1], w[2], w[3]);
+    }
 }
 
 // fmt: 0 ternary codes (3 bytes per 16 weights), 2 the 2.0-bit format (one byte per 4 weights, weight =
@@ -756,11 +784,12 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
     if (fmt == 0) group = effective_group(group);
     int slot = 0;
     const GemmKernelFn kernel = gemm_kernel_for<false>(fmt, group, &slot);      // sibling formats: groups of 8, 16 or 32
-    OJX_RETURN_IF(kernel == nullptr || !gemm_fast_ok(M, N, K, 32, x_dtype), OJX_ERR_UNSUPPORTED);
+    OJX_RETURN_IF(kernel == nullptr || !gemm_fast_ok(M, N, K, x_dtype), OJX_ERR_UNSUPPORTED);
     OJX_RETURN_IF(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) |
                     reinterpret_cast<uintptr_t>(scales)) & 15) != 0, OJX_ERR_ALIGN);
     const bool convert = x_dtype == OJX_BF16;
-    const size_t need = convert ? gemm_workspace_bytes_impl(M, N, K) : 256;
+    const bool ragged = K % 256 != 0;
+    const size_t need = (convert || ragged) ? gemm_workspace_bytes_impl(M, N, K) : 256;
     OJX_RETURN_IF(!workspace || workspace_bytes < need, OJX_ERR_WORKSPACE);
     OJX_RETURN_IF((reinterpret_cast<uintptr_t>(workspace) & 255) != 0, OJX_ERR_ALIGN);
     PFN_encodeTiled encode = get_encode_tiled();
@@ -797,6 +826,23 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
         if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
     }
 
+    // K not a multiple of 256: the kernel reads a padded copy of the weights; its contraction stops at K
+    const int64_t Kp = gemm_padded_k(K);
+    if (ragged) {
+        auto code_bytes = [&](int64_t k) { return fmt == 0 ? k * 3 / 16 : (fmt == 2 ? k / 4 : k / 8); };
+        uint8_t* wp = static_cast<uint8_t*>(workspace) + pad256(256 + gemm_up_bytes(M) + (size_t)M * (size_t)K * 2);
+        uint8_t* wsc = wp + N * code_bytes(Kp);                      // a multiple of 16 bytes per row
+        auto pad = [&](const void* src, uint8_t* dst, int64_t sb, int64_t db) {
+            const int64_t blocks = (N * (db / 16) + 255) / 256, cap = (int64_t)num_sms() * 32;
+            pad_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(static_cast<const uint8_t*>(src), dst, N, (int)sb, (int)db);
+        };
+        pad(packed, wp, code_bytes(K), code_bytes(Kp));
+        pad(scales, wsc, K / group * 2, Kp / group * 2);
+        if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
+        packed = wp;
+        scales = reinterpret_cast<const uint16_t*>(wsc);
+    }
+
     // One launch over the rectangle of weight rows [n0, N) x tokens [m0, M) of the problem, in tiles of
     // rows x bn, stopping after tile_limit tiles of the enumeration (token block major, weight-row block minor).
     auto launch_region = [&](int64_t n0, int64_t m0, int rows, int bn, int tile_limit) -> int32_t {
@@ -812,14 +858,14 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return OJX_ERR_LAUNCH;
         GemmParams prm;
-        prm.packed = packed + (fmt == 0 ? (size_t)n0 * (size_t)K * 3 / 16 : (size_t)n0 * (size_t)K / (fmt == 2 ? 4 : 8));
-        prm.scales = scales + (size_t)n0 * (size_t)K / (size_t)group;
+        prm.packed = packed + (fmt == 0 ? (size_t)n0 * (size_t)Kp * 3 / 16 : (size_t)n0 * (size_t)Kp / (fmt == 2 ? 4 : 8));
+        prm.scales = scales + (size_t)n0 * (size_t)Kp / (size_t)group;
         prm.bias = bias ? static_cast<const uint8_t*>(bias) + (size_t)n0 * dtype_size(x_dtype) : nullptr;
         prm.y = static_cast<uint8_t*>(y) + ((size_t)m0 * (size_t)N + (size_t)n0) * dtype_size(y_dtype);
         prm.status = static_cast<int32_t*>(workspace);
         prm.host_status = host_status_device_ptr(s);
         prm.clear_status = (n0 == 0 && m0 == 0) ? 1 : 0;
-        prm.M = (int)Ms; prm.N = (int)Ns; prm.K = (int)K;
+        prm.M = (int)Ms; prm.N = (int)Ns; prm.K = (int)Kp; prm.k_len = (int)K;
         prm.y_stride = (int)N;
         prm.y_dtype = y_dtype; prm.bias_dtype = x_dtype;
         prm.up = up ? up + m0 : nullptr;
@@ -934,6 +980,7 @@ int32_t gemm_dx_fmt_impl(int fmt, const void* gy, int gy_dtype, int64_t M, const
     prm.M = (int)M;
     prm.N = (int)K;                    // roles swapped: the output's feature dimension is the weight columns ...
     prm.K = (int)N;                    // ... and the contraction runs over the weight rows
+    prm.k_len = (int)N;
     prm.y_stride = (int)K;
     prm.y_dtype = dx_dtype; prm.bias_dtype = gy_dtype;
     prm.up = up;

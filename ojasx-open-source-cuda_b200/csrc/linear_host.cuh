@@ -17,10 +17,11 @@ constexpr int kForceDecode = 1, kForceGemm = 2;        // flags of ojx_e8t_linea
 //     decode kernel loses from four rows on (59 against 50 us at four rows, groups of 8).
 inline bool linear_uses_gemm(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, bool aligned, int flags) {
     if (flags & kForceDecode) return false;
-    const bool able = (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && K % 256 == 0 && aligned &&
+    const bool able = (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && K % 32 == 0 && aligned &&
                       (group == 32 || group == 16 || (fmt != 0 && group == 8));
     if (flags & kForceGemm) return true;               // the kernel's own checks report what it cannot take
     if (!able) return false;
+    if (K % 256 != 0) return M > 8;                    // K of any number of 32s: the weights are padded first
     if (fmt == 0) return M > 16 || (group == 16 && M > 2);
     const bool decode_tc = group == 32 && K % 2048 == 0;
     return M > 8 || (M >= 4 && !decode_tc);
@@ -31,7 +32,7 @@ inline int linear_group(int fmt, int group) { return fmt == 0 ? effective_group(
 size_t linear_workspace_bytes_impl(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, int flags) {
     group = linear_group(fmt, group);
     if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, true, flags))
-        return x_dtype == OJX_BF16 ? gemm_workspace_bytes_impl(M, N, K) : 256;
+        return (x_dtype == OJX_BF16 || K % 256 != 0) ? gemm_workspace_bytes_impl(M, N, K) : 256;
     return fmt == 0 ? gemv_workspace_bytes_impl(M, N, K) : 0;
 }
 

@@ -47,3 +47,18 @@ def test_operands_of_any_form_give_the_plain_call_s_result(P, bits):
         assert torch.equal(layer(x.view(m, 1, k)), plain.view(m, 1, n))          # native call
     y = layer(x.clone().requires_grad_(True))                                    # autograd node
     assert y.requires_grad and torch.equal(y.detach(), plain)
+
+
+@pytest.mark.parametrize("bits,group", [(1.5, 32), (1.5, 16), (2.0, 32), (2.0, 8), (1.0, 32), (1.0, 16), (1.0, 8)])
+@pytest.mark.parametrize("m,n,k", [(17, 40, 32), (130, 72, 288), (333, 520, 736), (64, 129, 2080)])
+def test_batches_of_tokens_with_k_a_multiple_of_32(P, bits, group, m, n, k):
+    """K that is no multiple of 256: rows start at any even address and the last 256-wide chunk is cut short."""
+    packed, scales, wd = _problem(P, bits, n, k, group)
+    fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    w16 = wd.half().float() if bits == 2.0 else wd           # the prefill kernel rounds 2.0-bit weights to fp16 once
+    for dt in (torch.bfloat16, torch.float16):
+        x = P.ops.generate(m * k, 8, 1.0, dt, torch.device(DEV)).view(m, k)
+        y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
+        bound = x.float().abs() @ w16.abs().t()
+        assert float(((y - x.float() @ w16.t()).abs() / (bound + 1e-20)).max()) <= 2e-5
+    P.ops.gemm_status(torch.device(DEV))
