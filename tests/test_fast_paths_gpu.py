@@ -62,3 +62,22 @@ def test_batches_of_tokens_with_k_a_multiple_of_32(P, bits, group, m, n, k):
         bound = x.float().abs() @ w16.abs().t()
         assert float(((y - x.float() @ w16.t()).abs() / (bound + 1e-20)).max()) <= 2e-5
     P.ops.gemm_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("group", [8, 32, 64])
+def test_root_packer_on_ties_zeros_and_non_finite_values(P, oracle, group):
+    """The pruned search against the oracle's walk over all 256 vectors where magnitudes coincide, vanish or are not finite."""
+    g = torch.Generator().manual_seed(3)
+    w = torch.randn(64, 512, generator=g)
+    w[8:16] = torch.round(w[8:16] * 2) / 2                              # many equal magnitudes
+    w[16:24] *= (torch.rand(8, 512, generator=g) < 0.4)                 # most magnitudes zero
+    w[24:32] = w[24:32].sign() * 0.37                                   # all equal
+    w[32:40] *= torch.where(torch.rand(8, 512, generator=g) < 0.3, 1e-7, 1.0)
+    w[40, ::64] = 0.0
+    w[41] = 0.0
+    for dt in (torch.float32, torch.bfloat16, torch.float16):
+        wt = w.to(dt)
+        packed, scales, _ = P.RootE8LatticePacker.pack(wt.to(DEV), group)
+        p_ref, s_ref, _ = oracle.encode_1bit(wt.float().numpy(), group)
+        assert (packed.cpu().numpy() == p_ref).all()
+        assert (scales.view(torch.int16).cpu().numpy().view("uint16") == s_ref.view("uint16")).all()
