@@ -24,7 +24,7 @@ GLUE_PATH = os.path.join(LIB_DIR, "_ojx_torch.so")       # CPython extension: th
 
 OJX_F32, OJX_F16, OJX_BF16 = 0, 1, 2
 OJX_GEMV_STATIC_WEIGHTS, OJX_GEMV_SIGNAL_PEERS, OJX_GEMV_WAIT_PEERS, OJX_GEMV_TEST_LOSE_COPY = 1, 2, 4, 8
-OJX_GEMV_INDEPENDENT = 16
+OJX_GEMV_INDEPENDENT, OJX_GEMV_SPLIT_K2, OJX_GEMV_SPLIT_K4 = 16, 32, 64
 OJX_ENCODE_HADAMARD = 1
 OJX_LINEAR_DECODE, OJX_LINEAR_GEMM = 1, 2
 PEER_SYNC_BYTES = 48        # sizeof(ojx_e8t_peer_sync): epoch, arrived, status, spin_limit, flag[8]
@@ -39,7 +39,7 @@ EXPORTED_SYMBOLS = (
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-shared", "-Xcompiler", "-fPIC", "--split-compile=0",
 ]
 
 _lock = threading.Lock()

@@ -1,19 +1,20 @@
 // Shared pieces of the decode-shape fused linear  y[M,N] = x[M,K] . dequant(W)[N,K]^T  for small M:
-// work-item geometry, shared-memory and cp.async helpers, the output-window map for column-sharded
-// launches, the partial-sum reduce kernel for K larger than one chunk, and the generic correctness kernel
-// for shapes and dtypes the tensor-core kernel (gemv_a16.cuh) does not cover.
+// the interface's tile units, shared-memory and cp.async helpers, the output-window map for column-sharded launches, launch
+// helpers, and the generic correctness kernel for shapes and dtypes the tensor-core kernels do not cover.
 //
 // Replaces, for small batches, _FusedE8GEMMFunction.forward (ojasx2/math/lattice.py:551-640)
 // and the reference's scalar fused kernel (ojasx2/math/csrc/ojasx_math_core.hpp:580-634):
 // per (m, n) the result is sum over groups of (sum_k x*coord) * scale, accumulated in fp32.
 #pragma once
 
+#include <atomic>
+#include <utility>
+
 #include "common.cuh"
 
 namespace ojx {
 
 constexpr int kGemvWarps = 16;
-constexpr int kGemvThreads = kGemvWarps * 32;
 
 __host__ __device__ inline int gemv_active_warps(int K) {
     const int slices = K / 256;
@@ -110,11 +111,6 @@ __device__ __noinline__ bool peer_wait(const PeerMap& pm) {
     return ok;
 }
 
-template <bool kBf16> __device__ __forceinline__ float load_act(const void* p, int64_t idx) {
-    if (kBf16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
-    return __half2float(static_cast<const __half*>(p)[idx]);
-}
-
 __device__ __forceinline__ void sts_u128(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -124,119 +120,14 @@ __device__ __forceinline__ uint4 lds_u128(uint32_t addr) {
     return v;
 }
 
-// Index of the problem that owns work item `item` (tile_begin ascends): the whole CTA counts the entries that
-// start at or before it, one coalesced pass over the table instead of a chain of dependent loads (a 64-entry
-// table walked entry by entry cost the last CTAs ~40 us at the start of every grouped launch).  Every thread of
-// the CTA must call this.
-__device__ __forceinline__ int find_problem(const ojx_e8t_gemv_problem* probs, int count, int item, int scale) {
-    if (count == 1) return 0;                                  // single-problem launches (a layer at a time) skip the pass
-    int found = 0;
-    for (int base = 0; base < count; base += (int)blockDim.x) {
-        const int t = base + (int)threadIdx.x;
-        found += __syncthreads_count(t < count && scale * probs[t].tile_begin <= item);
-    }
-    return max(found - 1, 0);
-}
-
-// 16-byte asynchronous copy global -> shared (L2 only, no L1 allocation) and the mbarrier arrive that
-// fires when all of this thread's earlier copies have landed.
+// 16-byte asynchronous copy global -> shared (L2 only, no L1 allocation).
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
-__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
-    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
-}
-
-// Geometry of a work item in shared memory: 32 rows of codes, then 32 rows of scales; a row holds one
-// 48-byte (codes) / 16-byte (scales) piece per 256-wide slice of the K chunk and ends in 16 bytes of padding,
-// so that the eight rows one shared-memory load touches fall on distinct banks.
-constexpr int kGemvMaxCodePitch = kGemvWarps * 48 + 16;     // 784
-constexpr int kGemvMaxScalePitch = kGemvWarps * 16 + 16;    // 272
-
 __device__ __forceinline__ float load_any(const void* p, int dt, int64_t i) {
     if (dt == OJX_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[i]);
     if (dt == OJX_F16) return __half2float(static_cast<const __half*>(p)[i]);
     return static_cast<const float*>(p)[i];
-}
-
-// The optional low-rank term of a problem for output (activation row col, weight row row).
-// Kept out of line: it is rare, and inlined into the decode kernels' epilogue it costs them registers they do not have.
-template <bool kBf16>
-__device__ __noinline__ float lora_term(const ojx_e8t_gemv_problem& P, int64_t col, int64_t row) {
-    float acc = 0.f;
-    const float* t = P.lora_t + col * P.lora_rank;
-    for (int r = 0; r < P.lora_rank; ++r) acc = fmaf(t[r], load_act<kBf16>(P.lora_b, (int64_t)r * P.N + row), acc);
-    return acc;
-}
-
-// Sums the K-chunk partials of every problem that has them (fixed order), adds bias and the low-rank term, casts,
-// stores - to this rank's buffer and to every peer's window.  16-bit outputs whose rows come in multiples of eight
-// are handled eight rows (one 16-byte vector) per thread.
-template <bool kBf16>
-__global__ void __launch_bounds__(256, 3) gemv_reduce_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev,
-                                                           const __grid_constant__ ojx_e8t_gemv_problem single,
-                                                           int count, int M, int y_dtype, const __grid_constant__ PeerMap peers) {
-    const ojx_e8t_gemv_problem* probs = probs_dev != nullptr ? probs_dev : &single;
-    for (int p = blockIdx.y; p < count; p += gridDim.y) {
-        const ojx_e8t_gemv_problem& P = probs[p];
-        if (P.partial == nullptr) continue;
-        const int kc = gemv_kchunks(P.K);
-        const int64_t total = (int64_t)M * P.N;
-        const int64_t ld = P.ldy > 0 ? P.ldy : P.N;
-        const bool vec = y_dtype != OJX_F32 && (P.N & 7) == 0 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(P.y) & 15) == 0 &&
-                         (reinterpret_cast<uintptr_t>(P.partial) & 31) == 0;
-        if (vec) {
-            const int64_t per_col = P.N / 8;
-            for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < (int64_t)M * per_col;
-                 v += (int64_t)gridDim.x * blockDim.x) {
-                const int64_t col = v / per_col, row = (v - col * per_col) * 8;
-                float s8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                for (int c = 0; c < kc; ++c) {
-                    const float4* src = reinterpret_cast<const float4*>(P.partial + (int64_t)c * total + col * P.N + row);
-                    const float4 a = __ldcg(src), b = __ldcg(src + 1);
-                    s8[0] += a.x; s8[1] += a.y; s8[2] += a.z; s8[3] += a.w;
-                    s8[4] += b.x; s8[5] += b.y; s8[6] += b.z; s8[7] += b.w;
-                }
-                uint32_t w[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    float lo = s8[2 * i], hi = s8[2 * i + 1];
-                    if (P.bias != nullptr) { lo += load_act<kBf16>(P.bias, row + 2 * i); hi += load_act<kBf16>(P.bias, row + 2 * i + 1); }
-                    if (P.lora_rank > 0) { lo += lora_term<kBf16>(P, col, row + 2 * i); hi += lora_term<kBf16>(P, col, row + 2 * i + 1); }
-                    if (y_dtype == OJX_BF16) {
-                        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
-                        w[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    } else {
-                        const __half2 h = __floats2half2_rn(lo, hi);
-                        w[i] = *reinterpret_cast<const uint32_t*>(&h);
-                    }
-                }
-                const uint4 val = make_uint4(w[0], w[1], w[2], w[3]);
-                uint8_t* dst = static_cast<uint8_t*>(P.y) + (col * ld + row) * 2;
-#pragma unroll 1
-                for (int r = 0; r < peers.world; ++r)              // delta is 0 for this rank itself
-                    *reinterpret_cast<uint4*>(dst + peers.delta[r]) = val;
-            }
-            continue;
-        }
-        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
-             i += (int64_t)gridDim.x * blockDim.x) {
-            float s = 0.f;
-            for (int c = 0; c < kc; ++c) s += P.partial[(int64_t)c * total + i];
-            const int64_t col = i / P.N, row = i - col * P.N;
-            if (P.bias != nullptr) s += load_act<kBf16>(P.bias, row);
-            if (P.lora_rank > 0) s += lora_term<kBf16>(P, col, row);
-            const int64_t at = col * ld + row;
-            store_any(P.y, y_dtype, at, s);
-#pragma unroll 1
-            for (int r = 0; r < peers.world; ++r)                  // the other ranks' windows (nothing when world == 1)
-                if (peers.delta[r] != 0) store_any(static_cast<uint8_t*>(P.y) + peers.delta[r], y_dtype, at, s);
-        }
-    }
-    if (peers.sync != nullptr && (peers.mode & OJX_GEMV_SIGNAL_PEERS)) {
-        __syncthreads();
-        if (threadIdx.x == 0) peer_signal(peers);
-    }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -307,6 +198,49 @@ static int num_sms() {
         cached[dev] = n > 0 ? n : 148;
     }
     return cached[dev];
+}
+
+// Opting in to more than 48 KB of dynamic shared memory is a per-device (per-context) attribute of a kernel:
+// `done` keeps one bit per device ordinal.
+template <typename Kernel>
+static int32_t ensure_dynamic_smem(Kernel kernel, size_t bytes, std::atomic<uint64_t>& done) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return OJX_ERR_LAUNCH;
+    const uint64_t bit = 1ull << dev;
+    if (done.load(std::memory_order_acquire) & bit) return OJX_OK;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    if (e != cudaSuccess) { last_cuda_error() = e; return OJX_ERR_LAUNCH; }
+    done.fetch_or(bit, std::memory_order_release);
+    return OJX_OK;
+}
+
+// Launch with the "programmatic stream serialization" attribute when `overlap` is set: the kernel may then start
+// (and run up to its griddepcontrol.wait) while the previous kernel of the stream is still draining.
+template <typename... Params, typename... Args>
+static int32_t launch_maybe_overlapped(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t s, bool overlap,
+                                       int cluster, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    int n = 0;
+    if (overlap) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+    if (e != cudaSuccess) { last_cuda_error() = e; (void)cudaGetLastError(); return OJX_ERR_LAUNCH; }
+    return OJX_OK;
 }
 
 }  // namespace ojx

@@ -21,7 +21,7 @@
 // needed because nothing is shared between rows).  Lane (g, t) owns rows g and g + 8 and the 64 codes 64t..64t+63 of
 // the round (two scale groups); its eight steps (word q = 0..3, register pair p = 0, 1) feed two MMAs each.
 //
-// Activations: 28-bit fixed point per scale group exactly as in the ternary one-row kernel (gemv_a16.cuh, kI8): the
+// Activations: 28-bit fixed point per scale group exactly as in the ternary one-row kernel (gemv_mma.cuh, kI8): the
 // group's largest finite magnitude fixes the exponent, the integers are split into four base-128 digits; accumulator
 // column 2t' + h takes digits 2h, 2h + 1 of the group that lane quarter t' decodes, so only lane (g, t) with
 // g >> 1 == t supplies a non-zero operand.  The operand words depend on the round only, so every CTA builds them once
@@ -30,7 +30,7 @@
 // which reproduces the dense product's NaN / Inf pattern.
 #pragma once
 
-#include "gemv_a16.cuh"
+#include "gemv_mma.cuh"
 
 namespace ojx {
 

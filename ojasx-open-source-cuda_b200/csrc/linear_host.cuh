@@ -9,22 +9,14 @@ namespace ojx {
 
 constexpr int kForceDecode = 1, kForceGemm = 2;        // flags of ojx_e8t_linear (tests)
 
-// Batches of tokens run the tcgen05 kernel, decode shapes the GEMV kernels.  Where the line lies (14336 x 4096):
-//   * ternary, groups of 32: the decode kernel takes up to 16 rows (its two column blocks);
-//   * ternary, groups of 16: no tensor-core decode kernel, the shared-memory fp32 kernel wins for one or two rows only
-//     (35 against 54 us at one row, 82 against 54 us at four);
-//   * 2.0 / 1.0 bits: groups of 32 with K % 2048 == 0 have int8 decode kernels for up to eight rows; elsewhere the fp32
-//     decode kernel loses from four rows on (59 against 50 us at four rows, groups of 8).
+// Batches of tokens run the tcgen05 kernel, up to sixteen rows the decode kernels: 28672 x 8192 at sixteen rows, 78 us against
+// 106 us and more (whose smallest tile takes 35 us at K = 4096 whatever the token count).
 inline bool linear_uses_gemm(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, bool aligned, int flags) {
+    (void)N;
     if (flags & kForceDecode) return false;
-    const bool able = (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && K % 32 == 0 && aligned &&
-                      (group == 32 || group == 16 || (fmt != 0 && group == 8));
     if (flags & kForceGemm) return true;               // the kernel's own checks report what it cannot take
-    if (!able) return false;
-    if (K % 256 != 0) return M > 8;                    // K of any number of 32s: the weights are padded first
-    if (fmt == 0) return M > 16 || (group == 16 && M > 2);
-    const bool decode_tc = group == 32 && K % 2048 == 0;
-    return M > 8 || (M >= 4 && !decode_tc);
+    return M > 16 && (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && K % 32 == 0 && aligned &&
+           (group == 32 || group == 16 || (fmt != 0 && group == 8));
 }
 
 inline int linear_group(int fmt, int group) { return fmt == 0 ? effective_group(group) : group; }
@@ -33,7 +25,7 @@ size_t linear_workspace_bytes_impl(int fmt, int x_dtype, int64_t M, int64_t N, i
     group = linear_group(fmt, group);
     if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, true, flags))
         return (x_dtype == OJX_BF16 || K % 256 != 0) ? gemm_workspace_bytes_impl(M, N, K) : 256;
-    return fmt == 0 ? gemv_workspace_bytes_impl(M, N, K) : 0;
+    return 0;
 }
 
 int32_t linear_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
@@ -46,7 +38,7 @@ int32_t linear_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint8_
                            reinterpret_cast<uintptr_t>(scales)) & 15) == 0;
     if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, aligned, flags))
         return gemm_fmt_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, ws, ws_bytes, s);
-    if (fmt == 0) return gemv_impl(x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, ws, ws_bytes, s);
+    if (fmt == 0) return gemv_impl(x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, nullptr, kNoScratch, s);
     return linear_lowbit_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, s, nullptr, nullptr, 0);
 }
 

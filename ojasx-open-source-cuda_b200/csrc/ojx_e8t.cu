@@ -9,7 +9,6 @@
 #include "codec1.cuh"
 #include "e8_project.cuh"
 #include "gemv.cuh"
-#include "gemv_a16.cuh"
 #include "gemv_host.cuh"
 #include "gemm_tcgen05.cuh"
 #include "linear_host.cuh"

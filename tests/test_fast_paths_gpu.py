@@ -81,3 +81,62 @@ def test_root_packer_on_ties_zeros_and_non_finite_values(P, oracle, group):
         p_ref, s_ref, _ = oracle.encode_1bit(wt.float().numpy(), group)
         assert (packed.cpu().numpy() == p_ref).all()
         assert (scales.view(torch.int16).cpu().numpy().view("uint16") == s_ref.view("uint16")).all()
+
+
+_DECODE_SHAPES = [(1, 256), (17, 512), (100, 4096), (1000, 4352), (65, 14336), (2500, 8448), (33, 32), (40, 96), (129, 2912), (50, 11040)]
+
+
+@pytest.mark.parametrize("bits,group", [(1.5, 32), (1.5, 16), (2.0, 32), (2.0, 16), (2.0, 8), (1.0, 32), (1.0, 16), (1.0, 8)])
+@pytest.mark.parametrize("n,k", _DECODE_SHAPES)
+def test_decode_kernels_at_the_edges_of_their_tiles(P, bits, group, n, k):
+    """One row of weights, remainders of a tile, one and several chunks of K (clusters that split them), K of any number of 32s."""
+    packed, scales, exact = _problem(P, bits, n, k, group)
+    fmt = {1.0: 1, 1.5: 0, 2.0: 2}[bits]
+    for m in (1, 2, 3, 8, 9, 16):
+        # from four (groups of 32 with K % 2048 == 0: nine) rows on, 2.0-bit weights are rounded to fp16 as in larger batches
+        rounded = bits == 2.0 and k % 256 == 0 and (m > 8 or (m >= 4 and not (group == 32 and k % 2048 == 0)))
+        wd = (exact.half().float() if rounded else exact)
+        for dt in (torch.bfloat16, torch.float16):
+            x = P.ops.generate(m * k, 8 + m, 1.0, dt, torch.device(DEV)).view(m, k).clone()
+            x[:, ::97] *= 30
+            bias = P.ops.generate(n, 9, 0.5, dt, torch.device(DEV))
+            y = P.ops._linear(fmt, x, packed, scales, bias, n, k, group, torch.float32, P._cabi.OJX_LINEAR_DECODE)
+            ref = x.double() @ wd.double().t() + bias.double()
+            bound = x.double().abs() @ wd.double().abs().t() + bias.double().abs()
+            assert float(((y.double() - ref).abs() / bound.clamp_min(1e-30)).max()) <= 5e-6, (m, dt)
+
+
+@pytest.mark.parametrize("bits,group,k", [(2.0, 8, 4096), (2.0, 32, 14336), (1.5, 16, 8192), (1.0, 8, 2080)])
+def test_decode_kernels_keep_non_finite_activations_in_their_row(P, bits, group, k):
+    n, m = 48, 5
+    packed, scales, wd = _problem(P, bits, n, k, group)
+    fmt = {1.0: 1, 1.5: 0, 2.0: 2}[bits]
+    x = P.ops.generate(m * k, 3, 1.0, torch.bfloat16, torch.device(DEV)).view(m, k).clone()
+    x[1] *= 2.0 ** 20
+    x[4] *= 2.0 ** 112
+    x[1, k - 5] = float("inf")
+    x[3, 7] = float("nan")
+    y = P.ops._linear(fmt, x, packed, scales, None, n, k, group, torch.float32, P._cabi.OJX_LINEAR_DECODE)
+    ref = x.float() @ wd.t()
+    assert torch.equal(torch.isnan(y), torch.isnan(ref)) and torch.equal(torch.isinf(y), torch.isinf(ref))
+    for row in (0, 2, 4):
+        assert float((y[row].double() - ref[row].double()).norm() / ref[row].double().norm()) < 1e-3
+
+
+@pytest.mark.parametrize("m", [1, 4, 12])
+def test_grouped_launch_over_many_matrices_of_different_shapes(P, m):
+    """Whole CTAs per matrix (few matrices), an even cut of the cost (many), K of one and of several chunks."""
+    dev = torch.device(DEV)
+    for count in (2, 40, 300):
+        entries, shapes, want = [], [], []
+        for i in range(count):
+            n, k = (48, 256) if count == 300 else (16 * (1 + i % 5) + (i % 3), 256 * (1 + (7 * i) % 19))
+            packed, scales, _ = _problem(P, 1.5, n, k, 32, seed=i)
+            x = P.ops.generate(m * k, 50 + i, 1.0, torch.bfloat16, dev).view(m, k)
+            y = torch.empty((m, n), dtype=torch.bfloat16, device=dev)
+            entries.append((x, packed, scales, None, y))
+            shapes.append((n, k))
+            want.append(P.ops.linear(x, packed, scales, None, n, k, 32))
+        P.ops.GroupedGemv(entries, shapes)()
+        for e, w in zip(entries, want):
+            assert float((e[4].float() - w.float()).norm() / w.float().norm()) <= 4e-3
