@@ -233,7 +233,7 @@ int32_t ojx_e8t_gemv(const void* x, int32_t x_dtype, int64_t M,
 /*
  * ojx_e8t_gemv with the adapter term of E8LatticeLinear.forward_fused (ojasx2/math/lattice.py:826-842) fused into the
  * epilogue: y = x . W^T (+ bias) + lora_t . lora_b, where lora_t [M, lora_rank] fp32 = scaling * (x . A) and lora_b
- * [lora_rank, N] has x's dtype.  Only the tensor-core decode shapes up to eight rows are served (1 <= M <= 8, K % 256 == 0, group 32,
+ * [lora_rank, N] has x's dtype.  Only the tensor-core decode shapes are served (1 <= M <= 16, K % 32 == 0, groups of 16 and 32,
  * 16-bit x, 16-byte aligned buffers, lora_rank <= 64); anything else returns OJX_ERR_UNSUPPORTED and the caller adds
  * the term itself.
  */
@@ -437,6 +437,21 @@ int32_t ojx_e8t_linear(int32_t format, const void* x, int32_t x_dtype, int64_t M
                        int64_t N, int64_t K, int32_t group,
                        void* y, int32_t y_dtype,
                        void* workspace, size_t workspace_bytes, int32_t flags, void* stream);
+
+/*
+ * The packed linear of a layer with a low-rank adapter, up to sixteen rows (E8LatticeLinear.forward_fused,
+ * ojasx2/math/lattice.py:826-842): y = H(x) . W^T (+ bias) + scaling * (x . A) . B with A [K, rank] and B [rank, N] in x's dtype,
+ * H the 32-point transform of ojx_e8t_fwht32 when `hadamard` is set and nothing otherwise; x . A and the sum are kept in fp32.
+ * 16-bit x, 1 <= M <= 16, K % 32 == 0, groups of 16 and 32 (format 1, 2: 8 too), 1 <= rank <= 64, 16-byte aligned x, codes,
+ * scales and workspace; anything else returns OJX_ERR_UNSUPPORTED and the caller adds the term itself.
+ */
+size_t  ojx_e8t_linear_adapter_workspace_bytes(int64_t M, int64_t K, int32_t rank, int32_t hadamard);
+int32_t ojx_e8t_linear_adapter(int32_t format, const void* x, int32_t x_dtype, int64_t M,
+                               const uint8_t* packed, const uint16_t* scales, const void* bias,
+                               int64_t N, int64_t K, int32_t group,
+                               const void* lora_a, const void* lora_b, int32_t rank, float scaling, int32_t hadamard,
+                               void* y, int32_t y_dtype,
+                               void* workspace, size_t workspace_bytes, void* stream);
 
 /*
  * Backward of the packed linear with respect to its input: dX[M, K] = dY[M, N] . W[N, K], W given packed, on the

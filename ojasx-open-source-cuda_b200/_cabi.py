@@ -35,11 +35,12 @@ EXPORTED_SYMBOLS = (
     "ojx_e8t_gemv_grouped", "ojx_e8t_gemv_grouped_peers", "ojx_e8t_gemv_grouped_ex", "ojx_e8t_peer_wait", "ojx_e8t_enable_peer_access", "ojx_e8t_gemm_workspace_bytes", "ojx_e8t_gemm", "ojx_e8t_gemm_lowbit", "ojx_e8t_gemm_status", "ojx_e8t_gemm_dx", "ojx_e8t_gemm_dx_lowbit", "ojx_e8t_gemm_dx_workspace_bytes",
     "ojx_e8t_generate", "ojx_e8t_last_cuda_error", "ojx_e8t_device_status", "ojx_e8t_poll_status", "ojx_e8t_set_wait_limit",
     "ojx_e8t_gemv_static_scratch", "ojx_e8t_gemv_static_scratch_capacity", "ojx_e8t_linear", "ojx_e8t_linear_workspace_bytes",
+    "ojx_e8t_linear_adapter", "ojx_e8t_linear_adapter_workspace_bytes",
 )
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
-    "-shared", "-Xcompiler", "-fPIC", "--split-compile=0",
+    "-shared", "-Xcompiler", "-fPIC",
 ]
 
 _lock = threading.Lock()
@@ -130,6 +131,10 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.ojx_e8t_decode_2bit.argtypes = [vp, vp, i64, i64, i32, i32, vp, vp]
     lib.ojx_e8t_linear_lowbit_lora.restype = i32
     lib.ojx_e8t_linear_lowbit_lora.argtypes = [i32, vp, i32, i64, vp, vp, vp, i64, i64, i32, vp, vp, i32, vp, i32, vp]
+    lib.ojx_e8t_linear_adapter_workspace_bytes.restype = sz
+    lib.ojx_e8t_linear_adapter_workspace_bytes.argtypes = [i64, i64, i32, i32]
+    lib.ojx_e8t_linear_adapter.restype = i32
+    lib.ojx_e8t_linear_adapter.argtypes = [i32, vp, i32, i64, vp, vp, vp, i64, i64, i32, vp, vp, i32, ctypes.c_float, i32, vp, i32, vp, sz, vp]
     lib.ojx_e8t_linear_2bit.restype = i32
     lib.ojx_e8t_linear_2bit.argtypes = [vp, i32, i64, vp, vp, vp, i64, i64, i32, vp, i32, vp]
     lib.ojx_e8t_encode_1bit.restype = i32

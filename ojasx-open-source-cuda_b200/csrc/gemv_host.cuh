@@ -108,10 +108,9 @@ static ojx_e8t_gemv_problem gemv_problem(const void* x, const uint8_t* packed, c
 int32_t gemv_impl(const void* x, int x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
                   const void* bias, int64_t N, int64_t K, int group, void* y, int y_dtype,
                   void* workspace, size_t workspace_bytes, cudaStream_t s,
-                  const float* lora_t, const void* lora_b, int lora_rank) {
+                  const float* lora_t, const void* lora_b, int lora_rank, int overlap) {
     OJX_RETURN_IF(!x || !packed || !scales || !y, OJX_ERR_NULL);
     OJX_RETURN_IF(lora_rank < 0 || lora_rank > 64 || (lora_rank > 0 && (!lora_t || !lora_b)), OJX_ERR_SHAPE);
-    OJX_RETURN_IF(lora_rank > 0 && M > 8, OJX_ERR_UNSUPPORTED);        // the 9-16 row kernels have no registers to spare for it
     OJX_RETURN_IF(M <= 0 || N <= 0 || K <= 0, OJX_ERR_SHAPE);
     OJX_RETURN_IF(dtype_size(x_dtype) == 0 || dtype_size(y_dtype) == 0, OJX_ERR_DTYPE);
     OJX_RETURN_IF(check_arch() != OJX_OK, OJX_ERR_ARCH);
@@ -124,7 +123,7 @@ int32_t gemv_impl(const void* x, int x_dtype, int64_t M, const uint8_t* packed, 
             const size_t need = gemv_workspace_bytes_impl(M, N, K);
             OJX_RETURN_IF(need > 0 && workspace_bytes != kNoScratch && (!workspace || workspace_bytes < need), OJX_ERR_WORKSPACE);
         }
-        return gemv_mma_single(0, gemv_problem(x, packed, scales, bias, y, N, K, lora_t, lora_b, lora_rank), group, M, x_dtype, y_dtype, s);
+        return gemv_mma_single(0, gemv_problem(x, packed, scales, bias, y, N, K, lora_t, lora_b, lora_rank), group, M, x_dtype, y_dtype, overlap, s);
     }
     OJX_RETURN_IF(lora_rank > 0, OJX_ERR_UNSUPPORTED);          // the low-rank epilogue exists in the tensor-core kernels only
     // fp32 activations and other groups: up to eight rows, any power-of-two group from 16, the shared-memory fp32 kernel
@@ -194,7 +193,7 @@ static bool launch_lowbit_gemv(const void* x, int x_dtype, int64_t M, const uint
 // output feature), any shape.
 int32_t linear_lowbit_impl(int bits, const void* x, int x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
                            const void* bias, int64_t N, int64_t K, int group, void* y, int y_dtype, cudaStream_t s,
-                           const float* lora_t, const void* lora_b, int lora_rank) {
+                           const float* lora_t, const void* lora_b, int lora_rank, int overlap) {
     OJX_RETURN_IF(!x || !packed || !scales || !y, OJX_ERR_NULL);
     OJX_RETURN_IF(lora_rank < 0 || lora_rank > 64 || (lora_rank > 0 && (!lora_t || !lora_b)), OJX_ERR_SHAPE);
     OJX_RETURN_IF(M <= 0 || N <= 0 || K <= 0 || group <= 0 || group % 8 != 0, OJX_ERR_SHAPE);
@@ -203,10 +202,10 @@ int32_t linear_lowbit_impl(int bits, const void* x, int x_dtype, int64_t M, cons
     // One row (1.0-bit: two) with groups of 32 and K % 2048 == 0 has int8 kernels that need no scale per weight (28672 x 8192, one
     // row: 36 us against 53); with more rows, and for every other shape, the fp16 tensor-core kernel is the faster one
     // (2.0-bit, two rows of 14336 x 4096: 17 against 20 us, eight rows of 28672 x 8192: 55 against 1550 us).
-    const bool int8_shape = group == 32 && K % 2048 == 0 && M <= (bits == 1 ? 2 : 1);
+    const bool int8_shape = group == 32 && K % 2048 == 0 && K <= 32768 && M <= (bits == 1 ? 2 : 1);
     if (!int8_shape && gemv_mma_ok(bits, M, N, K, group, x_dtype) &&
         ((reinterpret_cast<uintptr_t>(packed) | reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(scales)) & 15) == 0)
-        return gemv_mma_single(bits, gemv_problem(x, packed, scales, bias, y, N, K, lora_t, lora_b, lora_rank), group, M, x_dtype, y_dtype, s);
+        return gemv_mma_single(bits, gemv_problem(x, packed, scales, bias, y, N, K, lora_t, lora_b, lora_rank), group, M, x_dtype, y_dtype, overlap, s);
     // up to eight rows of the 2.0-bit format with groups of 32 and K a multiple of 2048: int8 tensor cores, no table
     if (bits == 2 && M >= 1 && M <= 8 && group == 32 && K % 2048 == 0 && K <= (1 << 20) && N < (1 << 30) &&
         b2_smem_bytes((int)M, 2, (int)K) <= 227 * 1024 &&

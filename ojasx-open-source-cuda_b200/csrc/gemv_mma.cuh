@@ -232,14 +232,12 @@ __device__ __noinline__ float mma_dense_2bit(const ojx_e8t_gemv_problem& P, int 
                         __half2float(__ushort_as_half(P.scales[at / group]));
         acc = fmaf(load_any(P.x, x_dtype, (int64_t)m * P.K + k), w, acc);
     }
+    for (int r = 0; r < P.lora_rank; ++r) acc = fmaf(P.lora_t[m * P.lora_rank + r], load_any(P.lora_b, x_dtype, (int64_t)r * P.N + n), acc);
     return acc;
 }
-
-__device__ __noinline__ float mma_lora_term(const ojx_e8t_gemv_problem& P, int x_dtype, int m, int n) {
-    float acc = 0.f;
-    const float* t = P.lora_t + m * P.lora_rank;
-    for (int r = 0; r < P.lora_rank; ++r) acc = fmaf(t[r], load_any(P.lora_b, x_dtype, (int64_t)r * P.N + n), acc);
-    return acc;
+__device__ __forceinline__ float mma_load16(const void* p, bool f16, int64_t i) {
+    const uint16_t v = __ldg(static_cast<const uint16_t*>(p) + i);
+    return f16 ? __half2float(__ushort_as_half(v)) : __uint_as_float((uint32_t)v << 16);
 }
 
 // Inf / NaN activations of a slice (fed to the int8 MMAs as 0): lane r adds, in fp32, the products of weight row r of the item
@@ -410,6 +408,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
     using F = MmaFmt<FMT, G>;
     using Sh = MmaShape<FMT, G, NB, kRag>;
     constexpr int S = Sh::kStages, D = Sh::kDepth, T = Sh::kTiles, R = Sh::kRows;
+    if constexpr (kI8) { M = 1; x_dtype = OJX_BF16; }                    // known, so that nothing below keeps registers for them
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t base = smem_u32(smem);                                // in a cluster: with this CTA's rank in its upper bits
     MmaCtl* ctl = reinterpret_cast<MmaCtl*>(smem + plan.off_ctl);
@@ -745,10 +744,9 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
             };
 
-            auto finish = [&](float sum, int col, int n, uint32_t bad_rows) {       // bias, low-rank term, store
+            auto finish = [&](float sum, int col, int n, uint32_t bad_rows) {       // bias, store
                 if (FMT == 2 && ((bad_rows >> col) & 1u)) sum = mma_dense_2bit(P, G, x_dtype, col, n);
                 if (P.bias != nullptr) sum += load_any(P.bias, x_dtype, n);
-                if (P.lora_rank > 0) sum += mma_lora_term(P, x_dtype, col, n);
                 const int64_t at = (int64_t)col * (P.ldy > 0 ? P.ldy : N) + n;
                 store_any(P.y, y_dtype, at, sum);
                 if (peers.world > 1) store_peers(peers, P.y, y_dtype, at, sum);
@@ -763,8 +761,15 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                     for (int w = 0; w < q_per; ++w)
                         if (w < act) sum += __uint_as_float(lds_u32(src + w * slot));
                 }
-                for (int o = 1; o < (1 << qs); o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
                 const int n = (b0 + pair * T) * 16 + q_row;
+                // the low-rank term, once per output: the lanes that share one split its ranks (one lane alone took 0.4 us a rank)
+                if (P.lora_rank > 0 && chunk == 0 && q_col < M && n < N) {
+                    const int rank = P.lora_rank;
+#pragma unroll 1
+                    for (int r = q_sub; r < rank; r += 1 << qs)
+                        sum = fmaf(__ldcg(P.lora_t + q_col * rank + r), mma_load16(P.lora_b, xf16, (int64_t)r * N + n), sum);
+                }
+                for (int o = 1; o < (1 << qs); o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
                 if (q_sub != 0 || q_col >= M || n >= N || n >= (b0 + nt) * 16) return;
                 if (chunks > 1) {
                     float* a = acc_sums + (pair * M + q_col) * R + q_row;
@@ -1022,28 +1027,29 @@ inline int mma_cluster_for(int tiles, int chunks) {
 }
 
 template <int FMT, int G>
-static int32_t mma_dispatch(bool rag, const ojx_e8t_gemv_problem& p, int tiles, int M, int x_dtype, int y_dtype, const PeerMap& peers, cudaStream_t s) {
+static int32_t mma_dispatch(bool rag, const ojx_e8t_gemv_problem& p, int tiles, int M, int x_dtype, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s) {
     // 2.0 bits: batches that the tcgen05 kernel took before this one did see the same weights, rounded to fp16 once; smaller ones
     // and K that is no multiple of 256 the exact ones
     const bool rounded = FMT == 2 && !rag && (M > 8 || (M >= 4 && !(G == 32 && p.K % 2048 == 0)));
     const int per = mma_per_chunk(p.K), chunks = mma_chunks(p.K), cluster = mma_cluster_for(tiles, chunks);
     const bool chunked = chunks > 1;
-    if (rag) return M <= 8 ? mma_launch<FMT, G, 1, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, 3, s)
-                           : mma_launch<FMT, G, 2, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, 3, s);
+    if (rag) return M <= 8 ? mma_launch<FMT, G, 1, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s)
+                           : mma_launch<FMT, G, 2, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
     if (FMT == 0 && G == 32 && M == 1 && x_dtype == OJX_BF16)
-        return mma_launch<0, 32, 1, false, false, true>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, 3, s);
-    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, 3, s, rounded)
-                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, 3, s, rounded);
+        return mma_launch<0, 32, 1, false, false, true>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
+    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded)
+                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded);
 }
 
-// One matrix; the caller has checked gemv_mma_ok and the alignment (16 bytes) of x, codes and scales.
-static int32_t gemv_mma_single(int fmt, const ojx_e8t_gemv_problem& p, int group, int64_t M, int x_dtype, int y_dtype, cudaStream_t s) {
+// One matrix; the caller has checked gemv_mma_ok and the alignment (16 bytes) of x, codes and scales.  `overlap` 3: nothing is read
+// before the launch ahead has ended; 1: codes and scales may be (the launch ahead does not write them).
+static int32_t gemv_mma_single(int fmt, const ojx_e8t_gemv_problem& p, int group, int64_t M, int x_dtype, int y_dtype, int overlap, cudaStream_t s) {
     PeerMap peers = peer_map_self();
     peers.host_status = host_status_device_ptr(s);
     if (wait_limit_override() != 0) peers.wait_limit = wait_limit_override();
     const bool rag = p.K % 256 != 0;
     const int tiles = (p.N + 15) / 16, m = (int)M;
-#define OJX_MMA(F, GG) return mma_dispatch<F, GG>(rag, p, tiles, m, x_dtype, y_dtype, peers, s)
+#define OJX_MMA(F, GG) return mma_dispatch<F, GG>(rag, p, tiles, m, x_dtype, y_dtype, peers, overlap, s)
     if (fmt == 0 && group == 32) OJX_MMA(0, 32);
     if (fmt == 0 && group == 16) OJX_MMA(0, 16);
     if (fmt == 2 && group == 32) OJX_MMA(2, 32);

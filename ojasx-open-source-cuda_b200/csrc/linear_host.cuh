@@ -39,7 +39,7 @@ int32_t linear_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint8_
     if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, aligned, flags))
         return gemm_fmt_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, ws, ws_bytes, s);
     if (fmt == 0) return gemv_impl(x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, nullptr, kNoScratch, s);
-    return linear_lowbit_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, s, nullptr, nullptr, 0);
+    return linear_lowbit_impl(fmt, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, s, nullptr, nullptr, 0, 3);
 }
 
 }  // namespace ojx

@@ -12,6 +12,7 @@
 #include "gemv_host.cuh"
 #include "gemm_tcgen05.cuh"
 #include "linear_host.cuh"
+#include "adapter.cuh"
 
 namespace ojx {
 
@@ -130,7 +131,7 @@ int32_t ojx_e8t_decode_2bit(const uint8_t* packed, const uint16_t* scales, int64
 
 int32_t ojx_e8t_linear_2bit(const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
                             const void* bias, int64_t N, int64_t K, int32_t group, void* y, int32_t y_dtype, void* stream) {
-    return ojx::linear_lowbit_impl(2, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, (cudaStream_t)stream, nullptr, nullptr, 0);
+    return ojx::linear_lowbit_impl(2, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, (cudaStream_t)stream, nullptr, nullptr, 0, 3);
 }
 
 int32_t ojx_e8t_encode_1bit(const void* w, int32_t w_dtype, int64_t rows, int64_t cols, int32_t group,
@@ -145,7 +146,7 @@ int32_t ojx_e8t_decode_1bit(const uint8_t* packed, const uint16_t* scales, int64
 
 int32_t ojx_e8t_linear_1bit(const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
                             const void* bias, int64_t N, int64_t K, int32_t group, void* y, int32_t y_dtype, void* stream) {
-    return ojx::linear_lowbit_impl(1, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, (cudaStream_t)stream, nullptr, nullptr, 0);
+    return ojx::linear_lowbit_impl(1, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, (cudaStream_t)stream, nullptr, nullptr, 0, 3);
 }
 
 int32_t ojx_e8t_linear_lowbit_lora(int32_t bits, const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed,
@@ -155,7 +156,7 @@ int32_t ojx_e8t_linear_lowbit_lora(int32_t bits, const void* x, int32_t x_dtype,
     if (bits != 1 && bits != 2) return OJX_ERR_UNSUPPORTED;
     if (lora_rank <= 0) return OJX_ERR_SHAPE;
     return ojx::linear_lowbit_impl(bits, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, (cudaStream_t)stream,
-                                   lora_t, lora_b, lora_rank);
+                                   lora_t, lora_b, lora_rank, 3);
 }
 
 int32_t ojx_e8t_project(const float* x, int64_t vectors, float* out, void* stream) {
@@ -282,6 +283,18 @@ int32_t ojx_e8t_linear(int32_t format, const void* x, int32_t x_dtype, int64_t M
                        void* workspace, size_t workspace_bytes, int32_t flags, void* stream) {
     return ojx::linear_impl(format, x, x_dtype, M, packed, scales, bias, N, K, group, y, y_dtype, workspace, workspace_bytes,
                             flags, (cudaStream_t)stream);
+}
+
+size_t ojx_e8t_linear_adapter_workspace_bytes(int64_t M, int64_t K, int32_t rank, int32_t hadamard) {
+    return ojx::linear_adapter_workspace_bytes_impl(M, K, rank, hadamard);
+}
+
+int32_t ojx_e8t_linear_adapter(int32_t format, const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
+                               const void* bias, int64_t N, int64_t K, int32_t group, const void* lora_a, const void* lora_b,
+                               int32_t rank, float scaling, int32_t hadamard, void* y, int32_t y_dtype,
+                               void* workspace, size_t workspace_bytes, void* stream) {
+    return ojx::linear_adapter_impl(format, x, x_dtype, M, packed, scales, bias, N, K, group, lora_a, lora_b, rank, scaling, hadamard,
+                                    y, y_dtype, workspace, workspace_bytes, (cudaStream_t)stream);
 }
 
 int32_t ojx_e8t_gemm_status(const void* workspace, void* stream) {

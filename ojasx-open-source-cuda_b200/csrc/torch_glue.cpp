@@ -107,6 +107,43 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     END_HANDLE_TH_ERRORS
 }
 
+// linear_adapter(fmt, x, packed, scales, bias, n, k, group, y_dtype, hadamard, lora_a, lora_b, scaling) -> y [..., n]; decode shapes
+PyObject* py_linear_adapter(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    OJX_ARGS(13);
+    const int fmt = (int)a.i(0);
+    const at::Tensor *x = a.t(1), *pk = a.t(2), *sc = a.t(3), *bias = args[4] == Py_None ? nullptr : a.t(4), *la = a.t(10), *lb = a.t(11);
+    const int64_t n = a.i(5), k = a.i(6);
+    const int group = (int)a.i(7), yd = (int)a.i(8), hadamard = args[9] == Py_True && k % 32 == 0;
+    const double scaling = PyFloat_AsDouble(args[12]);
+    if (PyErr_Occurred()) { PyErr_Clear(); Py_RETURN_NONE; }
+    if (!a.ok || !plain(x) || x->dim() < 1 || n <= 0 || k <= 0 || x->size(-1) != k || x->numel() == 0 || x->numel() / k > 16) Py_RETURN_NONE;
+    const c10::Device dev = x->device();
+    const at::ScalarType xt = x->scalar_type();
+    const int xd = dtype_code(xt);
+    if ((xd != OJX_BF16 && xd != OJX_F16) || !packed_pair(pk, sc, dev)) Py_RETURN_NONE;
+    if (args[4] != Py_None && (!plain(bias) || bias->device() != dev || bias->scalar_type() != xt || bias->numel() != n)) Py_RETURN_NONE;
+    if (!plain(la) || !plain(lb) || la->device() != dev || lb->device() != dev || la->scalar_type() != xt || lb->scalar_type() != xt ||
+        la->dim() != 2 || lb->dim() != 2 || la->size(0) != k || lb->size(1) != n || la->size(1) != lb->size(0))
+        Py_RETURN_NONE;
+    if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
+    const c10::cuda::CUDAGuard guard(dev);
+    const int64_t m = x->numel() / k;
+    const int rank = (int)la->size(1);
+    const size_t need = ojx_e8t_linear_adapter_workspace_bytes(m, k, rank, hadamard);
+    if (need == 0) Py_RETURN_NONE;
+    c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
+    sizes.back() = n;
+    const int y_code = yd < 0 ? xd : yd;
+    at::Tensor y = empty(sizes, scalar_type(y_code), dev), ws = empty({(int64_t)need}, at::kByte, dev);
+    const int32_t st = ojx_e8t_linear_adapter(fmt, data(*x), xd, m, static_cast<const uint8_t*>(data(*pk)), static_cast<const uint16_t*>(data(*sc)),
+                                              bias ? data(*bias) : nullptr, n, k, group, data(*la), data(*lb), rank, (float)scaling, hadamard,
+                                              data(y), y_code, data(ws), need, stream_of(dev));
+    if (st == OJX_ERR_UNSUPPORTED) Py_RETURN_NONE;
+    return status_or(st, std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
 // linear_dx(fmt, grad_y [m, n], packed, scales, n, k, group, out_dtype) -> dx [m, k]; 16-bit gradients
 PyObject* py_linear_dx(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
@@ -224,7 +261,7 @@ PyObject* py_grouped(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 #define OJX_METHOD(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {OJX_METHOD(linear), OJX_METHOD(linear_dx), OJX_METHOD(encode), OJX_METHOD(decode), OJX_METHOD(fwht32),
+PyMethodDef methods[] = {OJX_METHOD(linear), OJX_METHOD(linear_adapter), OJX_METHOD(linear_dx), OJX_METHOD(encode), OJX_METHOD(decode), OJX_METHOD(fwht32),
                          OJX_METHOD(grouped), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ojx_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -350,50 +350,59 @@ class E8LatticeLinear(nn.Module):
                                                          (self.out_features, self.in_features), dtype=dtype)
         return fwht_block32(w) if self.use_hadamard else w
 
+    def _adapter(self, x: torch.Tensor) -> Tuple[torch.Tensor, torch.Tensor]:
+        a, b = self.lora_A, self.lora_B
+        return (a if a.dtype == x.dtype else a.to(x.dtype)), (b if b.dtype == x.dtype else b.to(x.dtype))
+
     def _forward_decode_with_adapter(self, x: torch.Tensor) -> Optional[torch.Tensor]:
-        """Inference at decode shapes with an adapter: the low-rank term rides in the GEMV's epilogue (one launch for
-        the packed product, the adapter's second factor, the scaling and the addition); ``None`` when it does not apply."""
-        if self.rank <= 0 or self.lora_A is None or not x.is_cuda or torch.compiler.is_compiling():
+        """Inference at decode shapes with an adapter: one native call, the low-rank term in the decode kernel's epilogue;
+        ``None`` when it does not apply."""
+        if self.lora_A is None or self.lora_B is None or not x.is_cuda or x.shape[-1] != self.in_features:
             return None
-        if torch.is_grad_enabled() and (x.requires_grad or self.lora_A.requires_grad or self.lora_B.requires_grad
-                                        or (self.bias is not None and self.bias.requires_grad)):
+        rows = x.numel() // self.in_features
+        if rows > 16:
             return None
-        x_2d = x.reshape(-1, self.in_features)
-        if self.bitrate != 1.5:                          # the sibling formats: their int8 tensor-core decode kernels
-            if not ops.lowbit_lora_fusable(int(x_2d.shape[0]), self.in_features, self.group_size, self.rank):
-                return None
-            t = (x_2d @ self.lora_A.to(x.dtype)).float() * self.scaling
-            x_rot = fwht_block32(x_2d) if (self.use_hadamard and self.in_features % 32 == 0) else x_2d
-            y = ops.linear_lowbit_lora(_lowbit(self.bitrate), x_rot, self.packed_weight, self.block_scales, self.bias,
-                                       self.out_features, self.in_features, self.group_size, t, self.lora_B)
-            return y.reshape(*x.shape[:-1], self.out_features)
-        if not ops.lora_fusable(int(x_2d.shape[0]), self.in_features, self.group_size, x.dtype, self.rank):
-            return None
-        t = (x_2d @ self.lora_A.to(x.dtype)).float() * self.scaling
-        x_rot = fwht_block32(x_2d) if self.use_hadamard else x_2d
-        y = ops.linear_lora(x_rot, self.packed_weight, self.block_scales, self.bias, self.out_features, self.in_features,
-                            self.group_size, t, self.lora_B)
+        lora_a, lora_b = self._adapter(x)
+        adapter = dict(lora_a=lora_a, scaling=self.scaling, hadamard=self.use_hadamard)
+        if self.bitrate == 1.5 and ops.lora_fusable(rows, self.in_features, self.group_size, x.dtype, self.rank):
+            y = ops.linear_lora(x, self.packed_weight, self.block_scales, self.bias, self.out_features, self.in_features,
+                                self.group_size, None, lora_b, **adapter)
+        elif self.bitrate != 1.5 and ops.lowbit_lora_fusable(rows, self.in_features, self.group_size, self.rank):
+            y = ops.linear_lowbit_lora(_lowbit(self.bitrate), x, self.packed_weight, self.block_scales, self.bias,
+                                       self.out_features, self.in_features, self.group_size, None, lora_b, **adapter)
+        else:                                            # nine to sixteen rows, other groups, K of any number of 32s
+            return ops.layer_forward_adapter(_FORMATS[self.bitrate], x, self.packed_weight, self.block_scales, self.bias, self.out_features,
+                                             self.in_features, self.group_size, self.use_hadamard, lora_a, lora_b, self.scaling)
         return y.reshape(*x.shape[:-1], self.out_features)
 
     def forward_fused(self, x: torch.Tensor) -> torch.Tensor:
-        if self.rank == 0 and not torch.compiler.is_compiling():
-            bias = self._parameters["bias"]
-            if not torch.is_grad_enabled() or not (x.requires_grad or (bias is not None and bias.requires_grad)):
-                # nothing to differentiate: one native call, no autograd node
-                b = self._buffers
-                y = ops.layer_forward(_FORMATS[self.bitrate], x, b["packed_weight"], b["block_scales"], bias, self.out_features,
-                                      self.in_features, self.group_size, self.use_hadamard)
-                if y is not None:
-                    return y
-        fused = self._forward_decode_with_adapter(x)
-        if fused is not None:
-            return fused
-        out = _FusedE8GEMMFunction.apply(x, self.packed_weight, self.block_scales, self.bias, self.out_features,
-                                         self.in_features, self.group_size, self.bitrate, self.use_hadamard)
-        if self.rank > 0 and self.lora_A is not None and self.lora_B is not None:
-            lora_a = self.lora_A.to(x.dtype) if self.lora_A.dtype != x.dtype else self.lora_A
-            lora_b = self.lora_B.to(x.dtype) if self.lora_B.dtype != x.dtype else self.lora_B
-            out = out + self.scaling * ((x @ lora_a) @ lora_b)
+        params = self._parameters
+        bias, with_adapter = params["bias"], self.rank > 0 and params["lora_A"] is not None and params["lora_B"] is not None
+        out = None
+        if not torch.compiler.is_compiling() and not (
+                torch.is_grad_enabled() and (x.requires_grad or any(p is not None and p.requires_grad for p in params.values()))):
+            # nothing to differentiate: one native call, no autograd node
+            if with_adapter:
+                out = self._forward_decode_with_adapter(x)
+                if out is not None:
+                    return out
+            b = self._buffers
+            out = ops.layer_forward(_FORMATS[self.bitrate], x, b["packed_weight"], b["block_scales"], bias, self.out_features,
+                                    self.in_features, self.group_size, self.use_hadamard)
+        own = out is not None
+        if not own:
+            out = _FusedE8GEMMFunction.apply(x, self.packed_weight, self.block_scales, self.bias, self.out_features,
+                                             self.in_features, self.group_size, self.bitrate, self.use_hadamard)
+        if with_adapter:
+            lora_a, lora_b = self._adapter(x)
+            if out.dtype != x.dtype or torch.is_autocast_enabled():
+                return out + self.scaling * ((x @ lora_a) @ lora_b)
+            # scaling and sum inside the second product: no passes over the output of their own
+            low, flat = x.reshape(-1, self.in_features) @ lora_a, out.reshape(-1, self.out_features)
+            if own:
+                flat.addmm_(low, lora_b, alpha=self.scaling)
+            else:
+                out = torch.addmm(flat, low, lora_b, alpha=self.scaling).reshape(out.shape)
         return out
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:

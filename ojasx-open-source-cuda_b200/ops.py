@@ -203,6 +203,23 @@ def layer_forward(fmt: int, x: torch.Tensor, packed: torch.Tensor, scales: torch
     return _result(y, "ojx_e8t_linear")
 
 
+def layer_forward_adapter(fmt: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor], n: int, k: int,
+                          group_size: int, hadamard: bool, lora_a: torch.Tensor, lora_b: torch.Tensor, scaling: float,
+                          out_dtype: Optional[torch.dtype] = None) -> Optional[torch.Tensor]:
+    """:func:`layer_forward` of a layer with an adapter, up to sixteen rows: ``+ scaling * (x . A) . B`` in the same native call
+    (``ojx_e8t_linear_adapter``); ``None`` for operands or shapes it does not take."""
+    y = _cabi.glue().linear_adapter(fmt, x, packed, scales, bias, n, k, group_size, -1 if out_dtype is None else _dtype_code(out_dtype),
+                                    hadamard, lora_a, lora_b, scaling)
+    return None if y is None else _result(y, "ojx_e8t_linear_adapter")
+
+
+def _adapter_parts(x: torch.Tensor, lora_a: torch.Tensor, scaling: float, hadamard: bool) -> Tuple[torch.Tensor, torch.Tensor]:
+    """``scaling * (x . A)`` in fp32 and the x that the packed product takes, by tensor operations."""
+    x2 = x.reshape(-1, x.shape[-1])
+    t = (x2 @ lora_a.to(x.dtype)).float() * scaling
+    return t, (fwht32(x2) if hadamard else x2)
+
+
 def lowbit_lora_fusable(m: int, k: int, group_size: int, rank: int) -> bool:
     """Shapes for which the adapter term can ride in the epilogue of the 2.0-bit / 1.0-bit decode kernels
     (``ojx_e8t_linear_lowbit_lora``)."""
@@ -210,10 +227,17 @@ def lowbit_lora_fusable(m: int, k: int, group_size: int, rank: int) -> bool:
 
 
 def linear_lowbit_lora(bits: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor],
-                       n: int, k: int, group_size: int, lora_t: torch.Tensor, lora_b: torch.Tensor,
-                       out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+                       n: int, k: int, group_size: int, lora_t: Optional[torch.Tensor], lora_b: torch.Tensor,
+                       out_dtype: Optional[torch.dtype] = None, *, lora_a: Optional[torch.Tensor] = None, scaling: float = 1.0,
+                       hadamard: bool = False) -> torch.Tensor:
     """``y = x . W^T (+ bias) + lora_t . lora_b`` for the 2.0-bit (``bits`` 2) or 1.0-bit (``bits`` 1) format in ONE
-    decode-shape launch; ``lora_t`` [M, r] fp32 is ``scaling * (x . A)``, ``lora_b`` [r, N]."""
+    decode-shape launch; ``lora_t`` [M, r] fp32 is ``scaling * (x . A)``, ``lora_b`` [r, N].  With ``lora_a`` in place of
+    ``lora_t`` (``None``) the library computes it, and rotates x for the packed product when ``hadamard`` is set."""
+    if lora_t is None:
+        y = layer_forward_adapter(bits, x, packed, scales, bias, n, k, group_size, hadamard, lora_a, lora_b, scaling, out_dtype)
+        if y is not None:
+            return y
+        lora_t, x = _adapter_parts(x, lora_a, scaling, hadamard)
     dev = _require_cuda(x, packed, scales)
     x2 = x.detach().reshape(-1, k).contiguous()
     m, r = int(x2.shape[0]), int(lora_b.shape[0])
@@ -409,12 +433,19 @@ def lora_fusable(m: int, k: int, group_size: int, dtype: torch.dtype, rank: int)
 
 
 def linear_lora(x2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor],
-                out_features: int, in_features: int, group_size: int, lora_t: torch.Tensor, lora_b: torch.Tensor,
-                out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
+                out_features: int, in_features: int, group_size: int, lora_t: Optional[torch.Tensor], lora_b: torch.Tensor,
+                out_dtype: Optional[torch.dtype] = None, *, lora_a: Optional[torch.Tensor] = None, scaling: float = 1.0,
+                hadamard: bool = False) -> torch.Tensor:
     """``y = x . dequant(W)^T (+ bias) + lora_t . lora_b`` in ONE decode-shape launch: ``lora_t`` [M, r] fp32 is
     ``scaling * (x . A)``, ``lora_b`` [r, N]; the low-rank term is accumulated in fp32 in the kernel's epilogue
-    (the reference adds it with three more tensor operations, ``ojasx2/math/lattice.py:839-842``)."""
+    (the reference adds it with three more tensor operations, ``ojasx2/math/lattice.py:839-842``).  With ``lora_a`` in
+    place of ``lora_t`` (``None``) the library computes it, and rotates x for the packed product when ``hadamard`` is set."""
     n, k = int(out_features), int(in_features)
+    if lora_t is None:
+        y = layer_forward_adapter(0, x2d, packed, scales, bias, n, k, group_size, hadamard, lora_a, lora_b, scaling, out_dtype)
+        if y is not None:
+            return y
+        lora_t, x2d = _adapter_parts(x2d, lora_a, scaling, hadamard)
     dev, x2d, pk, sc, b = _prep_linear(x2d, packed, scales, bias, n, k)
     _cabi.raise_pending()
     m, r = int(x2d.shape[0]), int(lora_b.shape[0])

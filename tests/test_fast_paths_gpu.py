@@ -140,3 +140,41 @@ def test_grouped_launch_over_many_matrices_of_different_shapes(P, m):
         P.ops.GroupedGemv(entries, shapes)()
         for e, w in zip(entries, want):
             assert float((e[4].float() - w.float()).norm() / w.float().norm()) <= 4e-3
+
+
+@pytest.mark.parametrize("bits,group,n,k,rank,had", [(1.5, 32, 72, 4096, 16, True), (1.5, 16, 33, 96, 3, True), (2.0, 8, 40, 2912, 8, False),
+                                                     (2.0, 32, 64, 2048, 64, True), (1.0, 32, 48, 8192, 17, False), (1.0, 16, 100, 320, 1, True)])
+def test_adapter_layer_at_decode_shapes_in_one_call(P, bits, group, n, k, rank, had):
+    """Ranks that fill a slab of sixteen columns, less and more; K of less than one group per CTA; every row count of a block."""
+    dev = torch.device(DEV)
+    for dt in (torch.bfloat16, torch.float16):
+        lin = torch.nn.Linear(k, n, bias=True).to(dev).to(dt)
+        layer = P.E8LatticeLinear.from_linear(lin, rank=rank, bitrate=bits, group_size=group, use_hadamard=had).requires_grad_(False)
+        layer.lora_B.copy_(torch.randn_like(layer.lora_B) * 0.1)
+        wd = layer.unpack_weights(torch.float32).double()
+        for m in (1, 2, 4, 5, 8, 9, 16):
+            x = P.ops.generate(m * k, 8 + m, 1.0, dt, dev).view(1, m, k)
+            y = P.ops.layer_forward_adapter({1.0: 1, 1.5: 0, 2.0: 2}[bits], x, layer.packed_weight, layer.block_scales, layer.bias, n, k, group,
+                                            had, layer.lora_A, layer.lora_B, layer.scaling, torch.float32)
+            assert y is not None and y.shape == (1, m, n)
+            low = layer.scaling * ((x.double() @ layer.lora_A.double()) @ layer.lora_B.double())
+            ref = x.double() @ wd.t() + layer.bias.double() + low
+            assert float((y.double() - ref).norm() / ref.norm()) < (5e-3 if had and dt == torch.bfloat16 else 1.5e-3), (dt, m)
+            assert float((layer(x).double() - ref).norm() / ref.norm()) < 8e-3, (dt, m)
+
+
+def test_adapter_layer_on_a_batch_of_tokens(P):
+    dev = torch.device(DEV)
+    lin = torch.nn.Linear(512, 264, bias=True).to(dev).to(torch.bfloat16)
+    layer = P.E8LatticeLinear.from_linear(lin, rank=8, bitrate=1.5, group_size=32)
+    with torch.no_grad():
+        layer.lora_B.copy_(torch.randn_like(layer.lora_B) * 0.1)
+    x = torch.randn(2, 20, 512, device=dev).to(torch.bfloat16)
+    ref = (x.double() @ layer.unpack_weights(torch.float32).double().t() + layer.bias.double()
+           + layer.scaling * ((x.double() @ layer.lora_A.double()) @ layer.lora_B.double()))
+    with torch.no_grad():
+        y = layer(x)
+    y_grad = layer(x)
+    assert y.shape == y_grad.shape == (2, 20, 264) and y_grad.requires_grad
+    for v in (y, y_grad):
+        assert float((v.double() - ref).norm() / ref.norm()) < 8e-3
