@@ -49,7 +49,7 @@ constexpr int kGemmDecoderWarps = 8;
 constexpr uint32_t kXStageBytes = kGemmBN * kGemmBK * 2;      // 32768
 constexpr uint32_t kAStageBytes = kGemmBM * kGemmBK * 2;      // 32768 (rows 0-127, then rows 128-255)
 constexpr int kGemmDigitCopies = 16;
-constexpr uint32_t kGemmLutBytes = 16384;                     // digit table: 81 x 16 copies x 8 bytes = 10368; a corrupt rank (up to 4095) stays inside
+constexpr uint32_t kGemmLutBytes = 32768;                     // 1.0-bit table: 256 x 8 copies x 16 bytes; digit table: 81 x 16 x 8 = 10368, a corrupt rank (up to 4095) stays inside
 constexpr uint32_t kGemmSmemBytes = kGemmStages * (kXStageBytes + kAStageBytes) + kGemmLutBytes + 256 + 1024;
 
 struct GemmParams {
@@ -277,6 +277,27 @@ __device__ __noinline__ void gemm_drain_tile(void* __restrict__ y, int y_dtype, 
     }
 }
 
+// Eight 2-bit codes (the low or high half of a word) as four fp16 pairs code - 1.5, without a table: a code placed at bit 4 or 8 of the
+// mantissa of 1024.0 makes 1024 + 16 c or 1024 + 256 c, and one fused multiply-add leaves c - 1.5 exactly.  The kernel is bound by
+// shared-memory bandwidth (a stage writes and reads 160 KB at 128 B per clock); table reads added 48 KB to that
+// (2048 tokens, 14336 x 4096 weight: 236 -> 200 us).
+__device__ __forceinline__ void codes_2bit_f16(uint32_t word, int high, uint2& lo, uint2& hi) {
+    uint32_t v, p[4];                                            // even codes at their bits of the low half, odd ones 14 bits further up
+    if (high) v = (word >> 16) | ((word >> 2) & 0xFFFF0000u);
+    else v = (word & 0xFFFFu) | (word << 14);
+    const uint32_t a = v << 4, b = v >> 4;
+    asm("lop3.b32 %0, %1, 0x00300030, 0x64006400, 0xEA;" : "=r"(p[0]) : "r"(a));        // (x & mask) | 1024.0
+    asm("lop3.b32 %0, %1, 0x03000300, 0x64006400, 0xEA;" : "=r"(p[1]) : "r"(a));
+    asm("lop3.b32 %0, %1, 0x00300030, 0x64006400, 0xEA;" : "=r"(p[2]) : "r"(b));
+    asm("lop3.b32 %0, %1, 0x03000300, 0x64006400, 0xEA;" : "=r"(p[3]) : "r"(b));
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if (i & 1) asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(p[i]) : "r"(0x1C001C00u), "r"(0xC580C580u));   // / 256 - 5.5
+        else asm("fma.rn.f16x2 %0, %0, %1, %2;" : "+r"(p[i]) : "r"(0x2C002C00u), "r"(0xD418D418u));         // / 16 - 65.5
+    }
+    lo = make_uint2(p[0], p[1]);
+    hi = make_uint2(p[2], p[3]);
+}
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     const __half2 v = __hmul2(*reinterpret_cast<const __half2*>(&a), *reinterpret_cast<const __half2*>(&b));
     return *reinterpret_cast<const uint32_t*>(&v);
@@ -321,19 +342,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             for (int k = 0; k < 4; ++k) { const int d = e % 3; e /= 3; h[k] = d == 0 ? 0xBC00u : (d == 1 ? 0u : 0x3C00u); }
             reinterpret_cast<uint2*>(lut)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
         }
-    } else if constexpr (kFmt == 2) {
-        // 2.0-bit format: a code byte (four codes, code j in bits 2j) -> four fp16 values code - 1.5, eight interleaved copies
+    } else if constexpr (kFmt == 1) {
+        // 1.0-bit format: a code -> its eight coordinates (0, +-1, +-2) as fp16, eight interleaved copies (one per lane of the quarter warp
+        // that a 128-bit read serves at a time: with four, every second read met another one in its banks)
         for (int i = tid; i < 256 * 8; i += kGemmThreads) {
             const int e = i >> 3;
-            uint32_t h[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) { const int c = (e >> (2 * k)) & 3; h[k] = c == 0 ? 0xBE00u : (c == 1 ? 0xB800u : (c == 2 ? 0x3800u : 0x3E00u)); }
-            reinterpret_cast<uint2*>(lut)[i] = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16));
-        }
-    } else {
-        // 1.0-bit format: a code -> its eight coordinates (0, +-1, +-2) as fp16, four interleaved copies
-        for (int i = tid; i < 256 * 4; i += kGemmThreads) {
-            const int e = i >> 2;
             const uint32_t cw[2] = {g_root_coords[2 * e], g_root_coords[2 * e + 1]};
             uint32_t h[8];
 #pragma unroll
@@ -442,9 +455,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             // eight ranks = 12 bytes of codes and two scales, each rank one 16-byte chunk of the MN-major tile.
             const int r = (warp - 4) * 32 + lane;
             const int j = r & 63, kq = r >> 6;
-            // (the sibling formats: 16 or 8 bytes of codes; one or two reads of their table per 8 weights)
+            // (the sibling formats: 16 bytes of codes and no table, or 8 bytes and one read of their table per 8 weights)
             const uint8_t* digit_lane = reinterpret_cast<const uint8_t*>(lut) +
-                                        (kFmt == 0 ? (lane & (kGemmDigitCopies - 1)) * 8 : (kFmt == 2 ? (lane & 7) * 8 : (lane & 3) * 16));
+                                        (kFmt == 0 ? (lane & (kGemmDigitCopies - 1)) * 8 : (lane & 7) * 16);
             constexpr int kWords = kFmt == 0 ? 3 : (kFmt == 2 ? 4 : 2);            // 32-bit words of codes per 64 columns
             constexpr int kSW = 32 / kG;                                           // 32-bit words of scales per 64 columns
             const int64_t row_bytes = kFmt == 0 ? (int64_t)p.N * 3 / 16 : (kFmt == 2 ? p.N / 4 : p.N / 8), row_scales = p.N / kG;
@@ -459,8 +472,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                     const int row = kb * kGemmBK + j;
                     if (row < p.K && col0 < p.N) {
                         const uint32_t* cp = reinterpret_cast<const uint32_t*>(cbase + (int64_t)row * row_bytes);
-#pragma unroll
-                        for (int i = 0; i < kWords; ++i) cw[i] = __ldg(cp + i);
+                        if constexpr (kFmt == 2) { const uint4 v = __ldg(reinterpret_cast<const uint4*>(cp)); cw[0] = v.x; cw[1] = v.y; cw[2] = v.z; cw[3] = v.w; }
+                        else if constexpr (kFmt == 1) { const uint2 v = __ldg(reinterpret_cast<const uint2*>(cp)); cw[0] = v.x; cw[1] = v.y; }
+                        else { cw[0] = __ldg(cp); cw[1] = __ldg(cp + 1); cw[2] = __ldg(cp + 2); }
 #pragma unroll
                         for (int i = 0; i < kSW; ++i) sw[i] = __ldg(reinterpret_cast<const uint32_t*>(sbase + (int64_t)row * row_scales) + i);
                     } else if (kFmt == 0) {                                      // beyond the matrix: rank of the zero vector, scale 0
@@ -473,14 +487,24 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                         for (int i = 0; i < kSW; ++i) sw[i] = 0u;
                     }
                 };
-                uint32_t nw[4] = {0u, 0u, 0u, 0u}, ns[kSW];
-                fetch(0, nw, ns);
-                for (int kb = 0; kb < k_blocks && ok; ++kb, ++it) {
-                    uint32_t cw[4] = {nw[0], nw[1], nw[2], kWords == 4 ? nw[3] : 0u};
+                // Words of the next kAhead stages are on their way: rows lie far apart, so every read is a trip to L2 or DRAM of its
+                // own, and one stage ahead (0.7 us) did not cover it (1024 rows, 4096 x 14336 weight, 2.0 bits: 199 us, with three
+                // ahead and without the table 121).  Ternary codes, three words a read, are faster with one (256 against 270 us).
+                constexpr int kAhead = kFmt == 0 ? 1 : 3;
+                uint32_t nw[kAhead][4], ns[kAhead][kSW];
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u)
+                    if (u < k_blocks) fetch(u, nw[u], ns[u]);
+                for (int kb0 = 0; kb0 < k_blocks && ok; kb0 += kAhead)
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u, ++it) {
+                    const int kb = kb0 + u;
+                    if (kb >= k_blocks) break;
+                    uint32_t cw[4] = {nw[u][0], nw[u][1], kWords > 2 ? nw[u][2] : 0u, kWords == 4 ? nw[u][3] : 0u};
                     uint32_t sw[kSW];
 #pragma unroll
-                    for (int i = 0; i < kSW; ++i) sw[i] = ns[i];
-                    if (kb + 1 < k_blocks) fetch(kb + 1, nw, ns);                // the next stage's words travel during this one's decode
+                    for (int i = 0; i < kSW; ++i) sw[i] = ns[u][i];
+                    if (kb + kAhead < k_blocks) fetch(kb + kAhead, nw[u], ns[u]);
                     const int s = it % kGemmStages;
                     const uint32_t ph = (it / kGemmStages) & 1u;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, 4)) { ok = false; break; }
@@ -501,12 +525,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                                 const uint32_t u = R - 81u * v;
                                 lo8[q] = *reinterpret_cast<const uint2*>(digit_lane + u * (kGemmDigitCopies * 8));
                                 hi8[q] = *reinterpret_cast<const uint2*>(digit_lane + v * (kGemmDigitCopies * 8));
-                            } else if constexpr (kFmt == 2) {            // two code bytes: codes 0-3 and 4-7 of the chunk
-                                const uint32_t word = cw[c >> 1];
-                                lo8[q] = *reinterpret_cast<const uint2*>(digit_lane + prmt(word, 0u, 0x4440u | (uint32_t)(2 * (c & 1))) * 64u);
-                                hi8[q] = *reinterpret_cast<const uint2*>(digit_lane + prmt(word, 0u, 0x4440u | (uint32_t)(2 * (c & 1) + 1)) * 64u);
+                            } else if constexpr (kFmt == 2) {
+                                codes_2bit_f16(cw[c >> 1], c & 1, lo8[q], hi8[q]);
                             } else {                                     // one code byte
-                                const uint4 e = *reinterpret_cast<const uint4*>(digit_lane + prmt(cw[c >> 2], 0u, 0x4440u | (uint32_t)(c & 3)) * 64u);
+                                const uint4 e = *reinterpret_cast<const uint4*>(digit_lane + prmt(cw[c >> 2], 0u, 0x4440u | (uint32_t)(c & 3)) * 128u);
                                 lo8[q] = make_uint2(e.x, e.y);
                                 hi8[q] = make_uint2(e.z, e.w);
                             }
@@ -528,10 +550,10 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             }
         } else if constexpr (kFmt != 0) {
         // The sibling formats: thread r owns weight row r of the tile; 256 k are 64 (2.0-bit) or 32 (1.0-bit) bytes of
-        // codes and eight scales; every 8 weights are one table read (two for 2 bits) and four packed multiplies.
+        // codes and eight scales; every 8 weights are one table read (2.0-bit: arithmetic) and four packed multiplies.
         const int r = (warp - 4) * 32 + lane;
         constexpr int kVec = kFmt == 2 ? 4 : 2;          // 16-byte vectors of codes per 256 k
-        const uint8_t* tab_lane = reinterpret_cast<const uint8_t*>(lut) + (kFmt == 2 ? (lane & 7) * 8 : (lane & 3) * 16);   // entry stride 64 B
+        const uint8_t* tab_lane = reinterpret_cast<const uint8_t*>(lut) + (lane & 7) * 16;   // 1.0-bit: entry stride 128 B
         uint32_t it = 0;
         bool ok = true;
         constexpr int kSV = 32 / kG;                     // 16-byte vectors of scales per 256 k
@@ -572,13 +594,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
 #pragma unroll
                         for (int j = 0; j < 4; ++j) {
                             const int jj = half * 4 + j;                           // chunk of the stage: k = 64 q + 8 jj ..
-                            if constexpr (kFmt == 2) {                             // two code bytes
-                                const uint32_t word = cw[4 * q + (jj >> 1)];
-                                lo8[j] = *reinterpret_cast<const uint2*>(tab_lane + prmt(word, 0u, 0x4440u | (uint32_t)(2 * (jj & 1))) * 64u);
-                                hi8[j] = *reinterpret_cast<const uint2*>(tab_lane + prmt(word, 0u, 0x4440u | (uint32_t)(2 * (jj & 1) + 1)) * 64u);
+                            if constexpr (kFmt == 2) {
+                                codes_2bit_f16(cw[4 * q + (jj >> 1)], jj & 1, lo8[j], hi8[j]);
                             } else {                                               // one code byte
                                 const uint32_t word = cw[2 * q + (jj >> 2)];
-                                const uint4 e = *reinterpret_cast<const uint4*>(tab_lane + prmt(word, 0u, 0x4440u | (uint32_t)(jj & 3)) * 64u);
+                                const uint4 e = *reinterpret_cast<const uint4*>(tab_lane + prmt(word, 0u, 0x4440u | (uint32_t)(jj & 3)) * 128u);
                                 lo8[j] = make_uint2(e.x, e.y);
                                 hi8[j] = make_uint2(e.z, e.w);
                             }
