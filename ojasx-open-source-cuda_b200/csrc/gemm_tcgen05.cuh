@@ -453,8 +453,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
         if constexpr (kDX) {
             // Thread (j, kq) of a stage decodes weight row kb*64 + j, columns [64 kq, 64 kq + 64) of the tile's column range:
             // eight ranks = 12 bytes of codes and two scales, each rank one 16-byte chunk of the MN-major tile.
-            const int r = (warp - 4) * 32 + lane;
-            const int j = r & 63, kq = r >> 6;
+            // A warp takes eight rows and all their columns (tiles of 128: sixteen rows), so that one read of codes or scales touches
+            // eight lines of memory, not 32 (L1 serves a line at a time on the port that shared memory is bound by: 2048 tokens, 14336 x
+            // 4096 weight, ternary: 257 -> 190 us),
+            // and eight consecutive lanes still store to eight different 16-byte columns.
+            const bool wide = p.rows == kGemmBM;
+            const int j = (wide ? (warp - 4) * 8 : (warp - 4) * 16 + (lane >> 4) * 8) + (lane & 7), kq = wide ? lane >> 3 : (lane >> 3) & 1;
             // (the sibling formats: 16 bytes of codes and no table, or 8 bytes and one read of their table per 8 weights)
             const uint8_t* digit_lane = reinterpret_cast<const uint8_t*>(lut) +
                                         (kFmt == 0 ? (lane & (kGemmDigitCopies - 1)) * 8 : (lane & 7) * 16);
