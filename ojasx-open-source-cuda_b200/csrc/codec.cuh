@@ -237,7 +237,7 @@ template <> __device__ __forceinline__ uint32_t decode_scale_bits<__nv_bfloat16>
 }
 
 // A weight is 0, +scale or -scale, so its 16-bit pattern is assembled from the bytes of the scale with byte permutes
-// (two weights per permute; selectors from a table) instead of being computed: about seven
+// (two weights per permute; selectors from the table the GEMV uses) instead of being computed: about seven
 // instructions per weight became about three, which leaves the kernel to the memory system.  Two variants that were
 // measured and lost (145 and 137 us against 132 us for 28672 x 8192 to fp16): one 16-byte output chunk per lane, so
 // that every store instruction writes whole 32-byte sectors, and the same with four chunks in flight per thread.
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(256) decode_kernel(const uint8_t* __restrict__
                                                       const uint16_t* __restrict__ scales, int64_t total,
                                                       int group, T* __restrict__ out) {
     __shared__ uint2 lut[kNumPoints];                       // rank -> four 16-bit permute selectors (26 KB)
-    for (int i = threadIdx.x; i < kNumPoints; i += blockDim.x) lut[i] = reinterpret_cast<const uint2*>(g_lut_f16sel)[i];
+    for (int i = threadIdx.x; i < kNumPoints; i += blockDim.x) lut[i] = reinterpret_cast<const uint2*>(g_lut_f16sel)[2 * i];
     __syncthreads();
     const int64_t ntrip = (total + 15) / 16;
     const bool words = (reinterpret_cast<uintptr_t>(packed) & 3) == 0;

@@ -200,6 +200,116 @@ static int num_sms() {
     return cached[dev];
 }
 
+// ---- shared with the kernel of large grouped launches (gemv_a16.cuh) ----
+constexpr int kGemvThreads = kGemvWarps * 32;
+template <bool kBf16> __device__ __forceinline__ float load_act(const void* p, int64_t idx) {
+    if (kBf16) return __bfloat162float(static_cast<const __nv_bfloat16*>(p)[idx]);
+    return __half2float(static_cast<const __half*>(p)[idx]);
+}
+
+// Index of the problem that owns work item `item` (tile_begin ascends): the whole CTA counts the entries that
+// start at or before it, one coalesced pass over the table instead of a chain of dependent loads (a 64-entry
+// table walked entry by entry cost the last CTAs ~40 us at the start of every grouped launch).  Every thread of
+// the CTA must call this.
+__device__ __forceinline__ int find_problem(const ojx_e8t_gemv_problem* probs, int count, int item, int scale) {
+    if (count == 1) return 0;                                  // single-problem launches (a layer at a time) skip the pass
+    int found = 0;
+    for (int base = 0; base < count; base += (int)blockDim.x) {
+        const int t = base + (int)threadIdx.x;
+        found += __syncthreads_count(t < count && scale * probs[t].tile_begin <= item);
+    }
+    return max(found - 1, 0);
+}
+
+__device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+}
+// Geometry of a work item in shared memory: 32 rows of codes, then 32 rows of scales; a row holds one
+// 48-byte (codes) / 16-byte (scales) piece per 256-wide slice of the K chunk and ends in 16 bytes of padding,
+// so that the eight rows one shared-memory load touches fall on distinct banks.
+constexpr int kGemvMaxCodePitch = kGemvWarps * 48 + 16;     // 784
+constexpr int kGemvMaxScalePitch = kGemvWarps * 16 + 16;    // 272
+
+// The optional low-rank term of a problem for output (activation row col, weight row row).
+// Kept out of line: it is rare, and inlined into the decode kernels' epilogue it costs them registers they do not have.
+template <bool kBf16>
+__device__ __noinline__ float lora_term(const ojx_e8t_gemv_problem& P, int64_t col, int64_t row) {
+    float acc = 0.f;
+    const float* t = P.lora_t + col * P.lora_rank;
+    for (int r = 0; r < P.lora_rank; ++r) acc = fmaf(t[r], load_act<kBf16>(P.lora_b, (int64_t)r * P.N + row), acc);
+    return acc;
+}
+
+// Sums the K-chunk partials of every problem that has them (fixed order), adds bias and the low-rank term, casts,
+// stores - to this rank's buffer and to every peer's window.  16-bit outputs whose rows come in multiples of eight
+// are handled eight rows (one 16-byte vector) per thread.
+template <bool kBf16>
+__global__ void __launch_bounds__(256, 3) gemv_reduce_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev,
+                                                           const __grid_constant__ ojx_e8t_gemv_problem single,
+                                                           int count, int M, int y_dtype, const __grid_constant__ PeerMap peers) {
+    const ojx_e8t_gemv_problem* probs = probs_dev != nullptr ? probs_dev : &single;
+    for (int p = blockIdx.y; p < count; p += gridDim.y) {
+        const ojx_e8t_gemv_problem& P = probs[p];
+        if (P.partial == nullptr) continue;
+        const int kc = gemv_kchunks(P.K);
+        const int64_t total = (int64_t)M * P.N;
+        const int64_t ld = P.ldy > 0 ? P.ldy : P.N;
+        const bool vec = y_dtype != OJX_F32 && (P.N & 7) == 0 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(P.y) & 15) == 0 &&
+                         (reinterpret_cast<uintptr_t>(P.partial) & 31) == 0;
+        if (vec) {
+            const int64_t per_col = P.N / 8;
+            for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < (int64_t)M * per_col;
+                 v += (int64_t)gridDim.x * blockDim.x) {
+                const int64_t col = v / per_col, row = (v - col * per_col) * 8;
+                float s8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+                for (int c = 0; c < kc; ++c) {
+                    const float4* src = reinterpret_cast<const float4*>(P.partial + (int64_t)c * total + col * P.N + row);
+                    const float4 a = __ldcg(src), b = __ldcg(src + 1);
+                    s8[0] += a.x; s8[1] += a.y; s8[2] += a.z; s8[3] += a.w;
+                    s8[4] += b.x; s8[5] += b.y; s8[6] += b.z; s8[7] += b.w;
+                }
+                uint32_t w[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    float lo = s8[2 * i], hi = s8[2 * i + 1];
+                    if (P.bias != nullptr) { lo += load_act<kBf16>(P.bias, row + 2 * i); hi += load_act<kBf16>(P.bias, row + 2 * i + 1); }
+                    if (P.lora_rank > 0) { lo += lora_term<kBf16>(P, col, row + 2 * i); hi += lora_term<kBf16>(P, col, row + 2 * i + 1); }
+                    if (y_dtype == OJX_BF16) {
+                        const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+                        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                    } else {
+                        const __half2 h = __floats2half2_rn(lo, hi);
+                        w[i] = *reinterpret_cast<const uint32_t*>(&h);
+                    }
+                }
+                const uint4 val = make_uint4(w[0], w[1], w[2], w[3]);
+                uint8_t* dst = static_cast<uint8_t*>(P.y) + (col * ld + row) * 2;
+#pragma unroll 1
+                for (int r = 0; r < peers.world; ++r)              // delta is 0 for this rank itself
+                    *reinterpret_cast<uint4*>(dst + peers.delta[r]) = val;
+            }
+            continue;
+        }
+        for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total;
+             i += (int64_t)gridDim.x * blockDim.x) {
+            float s = 0.f;
+            for (int c = 0; c < kc; ++c) s += P.partial[(int64_t)c * total + i];
+            const int64_t col = i / P.N, row = i - col * P.N;
+            if (P.bias != nullptr) s += load_act<kBf16>(P.bias, row);
+            if (P.lora_rank > 0) s += lora_term<kBf16>(P, col, row);
+            const int64_t at = col * ld + row;
+            store_any(P.y, y_dtype, at, s);
+#pragma unroll 1
+            for (int r = 0; r < peers.world; ++r)                  // the other ranks' windows (nothing when world == 1)
+                if (peers.delta[r] != 0) store_any(static_cast<uint8_t*>(P.y) + peers.delta[r], y_dtype, at, s);
+        }
+    }
+    if (peers.sync != nullptr && (peers.mode & OJX_GEMV_SIGNAL_PEERS)) {
+        __syncthreads();
+        if (threadIdx.x == 0) peer_signal(peers);
+    }
+}
+
 // Opting in to more than 48 KB of dynamic shared memory is a per-device (per-context) attribute of a kernel:
 // `done` keeps one bit per device ordinal.
 template <typename Kernel>

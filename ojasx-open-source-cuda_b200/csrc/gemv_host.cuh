@@ -1,4 +1,4 @@
-// Host-side routing of the decode-shape entry points to the kernels.
+// Host-side routing of the decode-shape entry points to the kernels: gemv_mma.cuh for one matrix, gemv_a16.cuh for grouped launches.
 #pragma once
 
 #include <atomic>
@@ -7,6 +7,7 @@
 
 #include "gemv.cuh"
 #include "gemv_mma.cuh"
+#include "gemv_a16.cuh"
 #include "gemv_lowbit.cuh"
 #include "gemv_b2.cuh"
 #include "gemv_b1.cuh"
@@ -25,6 +26,34 @@ size_t gemv_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || M > 16 || N <= 0 || K <= 0 || K % 256 != 0 || N >= (1 << 30) || K >= (1 << 30)) return 0;
     const int kc = gemv_kchunks((int)K);
     return kc > 1 ? (size_t)kc * M * N * sizeof(float) : 0;
+}
+
+template <int NB, bool kXF16, bool kI8 = false>
+static int32_t launch_gemv_a16(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count, int total,
+                               int M, int y_dtype, const PeerMap& peers_in, int overlap, cudaStream_t s) {
+    PeerMap peers = peers_in;
+    peers.host_status = host_status_device_ptr(s);
+    peers.wait_limit = wait_limit_override() != 0 ? wait_limit_override() : kSpinLimit;
+    static std::atomic<uint64_t> configured{0};
+    using Cfg = A16Cfg<NB>;
+    const int32_t st = ensure_dynamic_smem(gemv_a16_kernel<NB, kXF16, kI8>, Cfg::kSmem, configured);
+    OJX_RETURN_IF(st != OJX_OK, st);
+    const int sms = num_sms();
+    const int per = (total + sms - 1) / sms;
+    const int grid = (total + per - 1) / per;
+    return launch_maybe_overlapped(gemv_a16_kernel<NB, kXF16, kI8>, grid, kGemvThreads, Cfg::kSmem, s, overlap != 0, 1,
+                                   probs, single, count, total, M, y_dtype, overlap, peers);
+}
+
+// One bf16 activation row takes the int8 path; one to eight rows take one block of eight columns per fp16 MMA, nine to
+// sixteen take two.
+static int32_t dispatch_gemv(bool bf16, const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count,
+                             int total, int M, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s) {
+    if (bf16 && M == 1) return launch_gemv_a16<1, false, true>(probs, single, count, total, M, y_dtype, peers, overlap, s);
+    if (bf16) return M <= 8 ? launch_gemv_a16<1, false>(probs, single, count, total, M, y_dtype, peers, overlap, s)
+                            : launch_gemv_a16<2, false>(probs, single, count, total, M, y_dtype, peers, overlap, s);
+    return M <= 8 ? launch_gemv_a16<1, true>(probs, single, count, total, M, y_dtype, peers, overlap, s)
+                  : launch_gemv_a16<2, true>(probs, single, count, total, M, y_dtype, peers, overlap, s);
 }
 
 int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int total_tiles, int64_t M,
@@ -49,7 +78,6 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     OJX_RETURN_IF((flags & OJX_GEMV_INDEPENDENT) != 0 && (flags & (OJX_GEMV_SIGNAL_PEERS | OJX_GEMV_WAIT_PEERS)) != 0, OJX_ERR_UNSUPPORTED);
     const int sync_mode = flags & (OJX_GEMV_SIGNAL_PEERS | OJX_GEMV_WAIT_PEERS);
     OJX_RETURN_IF(sync_mode != 0 && peer_sync == nullptr, OJX_ERR_NULL);
-    OJX_RETURN_IF(sync_mode != 0 && count > kMmaMaxProblems, OJX_ERR_SHAPE);       // one signal per call
     OJX_RETURN_IF((reinterpret_cast<uintptr_t>(peer_sync) & 3) != 0, OJX_ERR_ALIGN);
     if (peer_sync != nullptr) {
         peers.sync = peer_sync;
@@ -58,22 +86,28 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     peers.lose_copy = (flags & OJX_GEMV_TEST_LOSE_COPY) ? 1 : 0;
     // 0: ordered like any kernel; 1: starts early, waits for its predecessor before touching x and y; 2: never waits
     const int overlap = (flags & OJX_GEMV_INDEPENDENT) ? 2 : ((flags & OJX_GEMV_STATIC_WEIGHTS) ? 1 : 0);
+    // Launches over several matrices run gemv_a16_kernel: its work items are 32 rows that run across matrix borders, where
+    // gemv_mma_kernel starts each matrix anew (two of 14336 x 4096, one and sixteen rows: 19.9 and 39 us against 20.5 and 42.4,
+    // eight of them 59.5 and 119 against 65 and 138).  One matrix, the dependent steps of a chain, is the other's: it fills a smaller
+    // table and needs no reduce launch (1024 x 2560: 4.0 and 8.9 us against 4.8 and 12.7, 4096 x 14336: 15.4 against 15.8).
+    if (count > 1) {
+        if (needs_reduce && peers.sync != nullptr) peers.mode |= 0x100;      // a reduce kernel follows and stores (and signals) in its place
+        const int32_t st = dispatch_gemv(bf, problems, none, count, total_tiles, (int)M, y_dtype, peers, overlap, s);
+        OJX_RETURN_IF(st != OJX_OK || !needs_reduce, st);
+        // Problems whose K spans several chunks carry a partial buffer; the reduce pass skips the rest.
+        dim3 grid(64, count > 64 ? 64 : count);
+        if (bf) gemv_reduce_kernel<true><<<grid, 256, 0, s>>>(problems, none, count, (int)M, y_dtype, peers);
+        else gemv_reduce_kernel<false><<<grid, 256, 0, s>>>(problems, none, count, (int)M, y_dtype, peers);
+        return launch_status();
+    }
     peers.host_status = host_status_device_ptr(s);
     peers.wait_limit = wait_limit_override() != 0 ? wait_limit_override() : kSpinLimit;
     // tiles are known on the device only: units are bounded by the table's 32-row tiles
     const int units = 2 * total_tiles, cluster = (flags & OJX_GEMV_SPLIT_K4) ? 4 : ((flags & OJX_GEMV_SPLIT_K2) ? 2 : 1);
     const bool chunked = needs_reduce != 0;
-    // launches of more matrices than a kernel lists go out in parts
-    for (int first = 0; first < count; first += kMmaMaxProblems) {
-        const int part = count - first < kMmaMaxProblems ? count - first : kMmaMaxProblems;
-        const ojx_e8t_gemv_problem* table = problems + first;
-        int32_t st;
-        if (M == 1 && bf) st = mma_launch<0, 32, 1, false, true, true>(table, none, part, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
-        else if (M <= 8) st = mma_launch<0, 32, 1, false, true>(table, none, part, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
-        else st = mma_launch<0, 32, 2, false, true>(table, none, part, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
-        OJX_RETURN_IF(st != OJX_OK, st);
-    }
-    return OJX_OK;
+    if (M == 1 && bf) return mma_launch<0, 32, 1, false, true, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
+    if (M <= 8) return mma_launch<0, 32, 1, false, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
+    return mma_launch<0, 32, 2, false, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
 }
 
 __global__ void peer_wait_kernel(const __grid_constant__ PeerMap peers) {
