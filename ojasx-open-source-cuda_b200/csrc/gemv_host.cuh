@@ -105,9 +105,9 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     // tiles are known on the device only: units are bounded by the table's 32-row tiles
     const int units = 2 * total_tiles, cluster = (flags & OJX_GEMV_SPLIT_K4) ? 4 : ((flags & OJX_GEMV_SPLIT_K2) ? 2 : 1);
     const bool chunked = needs_reduce != 0;
-    if (M == 1 && bf) return mma_launch<0, 32, 1, false, true, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
-    if (M <= 8) return mma_launch<0, 32, 1, false, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
-    return mma_launch<0, 32, 2, false, true>(problems, none, count, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
+    if (M == 1 && bf) return mma_launch<0, 32, 1, false, true, true>(problems, none, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
+    if (M <= 8) return mma_launch<0, 32, 1, false, true>(problems, none, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
+    return mma_launch<0, 32, 2, false, true>(problems, none, units, cluster, 16, chunked, (int)M, x_dtype, y_dtype, peers, overlap, s);
 }
 
 __global__ void peer_wait_kernel(const __grid_constant__ PeerMap peers) {

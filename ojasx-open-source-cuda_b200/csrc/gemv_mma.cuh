@@ -37,7 +37,6 @@ namespace ojx {
 
 constexpr int kMmaWarps = 16;
 constexpr int kMmaThreads = kMmaWarps * 32;
-constexpr int kMmaMaxProblems = 256;                 // of one launch
 constexpr int kMmaAccTiles = 16;                     // tiles whose sums over K chunks are kept at a time
 constexpr int kMmaXStageRows = 2;                    // up to so many activation rows travel inside the stages
 constexpr int kMmaXRows = 2;                         // rows a warp brings into fragment order at a time
@@ -85,9 +84,7 @@ struct MmaCtl {
     uint64_t never;                                  // tests: a barrier that nothing completes
     int abort_flag;
     uint32_t bad_rows;                               // activation rows with Inf / NaN (2.0-bit format)
-    int range[4];                                    // first (problem, tile), end (problem, tile)
-    ojx_e8t_gemv_problem prob[2];                    // the current problem of a grouped launch and the one before
-    int prefix[kMmaMaxProblems + 1];                 // cost before each problem
+    ojx_e8t_gemv_problem prob;                       // the problem of a launch from a table
 };
 
 __device__ __forceinline__ uint2 lds_u64(uint32_t addr) {
@@ -336,61 +333,7 @@ __device__ __forceinline__ void mma_fill_table(uint8_t* smem, int tid, bool roun
     }
 }
 
-// The tiles of a CTA in a grouped launch: {first problem, first tile, last problem, end tile}.  Few matrices: whole CTAs per
-// matrix, in proportion to tiles x slices, worked out by every warp on its own.  Many: the launch's cost is cut evenly,
-// boundaries rounded to whole tiles; ends with a barrier.
-__device__ __forceinline__ int4 mma_group_range(const ojx_e8t_gemv_problem* probs, int count, MmaCtl* ctl, int cluster) {
-    const int tid = threadIdx.x, lane = tid & 31, grid = (int)gridDim.x / cluster, cta = (int)blockIdx.x / cluster;
-    if (count <= 32 && count * 8 <= grid) {
-        int tiles = 0, cost = 0;
-        if (lane < count) { tiles = (probs[lane].N + 15) / 16; cost = tiles * mma_slices(probs[lane].K); }
-        int pre = cost;                                              // inclusive prefix
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xFFFFFFFFu, pre, o); if (lane >= o) pre += u; }
-        const float scale = (float)grid / (float)__shfl_sync(0xFFFFFFFFu, pre, 31);
-        const int want = (int)((float)pre * scale + 0.5f);           // first CTA of the next problem, before every problem gets one
-        int first = 0, next = 0, mine = 0;
-        for (int p = 0; p < count; ++p) {
-            next = p + 1 == count ? grid : min(max(__shfl_sync(0xFFFFFFFFu, want, p), first + 1), grid - (count - 1 - p));
-            mine = p;
-            if (cta < next) break;
-            first = next;
-        }
-        const int64_t t = __shfl_sync(0xFFFFFFFFu, tiles, mine);
-        return make_int4(mine, (int)(t * (cta - first) / (next - first)), mine, (int)(t * (cta + 1 - first) / (next - first)));
-    }
-    for (int p = tid; p < count; p += kMmaThreads) ctl->prefix[p + 1] = ((probs[p].N + 15) / 16) * mma_slices(probs[p].K);
-    __syncthreads();
-    if (tid < 32) {
-        int run = 0;
-        for (int q = 0; q < count; q += 32) {
-            int v = q + lane < count ? ctl->prefix[q + lane + 1] : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) { const int u = __shfl_up_sync(0xFFFFFFFFu, v, o); if (lane >= o) v += u; }
-            if (q + lane < count) ctl->prefix[q + lane + 1] = run + v;
-            run += __shfl_sync(0xFFFFFFFFu, v, 31);
-        }
-        if (lane == 0) ctl->prefix[0] = 0;
-    }
-    __syncthreads();
-    const int64_t total = ctl->prefix[count];
-    for (int p = tid; p < count; p += kMmaThreads) {
-        const int64_t c0 = ctl->prefix[p], c1 = ctl->prefix[p + 1];
-        const int R = mma_slices(probs[p].K);
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int64_t b = total * (cta + e) / grid;
-            if ((c0 <= b && b < c1) || (b == total && p == count - 1)) {
-                ctl->range[2 * e] = p;
-                ctl->range[2 * e + 1] = (int)((b - c0 + R / 2) / R);
-            }
-        }
-    }
-    __syncthreads();
-    return make_int4(ctl->range[0], ctl->range[1], ctl->range[2], ctl->range[3]);
-}
-
-// One matrix (kGroup false: the problem is the kernel parameter) or the problems of a grouped launch.
+// One matrix: the problem is the kernel parameter, or (kGroup) the entry of a grouped launch's table in device memory.
 //
 // kI8: one bf16 activation row of ternary codes with groups of 32 on int8 MMAs (m16n8k32).  The table holds four coordinates
 // per 32-bit entry, 32 copies: two conflict-free reads ARE the two operand registers of a rank - half the wavefronts of the
@@ -402,7 +345,7 @@ __device__ __forceinline__ int4 mma_group_range(const ojx_e8t_gemv_problem* prob
 template <int FMT, int G, int NB, bool kRag, bool kGroup, bool kI8 = false>
 __global__ void __launch_bounds__(kMmaThreads, 1)
 gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_constant__ ojx_e8t_gemv_problem single,
-                int count, int M, int x_dtype, int y_dtype, int overlap, const __grid_constant__ MmaPlan plan,
+                int M, int x_dtype, int y_dtype, int overlap, const __grid_constant__ MmaPlan plan,
                 const __grid_constant__ PeerMap peers) {
     static_assert(!kI8 || (FMT == 0 && G == 32 && NB == 1 && !kRag), "the int8 form serves one bf16 row of ternary codes");
     using F = MmaFmt<FMT, G>;
@@ -429,15 +372,10 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
 
     // the CTAs of a cluster work on the same tiles, CTA `cr` on chunks cr, cr + cs, ... of K
     const int cs = plan.cluster, cr = (int)blockIdx.x % cs;
-    int p0 = 0, t_first = 0, p1 = 0, t_end = 0;
-    if constexpr (!kGroup) {                                             // an even share of the tiles
-        const int64_t tiles = (single.N + 15) / 16;
-        t_first = (int)(tiles * (blockIdx.x / cs) / (gridDim.x / cs));
-        t_end = (int)(tiles * (blockIdx.x / cs + 1) / (gridDim.x / cs));
-    } else {
-        const int4 r = mma_group_range(probs, count, ctl, cs);
-        p0 = r.x; t_first = r.y; p1 = r.z; t_end = r.w;
-    }
+    const int K = kGroup ? probs->K : single.K, N = kGroup ? probs->N : single.N;
+    // an even share of the tiles
+    const int64_t tiles = (N + 15) / 16;
+    const int t0 = (int)(tiles * (blockIdx.x / cs) / (gridDim.x / cs)), t1 = (int)(tiles * (blockIdx.x / cs + 1) / (gridDim.x / cs));
     const bool signal = peers.sync != nullptr && (peers.mode & OJX_GEMV_SIGNAL_PEERS) != 0;
 
     uint32_t xb[NB][8][4];                      // B fragments: [block][8-weight chunk j][k 0-1, 2-3, 4-5, 6-7 of the chunk]; kI8: [j][digit pair m, k half r] at [2 m + r]
@@ -470,17 +408,15 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
     int stage = 0, buf = 0;
     auto code_bytes = [](uint32_t k) { return FMT == 0 ? k / 16 * 3 : (FMT == 2 ? k / 4 : k / 8); };       // k: multiples of 32
 
-    for (int prob = p0; prob <= p1; ++prob) {
-        // a grouped problem's descriptor: what the loader needs in registers, the rest (read after the next barrier) in shared memory
-        const ojx_e8t_gemv_problem& P = kGroup ? ctl->prob[prob & 1] : single;
-        const ojx_e8t_gemv_problem& P0 = kGroup ? probs[prob] : single;
-        const int K = P0.K, N = P0.N;
+    {
+        // of a table's entry, what the loader needs is kept in registers, the rest (read after the next barrier) in shared memory
+        const ojx_e8t_gemv_problem& P = kGroup ? ctl->prob : single;
+        const ojx_e8t_gemv_problem& P0 = kGroup ? *probs : single;
         const uint8_t* const codes = P0.packed;
         const uint8_t* const scales = reinterpret_cast<const uint8_t*>(P0.scales);
         const void* const x = P0.x;
         if (kGroup && tid < (int)(sizeof(ojx_e8t_gemv_problem) / 8))
-            reinterpret_cast<uint64_t*>(&ctl->prob[prob & 1])[tid] = reinterpret_cast<const uint64_t*>(&probs[prob])[tid];
-        const int t0 = prob == p0 ? t_first : 0, t1 = prob == p1 ? t_end : (N + 15) / 16;
+            reinterpret_cast<uint64_t*>(&ctl->prob)[tid] = reinterpret_cast<const uint64_t*>(probs)[tid];
         const int slices = mma_slices(K), chunks = mma_chunks(K), per = mma_per_chunk(K);
         const int pc = mma_pitch(per, F::kCode, kRag), ps = mma_pitch(per, F::kScale, kRag);
         const uint32_t rc = code_bytes(K), rs = (uint32_t)K / G * 2;
@@ -997,7 +933,7 @@ static int mma_max_clusters(void (*kernel)(Params...), int size, size_t smem) {
 
 // `units`: CTAs (clusters, when `cluster` > 1) the work can occupy.
 template <int FMT, int G, int NB, bool kRag, bool kGroup, bool kI8 = false>
-static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count, int units, int cluster, int max_per,
+static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int units, int cluster, int max_per,
                           bool chunked, int M, int x_dtype, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s, bool rounded = false) {
     auto kernel = gemv_mma_kernel<FMT, G, NB, kRag, kGroup, kI8>;
     static std::atomic<uint64_t> configured{0};
@@ -1016,7 +952,7 @@ static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_
     const MmaPlan plan = mma_plan<FMT, G, NB, kRag, kI8>(M, max_per, chunked, cluster, rounded);
     const int grid = (units < room ? units : room) * cluster;
     return launch_maybe_overlapped(kernel, grid, kMmaThreads, plan.total, s, overlap != 0, cluster,
-                                   probs, single, count, M, x_dtype, y_dtype, overlap, plan, peers);
+                                   probs, single, M, x_dtype, y_dtype, overlap, plan, peers);
 }
 
 // K of several chunks over few tiles: the CTAs of a cluster split the chunks, so that each prepares x for its own chunks only
@@ -1033,12 +969,12 @@ static int32_t mma_dispatch(bool rag, const ojx_e8t_gemv_problem& p, int tiles, 
     const bool rounded = FMT == 2 && !rag && (M > 8 || (M >= 4 && !(G == 32 && p.K % 2048 == 0)));
     const int per = mma_per_chunk(p.K), chunks = mma_chunks(p.K), cluster = mma_cluster_for(tiles, chunks);
     const bool chunked = chunks > 1;
-    if (rag) return M <= 8 ? mma_launch<FMT, G, 1, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s)
-                           : mma_launch<FMT, G, 2, true, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
+    if (rag) return M <= 8 ? mma_launch<FMT, G, 1, true, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s)
+                           : mma_launch<FMT, G, 2, true, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
     if (FMT == 0 && G == 32 && M == 1 && x_dtype == OJX_BF16)
-        return mma_launch<0, 32, 1, false, false, true>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
-    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded)
-                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, 1, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded);
+        return mma_launch<0, 32, 1, false, false, true>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
+    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded)
+                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded);
 }
 
 // One matrix; the caller has checked gemv_mma_ok and the alignment (16 bytes) of x, codes and scales.  `overlap` 3: nothing is read
