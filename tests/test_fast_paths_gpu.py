@@ -178,3 +178,16 @@ def test_adapter_layer_on_a_batch_of_tokens(P):
     assert y.shape == y_grad.shape == (2, 20, 264) and y_grad.requires_grad
     for v in (y, y_grad):
         assert float((v.double() - ref).norm() / ref.norm()) < 8e-3
+
+
+@pytest.mark.parametrize("rows,cols,group", [(1, 3, 8), (5, 1023, 8), (7, 4096, 32), (33, 1021, 24), (1025, 33, 16)])
+def test_unpack_2bit_at_the_edges_of_its_chunks(P, rows, cols, group):
+    """Fewer weights than a chunk, a last chunk that is cut short, groups that are no power of two: every type against the fp32 values."""
+    dev = torch.device(DEV)
+    packed, scales = P.ops.encode_2bit(P.ops.generate(rows * cols, 5, 1.0, torch.float32, dev).view(rows, cols), group)
+    codes = torch.stack([(packed.int() >> (2 * i)) & 3 for i in range(4)], 1).reshape(-1)[:rows * cols]
+    index = torch.arange(rows * cols, device=dev) // group
+    for dt in (torch.float32, torch.float16, torch.bfloat16):
+        got = P.ops.decode_2bit(packed, scales, (rows, cols), dt)
+        want = (codes.float() - 1.5) * scales[index].to(dt).float()
+        assert torch.equal(got, want.to(dt).view(rows, cols)), dt
