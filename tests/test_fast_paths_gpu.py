@@ -191,3 +191,16 @@ def test_unpack_2bit_at_the_edges_of_its_chunks(P, rows, cols, group):
         got = P.ops.decode_2bit(packed, scales, (rows, cols), dt)
         want = (codes.float() - 1.5) * scales[index].to(dt).float()
         assert torch.equal(got, want.to(dt).view(rows, cols)), dt
+
+
+@pytest.mark.parametrize("rows,cols,group", [(1, 3, 8), (5, 1023, 8), (33, 1021, 24)])
+def test_unpack_1bit_at_the_edges_of_its_codes(P, rows, cols, group):
+    """A last code that is cut short, groups that are no power of two; every type against the fp32 values of whole codes."""
+    dev = torch.device(DEV)
+    total, codes = rows * cols, (rows * cols + 7) // 8
+    packed, scales = P.ops.encode_1bit(P.ops.generate(total, 5, 1.0, torch.float32, dev).view(rows, cols), group)
+    unit = P.ops.decode_1bit(packed, torch.ones(-(-codes * 8 // group), dtype=torch.float16, device=dev), (codes, 8), torch.float32)
+    index = torch.arange(total, device=dev) // group
+    for dt in (torch.float32, torch.float16, torch.bfloat16):
+        want = unit.reshape(-1)[:total] * scales[index].to(dt).float()
+        assert torch.equal(P.ops.decode_1bit(packed, scales, (rows, cols), dt), want.to(dt).view(rows, cols)), dt
