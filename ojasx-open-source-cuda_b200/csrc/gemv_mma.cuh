@@ -377,6 +377,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
     const int64_t tiles = (N + 15) / 16;
     const int t0 = (int)(tiles * (blockIdx.x / cs) / (gridDim.x / cs)), t1 = (int)(tiles * (blockIdx.x / cs + 1) / (gridDim.x / cs));
     const bool signal = peers.sync != nullptr && (peers.mode & OJX_GEMV_SIGNAL_PEERS) != 0;
+    const bool waits = peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS) != 0;
 
     uint32_t xb[NB][8][4];                      // B fragments: [block][8-weight chunk j][k 0-1, 2-3, 4-5, 6-7 of the chunk]; kI8: [j][digit pair m, k half r] at [2 m + r]
     uint32_t xc[NB][F::kSW][2];                 // 2.0-bit: half the scale groups' sums of x, high and low parts, two groups each
@@ -480,18 +481,20 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
-            // packed weights of a static launch do not depend on the launch ahead: their copies start before it has drained
-            for (int i = 0; i < D; ++i) issue(i, !(first_run && overlap == 1));
+            // packed weights of a static launch do not depend on the launch ahead: their copies start before it has drained.  x does,
+            // and where peers are waited for it is written by them until then: its copies follow both waits.
+            const bool late_x = first_run && (overlap == 1 || waits);
+            for (int i = 0; i < D; ++i) issue(i, !late_x);
             if (first_run) {
                 if (kGroup) mma_fill_table<FMT, kI8>(smem, tid, plan.rounded != 0);
                 // activations (and the output buffers) depend on the launch ahead, unless the caller declared this one independent
                 if (overlap == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
                 // ... and, in a column-sharded chain, on the same launch of every other rank
-                if (peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS)) {
+                if (waits) {
                     if (tid == 0) peer_wait(peers);
                     __syncthreads();
                 }
-                if (overlap == 1 && x_staged) {
+                if (late_x && x_staged) {
                     for (int i = 0; i < D && i < total; ++i)
                         if (i % np == 0) copy_x(cr + i / np * cs, base + plan.off_ring + i * plan.stage_bytes);
                     asm volatile("cp.async.wait_all;" ::: "memory");

@@ -3,6 +3,8 @@ faulting it: every wait in the kernels is bounded, so the tests make a wait run 
 a copy whose completion is never reported) and check that the kernel returns, that the failure is reported
 through every channel, and that the next normal call is correct."""
 
+import time
+
 import numpy as np
 import pytest
 
@@ -62,6 +64,34 @@ def test_chain_orders_itself_on_the_device(P):
     words = sync.cpu().numpy()
     assert words[0] == 9 and words[1] == 0 and words[2] == 0 and words[4] == 9      # epoch, arrived, status, flag[0]
     assert P._cabi.lib().ojx_e8t_device_status() == 0
+
+
+@pytest.mark.parametrize("static", [False, True])
+@pytest.mark.parametrize("m,k", [(1, 2048), (2, 2048), (2, 8192), (4, 2048)])
+def test_x_is_read_after_the_peers_have_published_it(P, m, k, static):
+    """A launch over one matrix that waits for its peers: x, in memory the host can write, changes after the kernel has started
+    and before the awaited flag is set (as another rank's stores would), and the result has to be the new x's.  The wait is bounded."""
+    dev, n = torch.device(DEV), 96
+    pk, sc, x = _problem(P, n, k, m, 60)
+    want = P.ops.linear(x, pk, sc, None, n, k, 32)
+    host_x = torch.zeros((m, k), dtype=torch.bfloat16).pin_memory()
+    sync = torch.zeros(16, dtype=torch.int32).pin_memory()
+    sync[0], sync[3] = 1, 1 << 20                               # one launch is awaited; polls before giving up
+    y, lib = torch.zeros((m, n), dtype=torch.bfloat16, device=dev), P._cabi.lib()
+    prob = P._cabi.GemvProblem(x=host_x.data_ptr(), packed=pk.data_ptr(), scales=sc.data_ptr(), y=y.data_ptr(), N=n, K=k)
+    table = torch.frombuffer(bytearray(bytes(prob)), dtype=torch.uint8).to(dev)
+    new_x = x.cpu()
+    torch.cuda.synchronize()
+    flags = P._cabi.OJX_GEMV_WAIT_PEERS | (P._cabi.OJX_GEMV_STATIC_WEIGHTS if static else 0)
+    st = lib.ojx_e8t_gemv_grouped_ex(table.data_ptr(), 1, lib.ojx_e8t_gemv_tiles(n, k), m, P._cabi.OJX_BF16, P._cabi.OJX_BF16,
+                                     int(lib.ojx_e8t_gemv_kchunks(k) > 1), None, 1, sync.data_ptr(), flags,
+                                     torch.cuda.current_stream().cuda_stream)
+    time.sleep(0.02)                                            # the kernel is at its wait
+    host_x.copy_(new_x)
+    sync[4] = 1                                                 # flag[0]
+    torch.cuda.synchronize()
+    assert st == 0 and int(sync[2]) == 0 and lib.ojx_e8t_device_status() == 0
+    assert float((y.float() - want.float()).norm() / want.float().norm()) <= 4e-3       # K split or not: a bf16 rounding each
 
 
 def test_wait_on_a_rank_that_never_signals_gives_up(P):
