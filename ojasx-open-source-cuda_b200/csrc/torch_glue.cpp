@@ -38,6 +38,16 @@ bool packed_pair(const at::Tensor* packed, const at::Tensor* scales, c10::Device
            packed->device() == dev && scales->device() == dev;
 }
 
+// The buffers hold the codes and scales of an [n, k] weight: every kernel reads all of them.  (What is too short takes the general
+// path, which raises; a group that no format has is refused by the library.)
+bool holds(int fmt, const at::Tensor& packed, const at::Tensor& scales, int64_t n, int64_t k, int64_t group) {
+    if (n > (int64_t{1} << 31) || k > (int64_t{1} << 31)) return false;
+    if (fmt == 0 && (group <= 0 || group % 16 != 0)) group = 16;
+    if (group <= 0) return true;
+    const int64_t total = n * k, codes = fmt == 0 ? (total + 15) / 16 * 3 : (fmt == 2 ? (total + 3) / 4 : (total + 7) / 8);
+    return packed.numel() >= codes && scales.numel() >= (total + group - 1) / group;
+}
+
 at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) {
     return at::detail::empty_cuda(sizes, t, dev, std::nullopt);
 }
@@ -77,7 +87,7 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!a.ok || !plain(x) || x->dim() < 1 || n <= 0 || k <= 0 || x->size(-1) != k || x->numel() == 0) Py_RETURN_NONE;
     const c10::Device dev = x->device();
     const int xd = dtype_code(x->scalar_type());
-    if (xd < 0 || !packed_pair(pk, sc, dev)) Py_RETURN_NONE;
+    if (xd < 0 || !packed_pair(pk, sc, dev) || !holds(fmt, *pk, *sc, n, k, group)) Py_RETURN_NONE;
     if (args[4] != Py_None &&
         (!plain(bias) || bias->device() != dev || bias->scalar_type() != x->scalar_type() || bias->numel() != n))
         Py_RETURN_NONE;
@@ -121,7 +131,7 @@ PyObject* py_linear_adapter(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
     const c10::Device dev = x->device();
     const at::ScalarType xt = x->scalar_type();
     const int xd = dtype_code(xt);
-    if ((xd != OJX_BF16 && xd != OJX_F16) || !packed_pair(pk, sc, dev)) Py_RETURN_NONE;
+    if ((xd != OJX_BF16 && xd != OJX_F16) || !packed_pair(pk, sc, dev) || !holds(fmt, *pk, *sc, n, k, group)) Py_RETURN_NONE;
     if (args[4] != Py_None && (!plain(bias) || bias->device() != dev || bias->scalar_type() != xt || bias->numel() != n)) Py_RETURN_NONE;
     if (!plain(la) || !plain(lb) || la->device() != dev || lb->device() != dev || la->scalar_type() != xt || lb->scalar_type() != xt ||
         la->dim() != 2 || lb->dim() != 2 || la->size(0) != k || lb->size(1) != n || la->size(1) != lb->size(0))
@@ -155,7 +165,7 @@ PyObject* py_linear_dx(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (!a.ok || !plain(gy) || gy->dim() != 2 || n <= 0 || k <= 0 || gy->size(1) != n || gy->size(0) == 0) Py_RETURN_NONE;
     const c10::Device dev = gy->device();
     const int gd = dtype_code(gy->scalar_type());
-    if ((gd != OJX_BF16 && gd != OJX_F16) || !packed_pair(pk, sc, dev)) Py_RETURN_NONE;
+    if ((gd != OJX_BF16 && gd != OJX_F16) || !packed_pair(pk, sc, dev) || !holds(fmt, *pk, *sc, n, k, group)) Py_RETURN_NONE;
     if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
     const c10::cuda::CUDAGuard guard(dev);
     const int64_t m = gy->size(0);

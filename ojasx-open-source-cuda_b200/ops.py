@@ -178,7 +178,7 @@ def _linear(fmt: int, x: torch.Tensor, packed: torch.Tensor, scales: torch.Tenso
     y = _cabi.glue().linear(fmt, x, packed, scales, bias, n, k, group_size, -1 if out_dtype is None else _dtype_code(out_dtype), flags, False)
     if y is not None:
         return _result(y, "ojx_e8t_linear")
-    dev, x2d, pk, sc, b = _prep_linear(x, packed, scales, bias, n, k)
+    dev, x2d, pk, sc, b = _prep_linear(fmt, x, packed, scales, bias, n, k, group_size)
     _cabi.raise_pending()
     m = int(x2d.shape[0])
     y = torch.empty((m, n), dtype=out_dtype or x2d.dtype, device=dev)
@@ -245,6 +245,7 @@ def linear_lowbit_lora(bits: int, x: torch.Tensor, packed: torch.Tensor, scales:
         raise ValueError("this shape cannot take the fused adapter term; add it separately")
     if tuple(lora_t.shape) != (m, r) or tuple(lora_b.shape) != (r, n):
         raise ValueError("lora_t must be [M, r] and lora_b [r, N]")
+    _check_packed(bits, packed, scales, n, k, group_size)
     t = lora_t.detach().to(torch.float32).contiguous()
     bb = lora_b.detach().to(x2.dtype).contiguous()
     b = None if bias is None else bias.detach().to(x2.dtype).contiguous()
@@ -411,12 +412,24 @@ def generate(count: int, seed: int, sigma: float, dtype: torch.dtype, device: to
     return out
 
 
-def _prep_linear(x2d, packed, scales, bias, n, k):
+def _check_packed(fmt: int, packed: torch.Tensor, scales: torch.Tensor, n: int, k: int, group_size: int) -> None:
+    """Raises unless the buffers hold the codes and scales of an ``[n, k]`` weight: every kernel reads all of them."""
+    if packed.dtype != torch.uint8 or scales.dtype != torch.float16:
+        raise TypeError("packed must be uint8 and scales float16")
+    g = effective_group(group_size) if fmt == 0 else int(group_size)
+    if g <= 0:
+        return                                             # the library refuses it
+    total = n * k
+    codes = -(-total // 16) * 3 if fmt == 0 else (-(-total // 4) if fmt == 2 else -(-total // 8))
+    if packed.numel() < codes or scales.numel() < -(-total // g):
+        raise ValueError(f"packed ({packed.numel()}) and scales ({scales.numel()}) are too short for a [{n}, {k}] weight in groups of {g}")
+
+
+def _prep_linear(fmt, x2d, packed, scales, bias, n, k, group_size):
     dev = _require_cuda(x2d, packed, scales, bias)
     if x2d.dim() != 2 or x2d.shape[1] != k:
         raise ValueError(f"x must be [M, {k}], got {tuple(x2d.shape)}")
-    if packed.dtype != torch.uint8 or scales.dtype != torch.float16:
-        raise TypeError("packed must be uint8 and scales float16")
+    _check_packed(fmt, packed, scales, n, k, group_size)
     x2d = x2d.contiguous()
     b = None
     if bias is not None:
@@ -446,7 +459,7 @@ def linear_lora(x2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, b
         if y is not None:
             return y
         lora_t, x2d = _adapter_parts(x2d, lora_a, scaling, hadamard)
-    dev, x2d, pk, sc, b = _prep_linear(x2d, packed, scales, bias, n, k)
+    dev, x2d, pk, sc, b = _prep_linear(0, x2d, packed, scales, bias, n, k, group_size)
     _cabi.raise_pending()
     m, r = int(x2d.shape[0]), int(lora_b.shape[0])
     if not lora_fusable(m, k, group_size, x2d.dtype, r):
@@ -498,8 +511,7 @@ def linear_dx(grad_y2d: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor
     dev = _require_cuda(grad_y2d, packed, scales)
     if grad_y2d.dim() != 2 or grad_y2d.shape[1] != n:
         raise ValueError(f"grad_y must be [M, {n}], got {tuple(grad_y2d.shape)}")
-    if packed.dtype != torch.uint8 or scales.dtype != torch.float16:
-        raise TypeError("packed must be uint8 and scales float16")
+    _check_packed(0, packed, scales, n, k, g)
     gy = grad_y2d.contiguous()
     m = int(gy.shape[0])
     ydt = out_dtype or gy.dtype
@@ -536,6 +548,7 @@ def linear_dx_lowbit(bits: int, grad_y2d: torch.Tensor, packed: torch.Tensor, sc
     dev = _require_cuda(grad_y2d, packed, scales)
     if grad_y2d.dim() != 2 or grad_y2d.shape[1] != n:
         raise ValueError(f"grad_y must be [M, {n}], got {tuple(grad_y2d.shape)}")
+    _check_packed(bits, packed, scales, n, k, group_size)
     gy = grad_y2d.contiguous()
     m = int(gy.shape[0])
     ydt = out_dtype or gy.dtype

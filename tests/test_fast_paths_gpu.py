@@ -204,3 +204,31 @@ def test_unpack_1bit_at_the_edges_of_its_codes(P, rows, cols, group):
     for dt in (torch.float32, torch.float16, torch.bfloat16):
         want = unit.reshape(-1)[:total] * scales[index].to(dt).float()
         assert torch.equal(P.ops.decode_1bit(packed, scales, (rows, cols), dt), want.to(dt).view(rows, cols)), dt
+
+
+@pytest.mark.parametrize("bits,group,k", [(1.5, 32, 512), (1.5, 16, 288), (2.0, 8, 512), (2.0, 32, 96), (1.0, 32, 512), (1.0, 8, 96)])
+def test_buffers_too_short_for_the_shape_are_refused(P, bits, group, k):
+    """Codes or scales of one row fewer: every entry point raises before anything is launched; longer buffers are taken."""
+    n, dev = 48, torch.device(DEV)
+    packed, scales, _ = _problem(P, bits, n, k, group)
+    fmt = {1.0: 1, 1.5: 0, 2.0: 2}[bits]
+    fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    short = [(packed[:-packed.numel() // n], scales), (packed, scales[:-1])]
+    lora_a, lora_b = torch.zeros(k, 8, dtype=torch.bfloat16, device=dev), torch.zeros(8, n, dtype=torch.bfloat16, device=dev)
+    for m in (1, 8, 40):
+        x, gy = torch.randn(m, k, device=dev).bfloat16(), torch.randn(m, n, device=dev).bfloat16()
+        y = fn(x, packed, scales, None, n, k, group)
+        assert torch.equal(y, fn(x, torch.cat([packed, packed]), torch.cat([scales, scales]), None, n, k, group))
+        for pk, sc in short:
+            with pytest.raises(ValueError):
+                fn(x, pk, sc, None, n, k, group)
+            with pytest.raises(ValueError):
+                fn(x.float(), pk, sc, None, n, k, group)
+            with pytest.raises(ValueError):
+                P.ops.linear_dx(gy, pk, sc, n, k, group) if fmt == 0 else P.ops.linear_dx_lowbit(fmt, gy, pk, sc, n, k, group)
+            assert P.ops.layer_forward(fmt, x, pk, sc, None, n, k, group, False) is None
+            assert P.ops.layer_forward_adapter(fmt, x, pk, sc, None, n, k, group, False, lora_a, lora_b, 1.0) is None
+            layer = P.E8LatticeLinear(k, n, bias=False, rank=8, group_size=group, bitrate=bits, device=dev, dtype=torch.bfloat16)
+            layer.packed_weight, layer.block_scales = pk, sc
+            with torch.no_grad(), pytest.raises(ValueError):
+                layer(x)

@@ -291,3 +291,16 @@ def test_adapter_epilogue_shape_rules(P):
     assert not ops.lowbit_lora_fusable(8, 8192, 32, 8)                   # eight rows of 8192 activations do not fit shared memory
     assert not ops.lowbit_lora_fusable(1, 4096, 8, 8) and not ops.lowbit_lora_fusable(1, 4352, 32, 8)
     assert not ops.lowbit_lora_fusable(9, 2048, 32, 8) and not ops.lowbit_lora_fusable(0, 2048, 32, 8)
+
+
+@pytest.mark.parametrize("fmt,group,n,k,codes,scales", [(0, 32, 4, 64, 48, 8), (0, 8, 3, 24, 15, 5), (2, 8, 3, 3, 3, 2), (2, 32, 4, 64, 64, 8),
+                                                        (1, 8, 3, 3, 2, 2), (1, 32, 4, 64, 32, 8)])
+def test_packed_buffers_have_to_hold_the_whole_weight(P, fmt, group, n, k, codes, scales):
+    """Codes of ceil(n k / 16) * 3, ceil(n k / 4) or ceil(n k / 8) bytes and one scale per started group, or a ValueError."""
+    pk, sc = torch.zeros(codes, dtype=torch.uint8), torch.zeros(scales, dtype=torch.float16)
+    P.ops._check_packed(fmt, pk, sc, n, k, group)
+    for a, b in ((pk[:-1], sc), (pk, sc[:-1])):
+        with pytest.raises(ValueError):
+            P.ops._check_packed(fmt, a, b, n, k, group)
+    with pytest.raises(TypeError):
+        P.ops._check_packed(fmt, pk, sc.float(), n, k, group)
