@@ -159,6 +159,7 @@ def _decode_lowbit(bits: int, packed: torch.Tensor, scales: torch.Tensor, shape:
     dev = _require_cuda(packed, scales)
     rows, cols = int(shape[0]), int(shape[1])
     group = (packed.numel() * (4 if bits == 2 else 8)) // max(1, scales.numel())
+    _check_packed(bits, packed, scales, rows, cols, group)
     name = "ojx_e8t_decode_2bit" if bits == 2 else "ojx_e8t_decode_1bit"
     w = _cabi.glue().decode(bits, packed, scales, rows, cols, group, _dtype_code(dtype))
     if w is not None:

@@ -232,3 +232,10 @@ def test_buffers_too_short_for_the_shape_are_refused(P, bits, group, k):
             layer.packed_weight, layer.block_scales = pk, sc
             with torch.no_grad(), pytest.raises(ValueError):
                 layer(x)
+
+
+@pytest.mark.parametrize("bits", [1.0, 2.0])
+def test_sibling_unpackers_refuse_buffers_too_short_for_the_shape(P, bits):
+    packed, scales, _ = _problem(P, bits, 64, 2048, 32)
+    with pytest.raises(ValueError):
+        P.ops._decode_lowbit(int(bits), packed, scales, (65, 2048), torch.float32)
