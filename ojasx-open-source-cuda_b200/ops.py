@@ -247,6 +247,7 @@ def linear_lowbit_lora(bits: int, x: torch.Tensor, packed: torch.Tensor, scales:
     if tuple(lora_t.shape) != (m, r) or tuple(lora_b.shape) != (r, n):
         raise ValueError("lora_t must be [M, r] and lora_b [r, N]")
     _check_packed(bits, packed, scales, n, k, group_size)
+    packed, scales = packed.contiguous(), scales.contiguous()
     t = lora_t.detach().to(torch.float32).contiguous()
     bb = lora_b.detach().to(x2.dtype).contiguous()
     b = None if bias is None else bias.detach().to(x2.dtype).contiguous()
@@ -550,7 +551,7 @@ def linear_dx_lowbit(bits: int, grad_y2d: torch.Tensor, packed: torch.Tensor, sc
     if grad_y2d.dim() != 2 or grad_y2d.shape[1] != n:
         raise ValueError(f"grad_y must be [M, {n}], got {tuple(grad_y2d.shape)}")
     _check_packed(bits, packed, scales, n, k, group_size)
-    gy = grad_y2d.contiguous()
+    gy, packed, scales = grad_y2d.contiguous(), packed.contiguous(), scales.contiguous()
     m = int(gy.shape[0])
     ydt = out_dtype or gy.dtype
     if m == 0:

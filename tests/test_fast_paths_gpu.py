@@ -239,3 +239,16 @@ def test_sibling_unpackers_refuse_buffers_too_short_for_the_shape(P, bits):
     packed, scales, _ = _problem(P, bits, 64, 2048, 32)
     with pytest.raises(ValueError):
         P.ops._decode_lowbit(int(bits), packed, scales, (65, 2048), torch.float32)
+
+
+@pytest.mark.parametrize("bits", [1.0, 2.0])
+def test_sibling_formats_on_buffers_with_strides(P, bits):
+    """Codes and scales that are every other element of a wider buffer give what contiguous ones give."""
+    n, k, m, fmt, dev = 64, 2048, 3, int(bits), torch.device(DEV)
+    packed, scales, _ = _problem(P, bits, n, k, 32)
+    wide_pk, wide_sc = torch.stack([packed, ~packed], 1)[:, 0], torch.stack([scales, scales + 1], 1)[:, 0]
+    gy, t = torch.randn(m, n, device=dev).bfloat16(), torch.randn(m, 8, device=dev)
+    x, b = torch.randn(m, k, device=dev).bfloat16(), torch.randn(8, n, device=dev).bfloat16()
+    for fn in (lambda p, s: P.ops.linear_dx_lowbit(fmt, gy, p, s, n, k, 32), lambda p, s: P.ops._decode_lowbit(fmt, p, s, (n, k), torch.float32),
+               lambda p, s: P.ops.linear_lowbit_lora(fmt, x, p, s, None, n, k, 32, t, b)):
+        assert torch.equal(fn(packed, scales), fn(wide_pk, wide_sc))
