@@ -164,9 +164,10 @@ def _decode_lowbit(bits: int, packed: torch.Tensor, scales: torch.Tensor, shape:
     w = _cabi.glue().decode(bits, packed, scales, rows, cols, group, _dtype_code(dtype))
     if w is not None:
         return _result(w, name)
+    pk, sc = packed.contiguous(), scales.contiguous()          # held until the launch: a copy's memory must not be given out again
     out = torch.empty((rows, cols), dtype=dtype, device=dev)
     with torch.cuda.device(dev):
-        st = getattr(_cabi.lib(), name)(packed.contiguous().data_ptr(), scales.contiguous().data_ptr(), rows, cols, group,
+        st = getattr(_cabi.lib(), name)(pk.data_ptr(), sc.data_ptr(), rows, cols, group,
                                         _dtype_code(dtype), out.data_ptr(), _stream_ptr(dev))
     _cabi.check(st, name)
     return out
