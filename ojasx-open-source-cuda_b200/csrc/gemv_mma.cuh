@@ -710,7 +710,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
                 for (int o = 1; o < (1 << qs); o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
                 if (q_sub != 0 || q_col >= M || n >= N || n >= (b0 + nt) * 16) return;
-                if (chunks > 1) {
+                if (chunks > 1 || cs > 1) {                              // (a cluster adds up what its CTAs left here, of one chunk too)
                     float* a = acc_sums + (pair * M + q_col) * R + q_row;
                     if (chunk > cr) sum += *a;
                     if (chunk + cs < chunks || cs > 1) { *a = sum; return; }

@@ -191,3 +191,22 @@ def test_independent_launches_overlap_without_changing_results(P):
     st = lib.ojx_e8t_gemv_grouped_ex(g0.table.data_ptr(), g0.count, g0.total_tiles, g0.M, 2, 2, g0.needs_reduce, None, 1,
                                      sync.data_ptr(), P._cabi.OJX_GEMV_INDEPENDENT | P._cabi.OJX_GEMV_WAIT_PEERS, None)
     assert st == -9
+
+
+@pytest.mark.parametrize("m", [1, 4, 16])
+@pytest.mark.parametrize("n,k", [(40, 256), (1000, 4096), (72, 4352)])
+def test_split_flags_do_not_change_results(P, m, n, k):
+    """OJX_GEMV_SPLIT_K2 / K4 are hints: K of one chunk, or of fewer than the cluster has CTAs, gives the unsplit launch's result."""
+    pk, sc, x = _problem(P, n, k, m, 70)
+    outs = []
+    for flag in (0, P._cabi.OJX_GEMV_SPLIT_K2, P._cabi.OJX_GEMV_SPLIT_K4):
+        y = torch.zeros((m, n), dtype=torch.float32, device=DEV)
+        g = P.ops.GroupedGemv([(x, pk, sc, None, y)], [(n, k)], extra_flags=flag)
+        g.flags = flag                                          # none that the constructor would choose itself
+        g()
+        outs.append(y)
+    torch.cuda.synchronize()
+    wd = P.ops.decode(pk, sc, (n, k), torch.float32).double()
+    bound = x.double().abs() @ wd.abs().t()
+    for y in outs:
+        assert float(((y.double() - x.double() @ wd.t()).abs() / bound).max()) <= 5e-6
