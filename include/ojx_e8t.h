@@ -341,7 +341,8 @@ int32_t ojx_e8t_gemv_grouped_peers(const ojx_e8t_gemv_problem* problems, int32_t
  *       it in `stream` that may still be running (for example the previous launches of a sweep over different
  *       matrices with their own outputs).  The launch then never waits for its predecessor: its CTAs start as
  *       multiprocessors become free, so the tail of one launch is filled by the head of the next.  Work queued
- *       AFTER the launch is ordered after it as usual.  Not allowed together with the peer flags.
+ *       AFTER the launch is ordered after it, and after what was queued ahead of it, as usual (one CTA stays until the
+ *       predecessor has ended).  Not allowed together with the peer flags.
  *   OJX_GEMV_SIGNAL_PEERS    (needs peer_sync and peer_delta) once every result of the launch has been stored into
  *       every rank's window, this rank publishes its next epoch into flag[this rank] of every rank's block
  *       (release at system scope, plain stores over NVLink) and advances its own epoch.

@@ -111,6 +111,13 @@ __device__ __noinline__ bool peer_wait(const PeerMap& pm) {
     return ok;
 }
 
+// Last step of an independent launch (overlap 2): one thread of its first CTA, which always has work, stays until the launch ahead
+// has ended.  The other CTAs and the launch's start are as free as before, but the launch has not ended before its predecessor, so
+// that one which follows with the same attribute and waits for IT comes after both.
+__device__ __forceinline__ void leave_after_predecessor(int overlap) {
+    if (overlap == 2 && blockIdx.x == 0 && threadIdx.x == 0) asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void sts_u128(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }

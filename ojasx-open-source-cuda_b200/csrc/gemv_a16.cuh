@@ -554,6 +554,7 @@ gemv_a16_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev, const __grid
         __syncthreads();
         if (tid == 0) peer_signal(peers);
     }
+    leave_after_predecessor(overlap);
 }
 
 }  // namespace ojx

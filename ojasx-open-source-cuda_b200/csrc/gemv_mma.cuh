@@ -883,6 +883,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
         __syncthreads();
         if (tid == 0) peer_signal(peers);
     }
+    leave_after_predecessor(overlap);
 }
 
 // ---- host side ---------------------------------------------------------------------------------------------------

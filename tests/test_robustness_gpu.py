@@ -210,3 +210,28 @@ def test_split_flags_do_not_change_results(P, m, n, k):
     bound = x.double().abs() @ wd.abs().t()
     for y in outs:
         assert float(((y.double() - x.double() @ wd.t()).abs() / bound).max()) <= 5e-6
+
+
+@pytest.mark.parametrize("count", [1, 2])
+def test_reader_behind_an_independent_launch_sees_what_came_before_it(P, count):
+    """linear -> independent launch -> linear that reads the first one's output: the reader may start early, but not before the
+    first has ended, although the launch between them waits for nobody.  (Both kernels of grouped launches.)"""
+    dev = torch.device(DEV)
+    pk, sc, _ = _problem(P, 14336, 4096, 1, 80)
+    pk2, sc2, _ = _problem(P, 64, 14336, 1, 82)
+    small = [_problem(P, 16, 256, 1, 84 + i) for i in range(count)]
+    outs = [torch.zeros((1, 16), dtype=torch.bfloat16, device=dev) for _ in range(count)]
+    between = P.ops.GroupedGemv([(x, p, s, None, y) for (p, s, x), y in zip(small, outs)], [(16, 256)] * count, independent=True)
+    xs = [P.ops.generate(16 * 4096, 90 + i, 1.0, torch.bfloat16, dev).view(16, 4096) for i in range(2)]
+    want = []
+    for x in xs:
+        y = P.ops.linear(x, pk, sc, None, 14336, 4096, 32)
+        torch.cuda.synchronize()
+        want.append(P.ops.linear(y, pk2, sc2, None, 64, 14336, 32))
+        del y
+    for i in range(40):                                     # the first output's memory is used again: a stale read is the other x's
+        y = P.ops.linear(xs[i % 2], pk, sc, None, 14336, 4096, 32)
+        between()
+        z = P.ops.linear(y, pk2, sc2, None, 64, 14336, 32)
+        assert torch.equal(z, want[i % 2]), i
+        del y
