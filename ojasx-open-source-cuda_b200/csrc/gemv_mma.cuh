@@ -73,7 +73,6 @@ __host__ __device__ inline int mma_per_chunk(int K) { const int c = mma_chunks(K
 struct MmaPlan {                                     // shared-memory layout, by the host
     int stage_bytes, scale_off, x_off;               // of a stage: scales, and x of a chunk's first item
     int x_staged;                                    // x travels inside the stages (up to kMmaXStageRows rows)
-    int rounded;                                     // 2.0-bit: weights (code - 1.5) * scale rounded to fp16, as the batch kernel has them
     int cluster;                                     // CTAs that share tiles and split the chunks of K
     int off_ring, off_part, off_acc, off_x, off_ctl; // byte offsets: ring, partial sums (two buffers), sums over chunks, x staging, control
     int total;
@@ -288,7 +287,7 @@ __device__ __forceinline__ float mma_ld_cluster(uint32_t addr, int rank) {
 // Decode table in shared memory, entry stride 128 bytes: sixteen 8-byte copies (1.0 bit: eight of 16 bytes, int8: 32 of 4
 // bytes), so that every lane of an access reads banks of its own.  Four threads per entry, two 16-byte stores each.
 template <int FMT, bool kI8>
-__device__ __forceinline__ void mma_fill_table(uint8_t* smem, int tid, bool rounded) {
+__device__ __forceinline__ void mma_fill_table(uint8_t* smem, int tid) {
     constexpr int kEntries = FMT == 0 ? 104 : 256;
 #pragma unroll
     for (int e0 = 0; e0 < kEntries; e0 += kMmaThreads / 4) {
@@ -311,8 +310,8 @@ __device__ __forceinline__ void mma_fill_table(uint8_t* smem, int tid, bool roun
             } else {
                 v = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[0] | (h[1] << 16), h[2] | (h[3] << 16));
             }
-        } else if constexpr (FMT == 2) {                       // a byte of codes -> four values code - 2 (rounded: code - 1.5)
-            const uint32_t lo = rounded ? 0xB800BE00u : 0xBC00C000u, hi = rounded ? 0x3E003800u : 0x3C000000u;
+        } else if constexpr (FMT == 2) {                       // a byte of codes -> four values code - 2
+            constexpr uint32_t lo = 0xBC00C000u, hi = 0x3C000000u;
             uint32_t h[4];
 #pragma unroll
             for (int k = 0; k < 4; ++k) { const int c = (entry >> (2 * k)) & 3; h[k] = ((c & 2 ? hi : lo) >> (16 * (c & 1))) & 0xFFFFu; }
@@ -367,7 +366,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
     const uint32_t lane_at = lane_off + base, lane_f = mma_lane_f(lane_off), lane_v = mma_lane_v(lane_at);
     // A launch whose weights were not promised static waits for the kernel ahead before it reads anything; its table is ready by
     // then.  A static launch starts its copies first and fills the table while they travel.
-    if (!kGroup) mma_fill_table<FMT, kI8>(smem, tid, plan.rounded != 0);
+    if (!kGroup) mma_fill_table<FMT, kI8>(smem, tid);
     if (overlap == 3) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // the CTAs of a cluster work on the same tiles, CTA `cr` on chunks cr, cr + cs, ... of K
@@ -486,7 +485,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
             const bool late_x = first_run && (overlap == 1 || waits);
             for (int i = 0; i < D; ++i) issue(i, !late_x);
             if (first_run) {
-                if (kGroup) mma_fill_table<FMT, kI8>(smem, tid, plan.rounded != 0);
+                if (kGroup) mma_fill_table<FMT, kI8>(smem, tid);
                 // activations (and the output buffers) depend on the launch ahead, unless the caller declared this one independent
                 if (overlap == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
                 // ... and, in a column-sharded chain, on the same launch of every other rank
@@ -643,7 +642,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                                 e = max(-100, (int)(amax >> 7) - 127 - kTop);
                             }
                             const float down = __uint_as_float((uint32_t)(127 - e) << 23), upg = __uint_as_float((uint32_t)(127 + e) << 23);
-                            if (FMT == 2 && bad && m < M && !plan.rounded) atomicOr(&ctl->bad_rows, 1u << m);
+                            if (FMT == 2 && bad && m < M) atomicOr(&ctl->bad_rows, 1u << m);
                             float gsum = 0.f, half_sum = 0.f;
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
@@ -671,10 +670,6 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                                         gsum = 0.f;
                                     }
                                 }
-                            }
-                            if (FMT == 2 && plan.rounded) {
-#pragma unroll
-                                for (int i = 0; i < F::kSW; ++i) xc[nb][i][0] = xc[nb][i][1] = 0u;
                             }
                             up[nb][0] = __shfl_sync(0xFFFFFFFFu, upg, 8 * t);          // lane (g' = 2t, *) holds activation row 2t
                             up[nb][1] = __shfl_sync(0xFFFFFFFFu, upg, 8 * t + 4);
@@ -894,12 +889,11 @@ inline bool gemv_mma_ok(int fmt, int64_t M, int64_t N, int64_t K, int group, int
 
 // `max_per`: slices per chunk of the launch's largest item.
 template <int FMT, int G, int NB, bool kRag, bool kI8>
-inline MmaPlan mma_plan(int M, int max_per, bool chunked, int cluster, bool rounded) {
+inline MmaPlan mma_plan(int M, int max_per, bool chunked, int cluster) {
     using F = MmaFmt<FMT, G>;
     using Sh = MmaShape<FMT, G, NB, kRag>;
     MmaPlan p;
     p.cluster = cluster;
-    p.rounded = rounded ? 1 : 0;
     auto up = [](int v) { return (v + 127) / 128 * 128; };
     p.scale_off = up(Sh::kRows * mma_pitch(max_per, F::kCode, kRag));
     p.x_off = up(p.scale_off + Sh::kRows * mma_pitch(max_per, F::kScale, kRag));
@@ -938,7 +932,7 @@ static int mma_max_clusters(void (*kernel)(Params...), int size, size_t smem) {
 // `units`: CTAs (clusters, when `cluster` > 1) the work can occupy.
 template <int FMT, int G, int NB, bool kRag, bool kGroup, bool kI8 = false>
 static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int units, int cluster, int max_per,
-                          bool chunked, int M, int x_dtype, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s, bool rounded = false) {
+                          bool chunked, int M, int x_dtype, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s) {
     auto kernel = gemv_mma_kernel<FMT, G, NB, kRag, kGroup, kI8>;
     static std::atomic<uint64_t> configured{0};
     const int32_t st = ensure_dynamic_smem(kernel, 227 * 1024, configured);
@@ -953,7 +947,7 @@ static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_
         room = f.load(std::memory_order_relaxed) - 1;
         if (room <= 0) { cluster = 1; room = num_sms(); }
     }
-    const MmaPlan plan = mma_plan<FMT, G, NB, kRag, kI8>(M, max_per, chunked, cluster, rounded);
+    const MmaPlan plan = mma_plan<FMT, G, NB, kRag, kI8>(M, max_per, chunked, cluster);
     const int grid = (units < room ? units : room) * cluster;
     return launch_maybe_overlapped(kernel, grid, kMmaThreads, plan.total, s, overlap != 0, cluster,
                                    probs, single, M, x_dtype, y_dtype, overlap, plan, peers);
@@ -968,17 +962,14 @@ inline int mma_cluster_for(int tiles, int chunks) {
 
 template <int FMT, int G>
 static int32_t mma_dispatch(bool rag, const ojx_e8t_gemv_problem& p, int tiles, int M, int x_dtype, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s) {
-    // 2.0 bits: batches that the tcgen05 kernel took before this one did see the same weights, rounded to fp16 once; smaller ones
-    // and K that is no multiple of 256 the exact ones
-    const bool rounded = FMT == 2 && !rag && (M > 8 || (M >= 4 && !(G == 32 && p.K % 2048 == 0)));
     const int per = mma_per_chunk(p.K), chunks = mma_chunks(p.K), cluster = mma_cluster_for(tiles, chunks);
     const bool chunked = chunks > 1;
     if (rag) return M <= 8 ? mma_launch<FMT, G, 1, true, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s)
                            : mma_launch<FMT, G, 2, true, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
     if (FMT == 0 && G == 32 && M == 1 && x_dtype == OJX_BF16)
         return mma_launch<0, 32, 1, false, false, true>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
-    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded)
-                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s, rounded);
+    return M <= 8 ? mma_launch<FMT, G, 1, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s)
+                  : mma_launch<FMT, G, 2, false, false>(nullptr, p, tiles, cluster, per, chunked, M, x_dtype, y_dtype, peers, overlap, s);
 }
 
 // One matrix; the caller has checked gemv_mma_ok and the alignment (16 bytes) of x, codes and scales.  `overlap` 3: nothing is read

@@ -90,12 +90,9 @@ _DECODE_SHAPES = [(1, 256), (17, 512), (100, 4096), (1000, 4352), (65, 14336), (
 @pytest.mark.parametrize("n,k", _DECODE_SHAPES)
 def test_decode_kernels_at_the_edges_of_their_tiles(P, bits, group, n, k):
     """One row of weights, remainders of a tile, one and several chunks of K (clusters that split them), K of any number of 32s."""
-    packed, scales, exact = _problem(P, bits, n, k, group)
+    packed, scales, wd = _problem(P, bits, n, k, group)             # fp32: the weights as they are, whatever the batch
     fmt = {1.0: 1, 1.5: 0, 2.0: 2}[bits]
     for m in (1, 2, 3, 8, 9, 16):
-        # from four (groups of 32 with K % 2048 == 0: nine) rows on, 2.0-bit weights are rounded to fp16 as in larger batches
-        rounded = bits == 2.0 and k % 256 == 0 and (m > 8 or (m >= 4 and not (group == 32 and k % 2048 == 0)))
-        wd = (exact.half().float() if rounded else exact)
         for dt in (torch.bfloat16, torch.float16):
             x = P.ops.generate(m * k, 8 + m, 1.0, dt, torch.device(DEV)).view(m, k).clone()
             x[:, ::97] *= 30
