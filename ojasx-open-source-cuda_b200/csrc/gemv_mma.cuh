@@ -6,7 +6,8 @@
 // Replaces the reference's scalar fused kernels (ojasx2/math/csrc/ojasx_math_core.hpp:444,580-634) and, for small batches,
 // _FusedE8GEMMFunction.forward (ojasx2/math/lattice.py:551-640).
 //
-// Weights enter the fp16 MMAs as EXACT fp16 values.  Ternary and 1.0-bit: coordinate * scale.  2.0-bit: (code - 2) * scale,
+// Weights enter the fp16 MMAs as EXACT fp16 values (sibling formats: for scales up to 32752; outputs over larger ones are computed
+// again in fp32, mma_dense).  Ternary and 1.0-bit: coordinate * scale.  2.0-bit: (code - 2) * scale,
 // which is exact where (code - 1.5) * scale is not; the missing 0.5 * scale per weight is 0.5 * sum over scale groups of
 // scale * (sum of the group's x), one extra MMA per two scales of a lane whose A registers ARE the scale words and whose B
 // registers hold the group sums as fp16 high and low parts.
@@ -82,7 +83,6 @@ struct MmaPlan {                                     // shared-memory layout, by
 struct MmaCtl {
     uint64_t never;                                  // tests: a barrier that nothing completes
     int abort_flag;
-    uint32_t bad_rows;                               // activation rows with Inf / NaN (2.0-bit format)
     ojx_e8t_gemv_problem prob;                       // the problem of a launch from a table
 };
 
@@ -217,16 +217,23 @@ __device__ __forceinline__ void mma_decode(uint32_t (&a)[4], const uint32_t (&w)
     a[0] = h2mul(lo.x, s2); a[1] = h2mul(lo.y, s2); a[2] = h2mul(hi.x, s2); a[3] = h2mul(hi.y, s2);
 }
 
-// One output of the 2.0-bit format in plain fp32: rows of x that hold Inf / NaN, where splitting code - 1.5 into
-// (code - 2) + 0.5 would turn an infinity into NaN.
-__device__ __noinline__ float mma_dense_2bit(const ojx_e8t_gemv_problem& P, int group, int x_dtype, int m, int n) {
-    float acc = 0.f;
+// One output of a sibling format in plain fp32, for sums `sum` that came out as Inf or NaN, by whatever cause: scales above 32752,
+// whose doubles ((code - 2) * scale, coordinates of +-2) fp16 does not have, and 2.0-bit products with Inf in x, where
+// (code - 2) + 0.5 turns an infinity into NaN.  1.0-bit sums over other scales are the dense product's as they are.
+template <int FMT>
+__device__ __noinline__ float mma_dense(const ojx_e8t_gemv_problem& P, int group, int x_dtype, int m, int n, float sum) {
     const int64_t r0 = (int64_t)n * P.K;
+    if (FMT == 1) {
+        bool large = false;
+        for (int i = 0; i < P.K / group; ++i) large = large || (P.scales[r0 / group + i] & 0x7FFFu) >= 0x7800u;
+        if (!large) return sum;
+    }
+    float acc = 0.f;
     for (int k = 0; k < P.K; ++k) {
         const int64_t at = r0 + k;
-        const float w = ((float)((P.packed[at >> 2] >> (2 * (int)(at & 3))) & 3) - 1.5f) *
-                        __half2float(__ushort_as_half(P.scales[at / group]));
-        acc = fmaf(load_any(P.x, x_dtype, (int64_t)m * P.K + k), w, acc);
+        const float c = FMT == 2 ? (float)((P.packed[at >> 2] >> (2 * (int)(at & 3))) & 3) - 1.5f
+                                 : (float)(int)(int8_t)((g_root_coords[2 * (int)P.packed[at >> 3] + (int)((at >> 2) & 1)] >> (8 * (int)(at & 3))) & 0xFFu);
+        acc = fmaf(load_any(P.x, x_dtype, (int64_t)m * P.K + k), c * __half2float(__ushort_as_half(P.scales[at / group])), acc);
     }
     for (int r = 0; r < P.lora_rank; ++r) acc = fmaf(P.lora_t[m * P.lora_rank + r], load_any(P.lora_b, x_dtype, (int64_t)r * P.N + n), acc);
     return acc;
@@ -360,7 +367,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
 
     // the launch that follows in the stream may start its own set-up now
     if (overlap) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    if (tid == 0) { ctl->abort_flag = 0; ctl->bad_rows = 0; }
+    if (tid == 0) ctl->abort_flag = 0;
     // this lane's copy of the table
     const uint32_t lane_off = kI8 ? lane * 4 : (FMT == 1 ? (lane & 7) * 16 : (lane & 15) * 8);
     const uint32_t lane_at = lane_off + base, lane_f = mma_lane_f(lane_off), lane_v = mma_lane_v(lane_at);
@@ -607,7 +614,6 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                             }
                         }
                         if (FMT == 2 || !xf16) {
-                            const int m = nb * 8 + g;
                             uint32_t m2 = 0;
 #pragma unroll
                             for (int j = 0; j < 8; ++j)
@@ -642,7 +648,6 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                                 e = max(-100, (int)(amax >> 7) - 127 - kTop);
                             }
                             const float down = __uint_as_float((uint32_t)(127 - e) << 23), upg = __uint_as_float((uint32_t)(127 + e) << 23);
-                            if (FMT == 2 && bad && m < M) atomicOr(&ctl->bad_rows, 1u << m);
                             float gsum = 0.f, half_sum = 0.f;
 #pragma unroll
                             for (int j = 0; j < 8; ++j) {
@@ -678,8 +683,8 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
             };
 
-            auto finish = [&](float sum, int col, int n, uint32_t bad_rows) {       // bias, store
-                if (FMT == 2 && ((bad_rows >> col) & 1u)) sum = mma_dense_2bit(P, G, x_dtype, col, n);
+            auto finish = [&](float sum, int col, int n) {                          // bias, store
+                if (FMT != 0 && (__float_as_uint(sum) & 0x7F800000u) == 0x7F800000u) sum = mma_dense<FMT>(P, G, x_dtype, col, n, sum);
                 if (P.bias != nullptr) sum += load_any(P.bias, x_dtype, n);
                 const int64_t at = (int64_t)col * (P.ldy > 0 ? P.ldy : N) + n;
                 store_any(P.y, y_dtype, at, sum);
@@ -710,7 +715,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                     if (chunk > cr) sum += *a;
                     if (chunk + cs < chunks || cs > 1) { *a = sum; return; }
                 }
-                finish(sum, q_col, n, ctl->bad_rows);
+                finish(sum, q_col, n);
             };
 
             int pair = 0, chunk = cr, act = 0, last_pair = -1, last_chunk = 0;
@@ -851,16 +856,13 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 // every CTA of the cluster holds its chunks' sums: each adds up a share of the outputs, chunks in CTA order
                 mma_cluster_sync();
                 const int ranks = min(cs, chunks);
-                uint32_t bad_rows = 0;
-                if (FMT == 2)
-                    for (int r = 0; r < ranks; ++r) bad_rows |= __float_as_uint(mma_ld_cluster(smem_u32(&ctl->bad_rows), r));
                 if (!dead)
                     for (int i = tid + cr * kMmaThreads; i < np * M * R; i += cs * kMmaThreads) {
                         const int row = i % R, pm = i / R, pr = pm / M, col = pm - pr * M, n = (b0 + pr * T) * 16 + row;
                         if (n >= N || n >= (b0 + nt) * 16) continue;
                         float sum = 0.f;
                         for (int r = 0; r < ranks; ++r) sum += mma_ld_cluster(base + plan.off_acc + i * 4, r);
-                        finish(sum, col, n, bad_rows);
+                        finish(sum, col, n);
                     }
                 mma_cluster_sync();         // nobody leaves, or writes these sums again, before all have read them
             } else if (chunks == 1) break;  // all tiles were one block

@@ -249,3 +249,26 @@ def test_sibling_formats_on_buffers_with_strides(P, bits):
     for fn in (lambda p, s: P.ops.linear_dx_lowbit(fmt, gy, p, s, n, k, 32), lambda p, s: P.ops._decode_lowbit(fmt, p, s, (n, k), torch.float32),
                lambda p, s: P.ops.linear_lowbit_lora(fmt, x, p, s, None, n, k, 32, t, b)):
         assert torch.equal(fn(packed, scales), fn(wide_pk, wide_sc))
+
+
+@pytest.mark.parametrize("bits,group,n,k", [(2.0, 32, 50, 4096), (2.0, 8, 17, 512), (2.0, 16, 40, 2912), (2.0, 32, 33, 14336),
+                                            (1.0, 32, 50, 4096), (1.0, 8, 17, 512), (1.0, 16, 40, 2912), (1.0, 32, 33, 14336)])
+def test_decode_kernels_with_scales_near_the_top_of_fp16(P, bits, group, n, k):
+    """Twice a scale above 32752 is no fp16 number: such rows still give the fp32 product, alone and with an adapter's term."""
+    packed, scales, _ = _problem(P, bits, n, k, group)
+    fmt, dev = int(bits), torch.device(DEV)
+    scales = scales.clone()
+    scales.view(n, -1)[3::4, ::5] = 33000.0
+    scales.view(n, -1)[7, 1] = 65504.0
+    wd = _packer(P, bits).unpack(packed, scales, (n, k), torch.float32).double()
+    a, b = torch.randn(k, 4, device=dev), torch.randn(4, n, device=dev)
+    for m in (1, 2, 5, 9, 16):
+        for dt in (torch.bfloat16, torch.float16):
+            x = P.ops.generate(m * k, 8 + m, 1.0, dt, dev).view(m, k)
+            y = P.ops._linear(fmt, x, packed, scales, None, n, k, group, torch.float32, P._cabi.OJX_LINEAR_DECODE)
+            ref, bound = x.double() @ wd.t(), x.double().abs() @ wd.abs().t()
+            assert float(((y.double() - ref).abs() / bound.clamp_min(1e-30)).max()) <= 5e-6, (m, dt)
+            y = P.ops.layer_forward_adapter(fmt, x, packed, scales, None, n, k, group, False, a.to(dt), b.to(dt), 0.5, torch.float32)
+            low = 0.5 * ((x.double() @ a.to(dt).double()) @ b.to(dt).double())
+            bound += 0.5 * ((x.double().abs() @ a.to(dt).double().abs()) @ b.to(dt).double().abs())
+            assert float(((y.double() - ref - low).abs() / bound.clamp_min(1e-30)).max()) <= 5e-6, (m, dt)
