@@ -383,7 +383,6 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
     const int64_t tiles = (N + 15) / 16;
     const int t0 = (int)(tiles * (blockIdx.x / cs) / (gridDim.x / cs)), t1 = (int)(tiles * (blockIdx.x / cs + 1) / (gridDim.x / cs));
     const bool signal = peers.sync != nullptr && (peers.mode & OJX_GEMV_SIGNAL_PEERS) != 0;
-    const bool waits = peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS) != 0;
 
     uint32_t xb[NB][8][4];                      // B fragments: [block][8-weight chunk j][k 0-1, 2-3, 4-5, 6-7 of the chunk]; kI8: [j][digit pair m, k half r] at [2 m + r]
     uint32_t xc[NB][F::kSW][2];                 // 2.0-bit: half the scale groups' sums of x, high and low parts, two groups each
@@ -429,7 +428,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
         const uint32_t rc = code_bytes(K), rs = (uint32_t)K / G * 2;
         // blocks of tiles: all of them when K is one chunk, else as many as there is room for running sums; chunk-major inside
         for (int b0 = t0; b0 < t1; b0 += kMmaAccTiles) {
-            const int nt = chunks == 1 && cs == 1 ? t1 - b0 : min(kMmaAccTiles, t1 - b0), np = (nt + T - 1) / T;
+            const int nt = chunks == 1 ? t1 - b0 : min(kMmaAccTiles, t1 - b0), np = (nt + T - 1) / T;
             const int total = chunks > cr ? np * ((chunks - cr + cs - 1) / cs) : 0;
 
             // ---- loader: warp w copies rows w and w + 16 of an item, 16-byte vector lane, lane + 32, ... of the codes and then of
@@ -487,20 +486,18 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
                 asm volatile("cp.async.commit_group;" ::: "memory");
             };
-            // packed weights of a static launch do not depend on the launch ahead: their copies start before it has drained.  x does,
-            // and where peers are waited for it is written by them until then: its copies follow both waits.
-            const bool late_x = first_run && (overlap == 1 || waits);
-            for (int i = 0; i < D; ++i) issue(i, !late_x);
+            // packed weights of a static launch do not depend on the launch ahead: their copies start before it has drained
+            for (int i = 0; i < D; ++i) issue(i, !(first_run && overlap == 1));
             if (first_run) {
                 if (kGroup) mma_fill_table<FMT, kI8>(smem, tid);
                 // activations (and the output buffers) depend on the launch ahead, unless the caller declared this one independent
                 if (overlap == 1) asm volatile("griddepcontrol.wait;" ::: "memory");
                 // ... and, in a column-sharded chain, on the same launch of every other rank
-                if (waits) {
+                if (peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS)) {
                     if (tid == 0) peer_wait(peers);
                     __syncthreads();
                 }
-                if (late_x && x_staged) {
+                if (overlap == 1 && x_staged) {
                     for (int i = 0; i < D && i < total; ++i)
                         if (i % np == 0) copy_x(cr + i / np * cs, base + plan.off_ring + i * plan.stage_bytes);
                     asm volatile("cp.async.wait_all;" ::: "memory");
@@ -710,7 +707,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
                 for (int o = 1; o < (1 << qs); o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
                 if (q_sub != 0 || q_col >= M || n >= N || n >= (b0 + nt) * 16) return;
-                if (chunks > 1 || cs > 1) {                              // (a cluster adds up what its CTAs left here, of one chunk too)
+                if (chunks > 1) {
                     float* a = acc_sums + (pair * M + q_col) * R + q_row;
                     if (chunk > cr) sum += *a;
                     if (chunk + cs < chunks || cs > 1) { *a = sum; return; }
@@ -852,6 +849,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
             __syncthreads();
             if (!dead && last_pair >= 0) reduce(last_pair, last_chunk, buf ^ 1);
             first_run = false;
+            if (chunks == 1) break;                                   // all tiles were one block, the cluster's first CTA had its chunk and stored
             if (cs > 1) {
                 // every CTA of the cluster holds its chunks' sums: each adds up a share of the outputs, chunks in CTA order
                 mma_cluster_sync();
@@ -865,7 +863,7 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                         finish(sum, col, n);
                     }
                 mma_cluster_sync();         // nobody leaves, or writes these sums again, before all have read them
-            } else if (chunks == 1) break;  // all tiles were one block
+            }
         }
     }
 
@@ -951,8 +949,10 @@ static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_
     }
     const MmaPlan plan = mma_plan<FMT, G, NB, kRag, kI8>(M, max_per, chunked, cluster);
     const int grid = (units < room ? units : room) * cluster;
+    // a launch that waits for its peers reads x after them whatever it may read before the launch ahead has ended
+    const bool late_x = peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS) != 0;
     return launch_maybe_overlapped(kernel, grid, kMmaThreads, plan.total, s, overlap != 0, cluster,
-                                   probs, single, M, x_dtype, y_dtype, overlap, plan, peers);
+                                   probs, single, M, x_dtype, y_dtype, overlap == 0 && late_x ? 1 : overlap, plan, peers);
 }
 
 // K of several chunks over few tiles: the CTAs of a cluster split the chunks, so that each prepares x for its own chunks only
