@@ -391,8 +391,8 @@ int32_t ojx_e8t_enable_peer_access(int32_t peer_device);
 /*
  * Prefill-shape linear (large M) on the tcgen05 tensor cores.  Same contract as ojx_e8t_gemv;
  * replaces the reference's TileLang builder (ojasx2/tilelang_kernels.py:277-363) and the
- * unpack + F.linear path (lattice.py:613-624).  Requires K % 256 == 0, group 32 or 16, bf16 or fp16 x (any M >= 1:
- * groups of 16, which have no decode-shape kernel of their own, are best sent here at every batch size).
+ * unpack + F.linear path (lattice.py:613-624).  Requires K % 32 == 0 (K % 256 != 0 costs a padded copy of the weights in the
+ * workspace), group 32 or 16, bf16 or fp16 x and any M >= 1.
  * `workspace` (256-byte aligned, size from ojx_e8t_gemm_workspace_bytes) holds a status block and,
  * for bf16 activations, one power-of-two factor per token row and the fp16 copy of the activations
  * scaled by it (each row's largest magnitude is brought into [2^14, 2^15); the row's outputs are
@@ -410,12 +410,12 @@ int32_t ojx_e8t_gemm(const void* x, int32_t x_dtype, int64_t M,
 int32_t ojx_e8t_gemm_status(const void* workspace, void* stream);
 
 /*
- * The same prefill kernel for the two sibling formats (`bits` 2 or 1; group 8, 16 or 32, K % 256 == 0, 16-bit activations,
+ * The same prefill kernel for the two sibling formats (`bits` 2 or 1; group 8, 16 or 32, K % 32 == 0, 16-bit activations,
  * workspace and status exactly as for ojx_e8t_gemm): the decoder warps read the 2-bit / 1-bit codes instead of the
  * ternary ranks.  Replaces the 2.0-bit / 1.0-bit branches of _FusedE8GEMMFunction.forward
  * (ojasx2/math/lattice.py:596-624) for batches of tokens.  The weights enter the tensor cores as fp16: for 1 bit
- * coordinate * scale is exact; for 2 bits (code - 1.5) * scale is rounded to fp16 once, i.e. the product equals
- * x . decode_2bit(fp16)^T with fp32 accumulation.
+ * coordinate * scale is exact; for 2 bits and K % 256 == 0 (code - 1.5) * scale is rounded to fp16 once, i.e. the product
+ * equals x . decode_2bit(fp16)^T with fp32 accumulation, for other K it enters in two parts and is exact.
  */
 int32_t ojx_e8t_gemm_lowbit(int32_t bits, const void* x, int32_t x_dtype, int64_t M,
                             const uint8_t* packed, const uint16_t* scales, const void* bias,

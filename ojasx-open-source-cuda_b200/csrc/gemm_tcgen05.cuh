@@ -34,6 +34,8 @@
 
 #include <cuda.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "gemv.cuh"
 
@@ -70,24 +72,28 @@ struct GemmParams {
     int rows;                      // weight rows per CTA tile: 128 or 256
     int bn;                        // tokens per CTA tile (MMA N): 128 or 256
     const float* up;               // per-token output factors 2^e written by the pre-pass (null: 1)
+    const float* row_up;           // per weight row: output factors 2^e of scales that were brought into fp16's middle (null: 1)
 };
 
 // Activation pre-pass: a group of TPR threads (a warp for rows of up to 4096 elements, else the whole CTA)
 // takes one token row, finds its largest magnitude, then writes the row as fp16 scaled by the power of two
 // that brings that magnitude into [2^14, 2^15), and the inverse factor for the epilogue.  Rows of up to
 // TPR * 8 * VECS elements stay in registers between the two steps (one global read); longer rows are read
-// twice.
-template <int TPR, int VECS>
-__global__ void __launch_bounds__(256) normalize_rows_bf16_to_f16_kernel(const __nv_bfloat16* __restrict__ x,
-                                                                          __half* __restrict__ out, float* __restrict__ up,
-                                                                          int64_t M, int64_t K) {
+// twice.  kSplit (2.0-bit weights in two parts): fp16 rows are not scaled, rows are written twice, each time filled up with zeros
+// to a multiple of 64, the second time with zeros in place of Inf and NaN.
+template <int TPR, int VECS, typename T, bool kSplit>
+__global__ void __launch_bounds__(256) normalize_rows_to_f16_kernel(const T* __restrict__ x, __half* __restrict__ out, float* __restrict__ up,
+                                                                     int64_t M, int64_t K) {
+    constexpr bool kBf16 = std::is_same<T, __nv_bfloat16>::value;
+    static_assert(kBf16 || kSplit, "fp16 rows are taken as they are");
     __shared__ uint32_t warp_max[8];
     constexpr int kRowsPerCta = 256 / TPR;
     const int t = threadIdx.x % TPR;
     const int64_t row = (int64_t)blockIdx.x * kRowsPerCta + threadIdx.x / TPR;
     const bool live = row < M;                                            // whole warps share `live`
-    const uint4* src = reinterpret_cast<const uint4*>(x + (live ? row : 0) * K);   // K % 256 == 0: rows are 16-byte aligned
-    uint4* dst = reinterpret_cast<uint4*>(out + (live ? row : 0) * K);
+    const int64_t part = kSplit ? (K + 63) / 64 * 8 : K / 8;              // vectors of a written row, of one part
+    const uint4* src = reinterpret_cast<const uint4*>(x + (live ? row : 0) * K);   // K % 8 == 0: rows are 16-byte aligned
+    uint4* dst = reinterpret_cast<uint4*>(out) + (live ? row : 0) * part * (kSplit ? 2 : 1);
     const int64_t vecs = live ? K / 8 : 0;
     const bool resident = vecs <= (int64_t)TPR * VECS;
     uint4 keep[VECS];
@@ -98,34 +104,36 @@ __global__ void __launch_bounds__(256) normalize_rows_bf16_to_f16_kernel(const _
             const int64_t i = t + TPR * j;
             keep[j] = i < vecs ? __ldg(src + i) : make_uint4(0, 0, 0, 0);
         }
-#pragma unroll
-        for (int j = 0; j < VECS; ++j) {
-            const uint32_t w[4] = {keep[j].x, keep[j].y, keep[j].z, keep[j].w};
-#pragma unroll
-            for (int q = 0; q < 4; ++q) m = max(m, max((w[q] << 16) & 0x7FFFFFFFu, w[q] & 0x7FFF0000u));
-        }
-    } else {
-        for (int64_t i = t; i < vecs; i += TPR) {
-            const uint4 v = __ldg(src + i);
+    }
+    float down = 1.f;
+    if constexpr (kBf16) {
+        auto largest = [&](const uint4& v) {
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) m = max(m, max((w[q] << 16) & 0x7FFFFFFFu, w[q] & 0x7FFF0000u));
+        };
+        if (resident) {
+#pragma unroll
+            for (int j = 0; j < VECS; ++j) largest(keep[j]);
+        } else {
+            for (int64_t i = t; i < vecs; i += TPR) largest(__ldg(src + i));
         }
-    }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
-    if (TPR > 32) {
-        if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
-        __syncthreads();
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+        if (TPR > 32) {
+            if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+            __syncthreads();
 #pragma unroll
-        for (int w = 0; w < 8; ++w) m = max(m, warp_max[w]);
+            for (int w = 0; w < 8; ++w) m = max(m, warp_max[w]);
+        }
+        int e = 0;
+        const int ex = (int)((m >> 23) & 0xFFu);
+        if (ex != 0 && ex != 0xFF) e = max(-100, min(100, ex - 127 - 14));
+        down = __int_as_float((127 - e) << 23);
+        if (t == 0 && live) up[row] = __int_as_float((127 + e) << 23);
     }
-    int e = 0;
-    const int ex = (int)((m >> 23) & 0xFFu);
-    if (ex != 0 && ex != 0xFF) e = max(-100, min(100, ex - 127 - 14));
-    const float down = __int_as_float((127 - e) << 23);
-    if (t == 0 && live) up[row] = __int_as_float((127 + e) << 23);
     auto convert = [&](const uint4& v) {
+        if constexpr (!kBf16) return v;
         const uint32_t w[4] = {v.x, v.y, v.z, v.w};
         uint32_t o[4];
 #pragma unroll
@@ -135,15 +143,37 @@ __global__ void __launch_bounds__(256) normalize_rows_bf16_to_f16_kernel(const _
         }
         return make_uint4(o[0], o[1], o[2], o[3]);
     };
+    auto write = [&](int64_t i, const uint4& v) {
+        const uint4 h = convert(v);
+        dst[i] = h;
+        if constexpr (kSplit) {
+            uint32_t o[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if ((o[q] & 0x7C00u) == 0x7C00u) o[q] &= 0xFFFF0000u;
+                if ((o[q] & 0x7C000000u) == 0x7C000000u) o[q] &= 0x0000FFFFu;
+            }
+            dst[part + i] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    };
     if (resident) {
 #pragma unroll
         for (int j = 0; j < VECS; ++j) {
             const int64_t i = t + TPR * j;
-            if (i < vecs) dst[i] = convert(keep[j]);
+            if (i < vecs) write(i, keep[j]);
         }
     } else {
-        for (int64_t i = t; i < vecs; i += TPR) dst[i] = convert(__ldg(src + i));
+        for (int64_t i = t; i < vecs; i += TPR) write(i, __ldg(src + i));
     }
+    if (kSplit && live)
+        for (int64_t i = vecs + t; i < part; i += TPR) dst[i] = dst[part + i] = make_uint4(0, 0, 0, 0);
+}
+template <typename T, bool kSplit>
+static int32_t normalize_rows(const void* x, void* out, float* up, int64_t M, int64_t K, cudaStream_t s) {
+    const T* xp = static_cast<const T*>(x);
+    if (K <= 4096) normalize_rows_to_f16_kernel<32, 16, T, kSplit><<<(unsigned)((M + 7) / 8), 256, 0, s>>>(xp, static_cast<__half*>(out), up, M, K);
+    else normalize_rows_to_f16_kernel<256, 8, T, kSplit><<<(unsigned)M, 256, 0, s>>>(xp, static_cast<__half*>(out), up, M, K);
+    return launch_status();
 }
 
 // ---- PTX wrappers (mbarrier helpers live in common.cuh) ------------------------------------------
@@ -238,14 +268,15 @@ __device__ __forceinline__ void gemm_store32(T* __restrict__ y, int64_t N, int n
 // One epilogue warp's share of a finished tile: TMEM lanes 32 * warp .. of both row blocks, all token columns.
 // Kept out of line so that its registers are allocated independently of the decoders' inner loop.
 __device__ __noinline__ void gemm_drain_tile(void* __restrict__ y, int y_dtype, const void* __restrict__ bias_ptr, int bias_dtype,
-                                             const float* __restrict__ up, int M, int N, int y_stride, int rows, int bn,
-                                             uint32_t tmem_base, int warp, int lane, int n_blk, int m_blk) {
+                                             const float* __restrict__ up, const float* __restrict__ row_up, int M, int N, int y_stride,
+                                             int rows, int bn, uint32_t tmem_base, int warp, int lane, int n_blk, int m_blk) {
     const int blocks = bn / 32;
     for (int h = 0; h < rows / kGemmHalf; ++h) {
         const int n = n_blk * rows + h * kGemmHalf + warp * 32 + lane;
         const bool live = n < N;
         float bias = 0.f;
         if (bias_ptr != nullptr && live) bias = load_any(bias_ptr, bias_dtype, n);
+        const float ru = row_up != nullptr && live ? __ldg(row_up + n) : 1.f;
         const uint32_t taddr = tmem_base + ((uint32_t)(warp * 32) << 16) + h * kGemmBN;
         // Token factors (lane l keeps the factor of token m0 + l) and accumulator blocks both travel one
         // 32-token block ahead of their use, so neither the global nor the TMEM load latency is exposed.
@@ -253,9 +284,13 @@ __device__ __noinline__ void gemm_drain_tile(void* __restrict__ y, int y_dtype, 
             const int m = m_blk * bn + cb * 32 + lane;
             return (up != nullptr && cb < blocks && m < M) ? __ldg(up + m) : 1.0f;
         };
-        auto store = [&](int cb, const uint32_t (&v)[32], float up_lane) {
+        auto store = [&](int cb, uint32_t (&v)[32], float up_lane) {
             const int m0 = m_blk * bn + cb * 32;
             if (m0 >= M) return;                                   // warp-uniform
+            if (row_up != nullptr) {
+#pragma unroll
+                for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * ru);
+            }
             if (y_dtype == OJX_BF16) gemm_store32(static_cast<__nv_bfloat16*>(y), y_stride, n, m0, M, v, up_lane, bias, live);
             else if (y_dtype == OJX_F16) gemm_store32(static_cast<__half*>(y), y_stride, n, m0, M, v, up_lane, bias, live);
             else gemm_store32(static_cast<float*>(y), y_stride, n, m0, M, v, up_lane, bias, live);
@@ -303,12 +338,24 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
     return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// a * b - c, c being a * b rounded: what the rounding left
+__device__ __forceinline__ uint32_t hrest2_u32(uint32_t a, uint32_t b, uint32_t c) {
+    uint32_t r;
+    asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c ^ 0x80008000u));
+    return r;
+}
+
 // kDX = false: y[M, N] = x . W^T, contraction over K (the weights' row direction), p.N = weight rows, p.K = columns.
 // kDX = true:  dX[M, K] = dY . W, contraction over the weight ROWS.  The roles are swapped in the parameters: p.N is
 //              the number of weight COLUMNS (the output's feature dimension, tiled like N above) and p.K the number
 //              of weight rows (the contraction length, any positive value: the last block is zero-filled).  The
 //              decoded weights enter the MMA as an MN-major operand, so a decoded rank is still one 16-byte store.
-template <bool kDX, int kFmt = 0, int kG = 32> // kFmt: 0 ternary codes, 2 the 2.0-bit format, 1 the 1.0-bit format; kG: weights per scale (8 and 16 only for the sibling formats)
+// kFmt: 0 ternary codes, 2 the 2.0-bit format, 1 the 1.0-bit format; kG: weights per scale (8 only for the sibling formats).
+// kSplit: 2.0-bit weights in two fp16 parts, the rounded (code - 1.5) * scale against x and what the rounding left (exact, one fused
+// multiply-add) against the finite x, one after the other along the contraction; x has both beside each other.
+// Twice the MMAs and tiles for weights that are exact: 333 tokens, 2912 -> 2000: 65 us (one rounded part 41, scalar fp32 kernel
+// 2940); error of fp16 outputs against 64 bits 2.077e-4 (one rounded part 2.87e-4, scalar fp32 kernel 2.076e-4).
+template <bool kDX, int kFmt = 0, int kG = 32, bool kSplit = false>
 __global__ void __launch_bounds__(kGemmThreads, 1)
 gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams p) {
     extern __shared__ uint8_t smem_raw[];
@@ -567,7 +614,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             const int row = min(n_blk * p.rows + r, p.N - 1);
             const uint4* cptr = reinterpret_cast<const uint4*>(p.packed + row * row_bytes);
             const uint4* sptr = reinterpret_cast<const uint4*>(p.scales + row * row_scales);
-            const int chunks = p.K / 256;
+            const int chunks = p.K / 256, part_blocks = kSplit ? k_blocks / 2 : k_blocks;
+            for (int part = 0; part < (kSplit ? 2 : 1) && ok; ++part) {
             uint4 cv[kVec], sv[kSV];
 #pragma unroll
             for (int i = 0; i < kVec; ++i) cv[i] = __ldg(cptr + i);
@@ -587,7 +635,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                 }
 #pragma unroll
                 for (int q = 0; q < 4; ++q, ++it) {
-                    if (ch * 4 + q >= k_blocks) break;                             // padded rows: the last chunk may be cut short
+                    if (ch * 4 + q >= part_blocks) break;                             // padded rows: the last chunk may be cut short
                     const int s = it % kGemmStages;
                     const uint32_t ph = (it / kGemmStages) & 1u;
                     if (!mbar_wait(empty_bar(s), ph ^ 1u, abort_flag, 4)) { ok = false; break; }
@@ -611,9 +659,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                         for (int j = 0; j < 4; ++j) {
                             const int jj = half * 4 + j;
                             const int si = (64 * q + 8 * jj) / kG;                 // scale of this 8-weight chunk inside the 256 k
-                            const uint32_t sc2 = prmt(sw[si >> 1], 0u, (si & 1) == 0 ? 0x1010u : 0x3232u);
-                            const uint4 v = make_uint4(hmul2_u32(lo8[j].x, sc2), hmul2_u32(lo8[j].y, sc2),
-                                                       hmul2_u32(hi8[j].x, sc2), hmul2_u32(hi8[j].y, sc2));
+                            uint32_t sc2 = prmt(sw[si >> 1], 0u, (si & 1) == 0 ? 0x1010u : 0x3232u);
+                            if (kSplit && part == 1 && (sc2 & 0x7C00u) == 0x7C00u) sc2 = 0u;      // Inf and NaN scales: the first part has them
+                            uint4 v = make_uint4(hmul2_u32(lo8[j].x, sc2), hmul2_u32(lo8[j].y, sc2),
+                                                 hmul2_u32(hi8[j].x, sc2), hmul2_u32(hi8[j].y, sc2));
+                            if (kSplit && part == 1) v = make_uint4(hrest2_u32(lo8[j].x, sc2, v.x), hrest2_u32(lo8[j].y, sc2, v.y),
+                                                                    hrest2_u32(hi8[j].x, sc2, v.z), hrest2_u32(hi8[j].y, sc2, v.w));
                             *reinterpret_cast<uint4*>(arow + ((jj ^ (r & 7)) << 4)) = v;
                         }
                     }
@@ -621,6 +672,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
                     __syncwarp();
                     if (lane == 0) mbar_arrive(full_bar(s));
                 }
+            }
             }
         }
         } else {
@@ -703,7 +755,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_x, const GemmParams
             ok = __all_sync(0xFFFFFFFFu, ok);          // warp-uniform decision before the aligned TMEM loads
             if (!ok) break;
             tc_fence_after();
-            gemm_drain_tile(p.y, p.y_dtype, p.bias, p.bias_dtype, p.up, p.M, p.N, p.y_stride, p.rows, p.bn, tmem_base, warp, lane, n_blk, m_blk);
+            gemm_drain_tile(p.y, p.y_dtype, p.bias, p.bias_dtype, p.up, p.row_up, p.M, p.N, p.y_stride, p.rows, p.bn, tmem_base, warp, lane, n_blk, m_blk);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(tempty_bar(0));
@@ -755,23 +807,34 @@ inline GemmKernelFn gemm_kernel_for(int fmt, int group, int* slot) {
     return nullptr;
 }
 
+inline GemmKernelFn gemm_split_kernel_for(int group, int* slot) {
+    if (group == 32) { *slot = 8; return gemm_tcgen05_kernel<false, 2, 32, true>; }
+    if (group == 16) { *slot = 9; return gemm_tcgen05_kernel<false, 2, 16, true>; }
+    if (group == 8) { *slot = 10; return gemm_tcgen05_kernel<false, 2, 8, true>; }
+    return nullptr;
+}
+
 inline bool gemm_fast_ok(int64_t M, int64_t N, int64_t K, int x_dtype) {
     return M >= 1 && N >= 1 && K >= 32 && K % 32 == 0 &&
-           (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && M < (1 << 30) && N < (1 << 30) && K < (1 << 30);
+           (x_dtype == OJX_BF16 || x_dtype == OJX_F16) && M < (1 << 30) && N < (1 << 30) && K < (1 << 29);
 }
 
 // Scratch: a 256-byte status block (word 0: give-up code of a bounded wait; zeroed by every call), the
 // per-token output factors (M floats, padded to 256 bytes), room for an fp16 copy of the activations and, when K is not
-// a multiple of 256, the weights with every row padded to one (sized for the largest format, 2 bits with groups of 8).
+// a multiple of 256, the weights with every row padded to one (sized for the largest format, 2 bits with groups of 8), a factor
+// per weight row and, for the 2.0-bit format, the activations' second part.
 inline size_t pad256(size_t n) { return (n + 255) & ~(size_t)255; }
 inline size_t gemm_up_bytes(int64_t M) { return pad256((size_t)M * 4); }
 inline int64_t gemm_padded_k(int64_t K) { return (K + 255) / 256 * 256; }
-size_t gemm_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
+inline bool gemm_split(int fmt, int64_t K) { return fmt == 2 && K % 256 != 0; }
+inline size_t gemm_x_row_bytes(int fmt, int64_t K) { return gemm_split(fmt, K) ? (size_t)((K + 63) / 64 * 64) * 4 : (size_t)K * 2; }
+size_t gemm_fmt_workspace_bytes(int fmt, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || K <= 0) return 256;
-    size_t need = 256 + gemm_up_bytes(M) + (size_t)M * (size_t)K * 2;
-    if (K % 256 != 0 && N > 0) need = pad256(need) + 2 * (size_t)N * (size_t)(gemm_padded_k(K) / 4);
+    size_t need = 256 + gemm_up_bytes(M) + (size_t)M * gemm_x_row_bytes(fmt, K);
+    if (K % 256 != 0 && N > 0) need = pad256(need) + 2 * (size_t)N * (size_t)(gemm_padded_k(K) / 4) + (size_t)N * 4;
     return need;
 }
+size_t gemm_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) { return gemm_fmt_workspace_bytes(2, M, N, K); }
 
 // Copies rows of `src_bytes` (even) to rows of `dst_bytes` (a multiple of 16), the rest of a row zero: codes or scales of
 // a matrix whose K is not a multiple of 256, whose rows start at any even address, for the 16-byte loads of the decoders.
@@ -794,9 +857,34 @@ __global__ void __launch_bounds__(256) pad_rows_kernel(const uint8_t* __restrict
     }
 }
 
+// The scales of such a matrix, brought into the middle of fp16: a row's are multiplied by the power of two that takes its largest
+// finite one into [2^13, 2^14), the inverse goes to row_up.  Twice a scale above 32752 (1.0 bit) and 1.5 times one above 43669 are
+// no fp16 numbers, and what rounding (code - 1.5) * scale leaves of scales below 2^-13 neither.  Warp = one row; scales smaller than
+// the row's largest by 2^-27 and more lose bits, 2^-38 of it.
+__global__ void __launch_bounds__(256) pad_scales_kernel(const uint16_t* __restrict__ src, uint16_t* __restrict__ dst, float* __restrict__ row_up,
+                                                          int64_t rows, int per_row, int padded) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t row = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (int64_t)gridDim.x * 8) {
+        const uint16_t* s = src + row * per_row;
+        float top = 0.f;
+        for (int i = lane; i < per_row; i += 32) {
+            const uint32_t mag = __ldg(s + i) & 0x7FFFu;
+            if (mag < 0x7C00u) top = fmaxf(top, __half2float(__ushort_as_half((uint16_t)mag)));
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, o));
+        const int e = top > 0.f ? 13 - ((int)(__float_as_uint(top) >> 23) - 127) : 0;         // in [-2, 37]
+        const float f = __uint_as_float((uint32_t)(127 + e) << 23);
+        for (int i = lane; i < padded; i += 32)
+            dst[row * padded + i] = i < per_row ? __half_as_ushort(__float2half_rn(__half2float(__ushort_as_half(__ldg(s + i))) * f)) : 0;
+        if (lane == 0) row_up[row] = __uint_as_float((uint32_t)(127 - e) << 23);
+    }
+}
+
 // fmt: 0 ternary codes (3 bytes per 16 weights), 2 the 2.0-bit format (one byte per 4 weights, weight =
-// (code - 1.5) * scale rounded to fp16 once, exactly the fp16 output of its decoder), 1 the 1.0-bit format (one byte
-// per 8 weights, coordinate * scale exact in fp16).
+// (code - 1.5) * scale rounded to fp16 once, exactly the fp16 output of its decoder; where K is no multiple of 256, a form that
+// the fp32 kernel used to serve, in two parts and so exact), 1 the 1.0-bit format (one byte per 8 weights, coordinate * scale
+// exact in fp16).
 int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint8_t* packed, const uint16_t* scales,
                       const void* bias, int64_t N, int64_t K, int group, void* y, int y_dtype,
                       void* workspace, size_t workspace_bytes, cudaStream_t s) {
@@ -807,20 +895,22 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
     OJX_RETURN_IF(check_arch() != OJX_OK, OJX_ERR_ARCH);
     if (fmt == 0) group = effective_group(group);
     int slot = 0;
-    const GemmKernelFn kernel = gemm_kernel_for<false>(fmt, group, &slot);      // sibling formats: groups of 8, 16 or 32
+    const bool split = gemm_split(fmt, K);
+    const GemmKernelFn kernel = split ? gemm_split_kernel_for(group, &slot) : gemm_kernel_for<false>(fmt, group, &slot);      // sibling formats: groups of 8, 16 or 32
     OJX_RETURN_IF(kernel == nullptr || !gemm_fast_ok(M, N, K, x_dtype), OJX_ERR_UNSUPPORTED);
     OJX_RETURN_IF(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(packed) |
                     reinterpret_cast<uintptr_t>(scales)) & 15) != 0, OJX_ERR_ALIGN);
     const bool convert = x_dtype == OJX_BF16;
     const bool ragged = K % 256 != 0;
-    const size_t need = (convert || ragged) ? gemm_workspace_bytes_impl(M, N, K) : 256;
+    const size_t need = (convert || ragged) ? gemm_fmt_workspace_bytes(fmt, M, N, K) : 256;
     OJX_RETURN_IF(!workspace || workspace_bytes < need, OJX_ERR_WORKSPACE);
     OJX_RETURN_IF((reinterpret_cast<uintptr_t>(workspace) & 255) != 0, OJX_ERR_ALIGN);
     PFN_encodeTiled encode = get_encode_tiled();
     OJX_RETURN_IF(encode == nullptr, OJX_ERR_LAUNCH);
 
     float* up = convert ? reinterpret_cast<float*>(static_cast<uint8_t*>(workspace) + 256) : nullptr;
-    void* x_f16 = convert ? static_cast<void*>(static_cast<uint8_t*>(workspace) + 256 + gemm_up_bytes(M)) : const_cast<void*>(x);
+    const size_t x_row = gemm_x_row_bytes(fmt, K);
+    void* x_f16 = convert || split ? static_cast<void*>(static_cast<uint8_t*>(workspace) + 256 + gemm_up_bytes(M)) : const_cast<void*>(x);
 
     // Tile shape: the choice that minimises (waves over the SMs) x (work per tile), with a small
     // penalty for the shapes that reuse each fetched x tile or decoded weight tile less.
@@ -838,30 +928,33 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
             }
     }
 
-    static std::atomic<uint64_t> configured[8];                  // per kernel; one bit per device: the opt-in is per context
+    static std::atomic<uint64_t> configured[11];                 // per kernel; one bit per device: the opt-in is per context
     OJX_RETURN_IF(ensure_dynamic_smem(kernel, kGemmSmemBytes, configured[slot]) != OJX_OK, OJX_ERR_LAUNCH);
-    if (convert) {
-        if (K <= 4096)
-            normalize_rows_bf16_to_f16_kernel<32, 16><<<(unsigned)((M + 7) / 8), 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K);
-        else
-            normalize_rows_bf16_to_f16_kernel<256, 8><<<(unsigned)M, 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(x), static_cast<__half*>(x_f16), up, M, K);
-        if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
+    if (convert || split) {
+        const int32_t st = split ? (convert ? normalize_rows<__nv_bfloat16, true>(x, x_f16, up, M, K, s) : normalize_rows<__half, true>(x, x_f16, up, M, K, s))
+                                 : normalize_rows<__nv_bfloat16, false>(x, x_f16, up, M, K, s);
+        OJX_RETURN_IF(st != OJX_OK, st);
     }
 
     // K not a multiple of 256: the kernel reads a padded copy of the weights; its contraction stops at K
-    const int64_t Kp = gemm_padded_k(K);
+    const int64_t Kp = gemm_padded_k(K), k_len = split ? (int64_t)(x_row / 2) : K;
+    float* row_up = nullptr;
     if (ragged) {
         auto code_bytes = [&](int64_t k) { return fmt == 0 ? k * 3 / 16 : (fmt == 2 ? k / 4 : k / 8); };
-        uint8_t* wp = static_cast<uint8_t*>(workspace) + pad256(256 + gemm_up_bytes(M) + (size_t)M * (size_t)K * 2);
+        uint8_t* wp = static_cast<uint8_t*>(workspace) + pad256(256 + gemm_up_bytes(M) + (size_t)M * x_row);
         uint8_t* wsc = wp + N * code_bytes(Kp);                      // a multiple of 16 bytes per row
         auto pad = [&](const void* src, uint8_t* dst, int64_t sb, int64_t db) {
             const int64_t blocks = (N * (db / 16) + 255) / 256, cap = (int64_t)num_sms() * 32;
             pad_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(static_cast<const uint8_t*>(src), dst, N, (int)sb, (int)db);
         };
         pad(packed, wp, code_bytes(K), code_bytes(Kp));
-        pad(scales, wsc, K / group * 2, Kp / group * 2);
+        if (fmt != 2) {
+            pad(scales, wsc, K / group * 2, Kp / group * 2);
+        } else {
+            row_up = reinterpret_cast<float*>(wsc + N * (Kp / group * 2));
+            const int64_t blocks = (N + 7) / 8, cap = (int64_t)num_sms() * 32;
+            pad_scales_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(scales, reinterpret_cast<uint16_t*>(wsc), row_up, N, (int)(K / group), (int)(Kp / group));
+        }
         if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
         packed = wp;
         scales = reinterpret_cast<const uint16_t*>(wsc);
@@ -872,11 +965,11 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
     auto launch_region = [&](int64_t n0, int64_t m0, int rows, int bn, int tile_limit) -> int32_t {
         const int64_t Ns = N - n0, Ms = M - m0;
         CUtensorMap tmap;
-        const cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)Ms};
-        const cuuint64_t strides[1] = {(cuuint64_t)K * 2};
+        const cuuint64_t dims[2] = {(cuuint64_t)k_len, (cuuint64_t)Ms};
+        const cuuint64_t strides[1] = {(cuuint64_t)x_row};
         const cuuint32_t box[2] = {(cuuint32_t)kGemmBK, (cuuint32_t)bn};
         const cuuint32_t estr[2] = {1, 1};
-        void* xs = static_cast<uint8_t*>(x_f16) + (size_t)m0 * (size_t)K * 2;
+        void* xs = static_cast<uint8_t*>(x_f16) + (size_t)m0 * x_row;
         if (encode(&tmap, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, xs, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
@@ -889,10 +982,11 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
         prm.status = static_cast<int32_t*>(workspace);
         prm.host_status = host_status_device_ptr(s);
         prm.clear_status = (n0 == 0 && m0 == 0) ? 1 : 0;
-        prm.M = (int)Ms; prm.N = (int)Ns; prm.K = (int)Kp; prm.k_len = (int)K;
+        prm.M = (int)Ms; prm.N = (int)Ns; prm.K = (int)Kp; prm.k_len = (int)k_len;
         prm.y_stride = (int)N;
         prm.y_dtype = y_dtype; prm.bias_dtype = x_dtype;
         prm.up = up ? up + m0 : nullptr;
+        prm.row_up = row_up ? row_up + n0 : nullptr;
         prm.rows = rows; prm.bn = bn;
         // instruction descriptor: fp32 accumulate (bits 4-5 = 1), A and B both fp16 (format 0), both K-major,
         // N >> 3 at bits 17-22, M >> 4 at bits 24-28
@@ -979,13 +1073,8 @@ int32_t gemm_dx_fmt_impl(int fmt, const void* gy, int gy_dtype, int64_t M, const
     OJX_RETURN_IF(ensure_dynamic_smem(kernel, kGemmSmemBytes, configured[slot]) != OJX_OK, OJX_ERR_LAUNCH);
     if (convert) {
         // per-token power-of-two factors exactly as in the forward launch; rows here are N long (any multiple of 8)
-        if (N <= 4096)
-            normalize_rows_bf16_to_f16_kernel<32, 16><<<(unsigned)((M + 7) / 8), 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N);
-        else
-            normalize_rows_bf16_to_f16_kernel<256, 8><<<(unsigned)M, 256, 0, s>>>(
-                static_cast<const __nv_bfloat16*>(gy), static_cast<__half*>(gy_f16), up, M, N);
-        if (cudaGetLastError() != cudaSuccess) return OJX_ERR_LAUNCH;
+        const int32_t st = normalize_rows<__nv_bfloat16, false>(gy, gy_f16, up, M, N, s);
+        OJX_RETURN_IF(st != OJX_OK, st);
     }
     CUtensorMap tmap;
     const cuuint64_t dims[2] = {(cuuint64_t)N, (cuuint64_t)M};
@@ -1008,6 +1097,7 @@ int32_t gemm_dx_fmt_impl(int fmt, const void* gy, int gy_dtype, int64_t M, const
     prm.y_stride = (int)K;
     prm.y_dtype = dx_dtype; prm.bias_dtype = gy_dtype;
     prm.up = up;
+    prm.row_up = nullptr;
     prm.rows = rows; prm.bn = bn;
     // as the forward descriptor, plus bit 15: the A operand is MN-major
     prm.idesc = (1u << 4) | (1u << 15) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(kGemmHalf >> 4) << 24);

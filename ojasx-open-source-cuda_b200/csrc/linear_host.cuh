@@ -11,6 +11,7 @@ constexpr int kForceDecode = 1, kForceGemm = 2;        // flags of ojx_e8t_linea
 
 // Batches of tokens run the tcgen05 kernel, up to sixteen rows the decode kernels: 28672 x 8192 at sixteen rows, 78 us against
 // 106 us and more (whose smallest tile takes 35 us at K = 4096 whatever the token count).
+// (2.0-bit weights are rounded to fp16 there, except where K is no multiple of 256: gemm_split.)
 inline bool linear_uses_gemm(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, bool aligned, int flags) {
     (void)N;
     if (flags & kForceDecode) return false;
@@ -24,7 +25,7 @@ inline int linear_group(int fmt, int group) { return fmt == 0 ? effective_group(
 size_t linear_workspace_bytes_impl(int fmt, int x_dtype, int64_t M, int64_t N, int64_t K, int group, int flags) {
     group = linear_group(fmt, group);
     if (linear_uses_gemm(fmt, x_dtype, M, N, K, group, true, flags))
-        return (x_dtype == OJX_BF16 || K % 256 != 0) ? gemm_workspace_bytes_impl(M, N, K) : 256;
+        return (x_dtype == OJX_BF16 || K % 256 != 0) ? gemm_fmt_workspace_bytes(fmt, M, N, K) : 256;
     return 0;
 }
 

@@ -55,12 +55,11 @@ def test_batches_of_tokens_with_k_a_multiple_of_32(P, bits, group, m, n, k):
     """K that is no multiple of 256: rows start at any even address and the last 256-wide chunk is cut short."""
     packed, scales, wd = _problem(P, bits, n, k, group)
     fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
-    w16 = wd.half().float() if bits == 2.0 else wd           # the prefill kernel rounds 2.0-bit weights to fp16 once
     for dt in (torch.bfloat16, torch.float16):
         x = P.ops.generate(m * k, 8, 1.0, dt, torch.device(DEV)).view(m, k)
         y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
-        bound = x.float().abs() @ w16.abs().t()
-        assert float(((y - x.float() @ w16.t()).abs() / (bound + 1e-20)).max()) <= 2e-5
+        bound = x.float().abs() @ wd.abs().t()                # fp32 weights: of every format exact here
+        assert float(((y - x.float() @ wd.t()).abs() / (bound + 1e-20)).max()) <= 2e-5
     P.ops.gemm_status(torch.device(DEV))
 
 
@@ -272,3 +271,31 @@ def test_decode_kernels_with_scales_near_the_top_of_fp16(P, bits, group, n, k):
             low = 0.5 * ((x.double() @ a.to(dt).double()) @ b.to(dt).double())
             bound += 0.5 * ((x.double().abs() @ a.to(dt).double().abs()) @ b.to(dt).double().abs())
             assert float(((y.double() - ref - low).abs() / bound.clamp_min(1e-30)).max()) <= 5e-6, (m, dt)
+
+
+@pytest.mark.parametrize("bits", [2.0])
+@pytest.mark.parametrize("group,m,n,k", [(32, 40, 136, 2912), (8, 130, 40, 544), (16, 17, 33, 96), (32, 300, 300, 4128)])
+def test_batches_of_tokens_over_scales_of_every_size(P, bits, group, m, n, k):
+    """K that is no multiple of 256: scales whose 1.5- or 2-fold fp16 does not have, and ones whose halves it does not, in rows of
+    their own and beside ordinary ones; Inf and NaN stay in their token and give the dense product's pattern."""
+    packed, scales, _ = _problem(P, bits, n, k, group)
+    fn = {1.0: P.ops.linear_1bit, 2.0: P.ops.linear_2bit}[bits]
+    scales = scales.clone()
+    rows = scales.view(n, -1)
+    rows[1::8, ::2] = 65504.0
+    rows[2::8] = 44000.0
+    rows[3::8] *= 2.0 ** -14
+    rows[4::8] = 2.0 ** -24 * torch.randint(1, 4, rows[4::8].shape, device=DEV)
+    rows[5::8] = 0.0
+    wd = _packer(P, bits).unpack(packed, scales, (n, k), torch.float32).double()
+    for dt in (torch.bfloat16, torch.float16):
+        x = P.ops.generate(m * k, 8, 1.0, dt, torch.device(DEV)).view(m, k).clone()
+        y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
+        ref, bound = x.double() @ wd.t(), x.double().abs() @ wd.abs().t()
+        assert float(((y.double() - ref).abs() / bound.clamp_min(1e-35)).max()) <= 2e-5, dt
+        x[3, k - 1], x[9, 5], x[10, 0] = float("inf"), float("nan"), -float("inf")
+        y2, ref = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32), x.float() @ wd.float().t()
+        assert torch.equal(torch.isnan(y2), torch.isnan(ref)) and torch.equal(torch.isinf(y2), torch.isinf(ref))
+        keep = [i for i in range(m) if i not in (3, 9, 10)]
+        assert torch.equal(y2[keep], y[keep])
+    P.ops.gemm_status(torch.device(DEV))
