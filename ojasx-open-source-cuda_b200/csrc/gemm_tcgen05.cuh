@@ -948,7 +948,7 @@ int32_t gemm_fmt_impl(int fmt, const void* x, int x_dtype, int64_t M, const uint
             pad_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(static_cast<const uint8_t*>(src), dst, N, (int)sb, (int)db);
         };
         pad(packed, wp, code_bytes(K), code_bytes(Kp));
-        if (fmt != 2) {
+        if (fmt == 0) {
             pad(scales, wsc, K / group * 2, Kp / group * 2);
         } else {
             row_up = reinterpret_cast<float*>(wsc + N * (Kp / group * 2));

@@ -273,7 +273,7 @@ def test_decode_kernels_with_scales_near_the_top_of_fp16(P, bits, group, n, k):
             assert float(((y.double() - ref - low).abs() / bound.clamp_min(1e-30)).max()) <= 5e-6, (m, dt)
 
 
-@pytest.mark.parametrize("bits", [2.0])
+@pytest.mark.parametrize("bits", [2.0, 1.0])
 @pytest.mark.parametrize("group,m,n,k", [(32, 40, 136, 2912), (8, 130, 40, 544), (16, 17, 33, 96), (32, 300, 300, 4128)])
 def test_batches_of_tokens_over_scales_of_every_size(P, bits, group, m, n, k):
     """K that is no multiple of 256: scales whose 1.5- or 2-fold fp16 does not have, and ones whose halves it does not, in rows of
