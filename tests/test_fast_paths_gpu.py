@@ -55,11 +55,14 @@ def test_batches_of_tokens_with_k_a_multiple_of_32(P, bits, group, m, n, k):
     """K that is no multiple of 256: rows start at any even address and the last 256-wide chunk is cut short."""
     packed, scales, wd = _problem(P, bits, n, k, group)
     fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    fmt, gemm = {1.0: 1, 1.5: 0, 2.0: 2}[bits], P._cabi.OJX_LINEAR_GEMM
     for dt in (torch.bfloat16, torch.float16):
         x = P.ops.generate(m * k, 8, 1.0, dt, torch.device(DEV)).view(m, k)
-        y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
-        bound = x.float().abs() @ wd.abs().t()                # fp32 weights: of every format exact here
-        assert float(((y - x.float() @ wd.t()).abs() / (bound + 1e-20)).max()) <= 2e-5
+        ref, bound = x.double() @ wd.double().t(), x.double().abs() @ wd.double().abs().t()     # unrounded weights: of every format exact here
+        for flags, limit in ((gemm, 2e-5), (0, 5e-6)):                   # fp32 outputs: the tcgen05 kernel, and the decode kernel that serves them
+            y = P.ops._linear(fmt, x, packed, scales, None, n, k, group, torch.float32, flags)
+            assert float(((y.double() - ref).abs() / (bound + 1e-20)).max()) <= limit
+        assert torch.equal(fn(x, packed, scales, None, n, k, group), P.ops._linear(fmt, x, packed, scales, None, n, k, group, None, gemm))
     P.ops.gemm_status(torch.device(DEV))
 
 
@@ -279,7 +282,7 @@ def test_batches_of_tokens_over_scales_of_every_size(P, bits, group, m, n, k):
     """K that is no multiple of 256: scales whose 1.5- or 2-fold fp16 does not have, and ones whose halves it does not, in rows of
     their own and beside ordinary ones; Inf and NaN stay in their token and give the dense product's pattern."""
     packed, scales, _ = _problem(P, bits, n, k, group)
-    fn = {1.0: P.ops.linear_1bit, 2.0: P.ops.linear_2bit}[bits]
+    call = lambda x: P.ops._linear(int(bits), x, packed, scales, None, n, k, group, torch.float32, P._cabi.OJX_LINEAR_GEMM)
     scales = scales.clone()
     rows = scales.view(n, -1)
     rows[1::8, ::2] = 65504.0
@@ -290,11 +293,11 @@ def test_batches_of_tokens_over_scales_of_every_size(P, bits, group, m, n, k):
     wd = _packer(P, bits).unpack(packed, scales, (n, k), torch.float32).double()
     for dt in (torch.bfloat16, torch.float16):
         x = P.ops.generate(m * k, 8, 1.0, dt, torch.device(DEV)).view(m, k).clone()
-        y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
+        y = call(x)
         ref, bound = x.double() @ wd.t(), x.double().abs() @ wd.abs().t()
         assert float(((y.double() - ref).abs() / bound.clamp_min(1e-35)).max()) <= 2e-5, dt
         x[3, k - 1], x[9, 5], x[10, 0] = float("inf"), float("nan"), -float("inf")
-        y2, ref = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32), x.float() @ wd.float().t()
+        y2, ref = call(x), x.float() @ wd.float().t()
         assert torch.equal(torch.isnan(y2), torch.isnan(ref)) and torch.equal(torch.isinf(y2), torch.isinf(ref))
         keep = [i for i in range(m) if i not in (3, 9, 10)]
         assert torch.equal(y2[keep], y[keep])
