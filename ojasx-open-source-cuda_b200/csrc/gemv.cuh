@@ -44,6 +44,7 @@ __device__ __forceinline__ void store_any(void* y, int y_dtype, int64_t idx, flo
 struct PeerMap {
     int64_t delta[8];
     int world;
+    int wide;                      // every delta is a multiple of 16 bytes
     int mode;                      // OJX_GEMV_SIGNAL_PEERS | OJX_GEMV_WAIT_PEERS, only with a sync block
     ojx_e8t_peer_sync* sync;       // this rank's block inside the window (peers' blocks at + delta[r]), or null
     // not about peers, but travelling in the same kernel argument:
@@ -51,7 +52,7 @@ struct PeerMap {
     uint32_t wait_limit;           // polls before a wait on a copy gives up
     int lose_copy;                 // tests: never report the first item's copies complete
 };
-inline PeerMap peer_map_self() { PeerMap m = {}; m.world = 1; m.wait_limit = kSpinLimit; return m; }
+inline PeerMap peer_map_self() { PeerMap m = {}; m.world = 1; m.wide = 1; m.wait_limit = kSpinLimit; return m; }
 // The copies for the other ranks (delta != 0), kept out of line: rare, and the callers run at the register cap.
 __device__ __noinline__ void store_peers(const PeerMap& pm, void* y, int y_dtype, int64_t idx, float v) {
     for (int r = 0; r < pm.world; ++r)

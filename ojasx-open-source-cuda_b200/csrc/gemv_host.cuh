@@ -63,7 +63,10 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     PeerMap peers = peer_map_self();
     if (peer_delta != nullptr) {
         peers.world = world;
-        for (int r = 0; r < world; ++r) peers.delta[r] = peer_delta[r];
+        for (int r = 0; r < world; ++r) {
+            peers.delta[r] = peer_delta[r];
+            if (peer_delta[r] % 16 != 0) peers.wide = 0;
+        }
     }
     OJX_RETURN_IF(!problems, OJX_ERR_NULL);
     OJX_RETURN_IF(count <= 0 || total_tiles <= 0 || M < 1 || M > 16, OJX_ERR_SHAPE);

@@ -291,6 +291,28 @@ __device__ __forceinline__ float mma_ld_cluster(uint32_t addr, int rank) {
     return v;
 }
 
+// The other ranks' copies of an output per lane, by all lanes of a warp: 8 << qs neighbouring lanes hold eight consecutive weight rows,
+// each row's value in the first of its 1 << qs lanes (`out`: that lane has one).  Eight 16-bit outputs leave as one 16-byte vector per
+// rank, a lane of the group each, instead of eight 2-byte stores (eight windows, here on one GPU, 4096 x 4096: 7.4 -> 6.6 us at one row,
+// 15.5 -> 13.6 at sixteen; two windows 6.4 and 13.6 either way).
+__device__ __noinline__ void mma_store_peers(const PeerMap& pm, void* y, int y_dtype, int64_t ld, int col, int n, int qs, bool out, float v) {
+    const int lane = threadIdx.x & 31, base = lane & -(8 << qs);
+    const uint32_t h = y_dtype == OJX_BF16 ? __bfloat16_as_ushort(__float2bfloat16_rn(v)) : __half_as_ushort(__float2half_rn(v));
+    const uint32_t rows = qs == 0 ? 0xFFu : (qs == 1 ? 0x5555u : 0x11111111u);
+    const bool whole = ((__ballot_sync(0xFFFFFFFFu, out) >> base) & rows) == rows;
+    uint32_t w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w[i] = __shfl_sync(0xFFFFFFFFu, h, base + ((2 * i) << qs)) | (__shfl_sync(0xFFFFFFFFu, h, base + ((2 * i + 1) << qs)) << 16);
+    if (whole && pm.wide && y_dtype != OJX_F32 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+        const int r = lane - base;
+        if (r < pm.world && pm.delta[r] != 0)
+            *reinterpret_cast<uint4*>(static_cast<uint8_t*>(y) + pm.delta[r] + (col * ld + (n & ~7)) * 2) = make_uint4(w[0], w[1], w[2], w[3]);
+    } else if (out) {
+        store_peers(pm, y, y_dtype, col * ld + n, v);
+    }
+}
+
 // Decode table in shared memory, entry stride 128 bytes: sixteen 8-byte copies (1.0 bit: eight of 16 bytes, int8: 32 of 4
 // bytes), so that every lane of an access reads banks of its own.  Four threads per entry, two 16-byte stores each.
 template <int FMT, bool kI8>
@@ -680,12 +702,15 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 }
             };
 
-            auto finish = [&](float sum, int col, int n) {                          // bias, store
+            auto finish = [&](float sum, int col, int n) {                          // bias, store; returns what was stored
                 if (FMT != 0 && (__float_as_uint(sum) & 0x7F800000u) == 0x7F800000u) sum = mma_dense<FMT>(P, G, x_dtype, col, n, sum);
                 if (P.bias != nullptr) sum += load_any(P.bias, x_dtype, n);
-                const int64_t at = (int64_t)col * (P.ldy > 0 ? P.ldy : N) + n;
-                store_any(P.y, y_dtype, at, sum);
-                if (peers.world > 1) store_peers(peers, P.y, y_dtype, at, sum);
+                store_any(P.y, y_dtype, (int64_t)col * (P.ldy > 0 ? P.ldy : N) + n, sum);
+                return sum;
+            };
+            // launches from a table only have peers; every lane of the warp
+            auto to_peers = [&](float sum, int col, int n, int q, bool out) {
+                if (kGroup && peers.world > 1) mma_store_peers(peers, P.y, y_dtype, P.ldy > 0 ? P.ldy : N, col, n, q, out, sum);
             };
             // ---- adds up an item's partial sums (pair, chunk) in buffer b ----
             auto reduce = [&](int pair, int chunk, int b) {
@@ -706,13 +731,15 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                         sum = fmaf(__ldcg(P.lora_t + q_col * rank + r), mma_load16(P.lora_b, xf16, (int64_t)r * N + n), sum);
                 }
                 for (int o = 1; o < (1 << qs); o <<= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-                if (q_sub != 0 || q_col >= M || n >= N || n >= (b0 + nt) * 16) return;
+                const bool out = q_sub == 0 && q_col < M && n < N && n < (b0 + nt) * 16;
                 if (chunks > 1) {
                     float* a = acc_sums + (pair * M + q_col) * R + q_row;
-                    if (chunk > cr) sum += *a;
-                    if (chunk + cs < chunks || cs > 1) { *a = sum; return; }
+                    if (out && chunk > cr) sum += *a;
+                    if (out && (chunk + cs < chunks || cs > 1)) *a = sum;
+                    if (chunk + cs < chunks || cs > 1) return;
                 }
-                finish(sum, q_col, n);
+                if (out) sum = finish(sum, q_col, n);
+                to_peers(sum, q_col, n, qs, out);
             };
 
             int pair = 0, chunk = cr, act = 0, last_pair = -1, last_chunk = 0;
@@ -855,12 +882,15 @@ gemv_mma_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, const __grid_con
                 mma_cluster_sync();
                 const int ranks = min(cs, chunks);
                 if (!dead)
-                    for (int i = tid + cr * kMmaThreads; i < np * M * R; i += cs * kMmaThreads) {
+                    for (int i = tid + cr * kMmaThreads; i - lane < np * M * R; i += cs * kMmaThreads) {
                         const int row = i % R, pm = i / R, pr = pm / M, col = pm - pr * M, n = (b0 + pr * T) * 16 + row;
-                        if (n >= N || n >= (b0 + nt) * 16) continue;
+                        const bool out = i < np * M * R && n < N && n < (b0 + nt) * 16;
                         float sum = 0.f;
-                        for (int r = 0; r < ranks; ++r) sum += mma_ld_cluster(base + plan.off_acc + i * 4, r);
-                        finish(sum, col, n);
+                        if (out) {
+                            for (int r = 0; r < ranks; ++r) sum += mma_ld_cluster(base + plan.off_acc + i * 4, r);
+                            sum = finish(sum, col, n);
+                        }
+                        to_peers(sum, col, n, 0, out);
                     }
                 mma_cluster_sync();         // nobody leaves, or writes these sums again, before all have read them
             }

@@ -235,3 +235,26 @@ def test_reader_behind_an_independent_launch_sees_what_came_before_it(P, count):
         z = P.ops.linear(y, pk2, sc2, None, 64, 14336, 32)
         assert torch.equal(z, want[i % 2]), i
         del y
+
+
+@pytest.mark.parametrize("m", [1, 2, 5, 16])
+@pytest.mark.parametrize("n,k,ld,shift,dt", [(256, 1024, 256, 0, "bfloat16"), (100, 512, 104, 0, "float16"), (33, 14336, 40, 0, "bfloat16"),
+                                             (520, 8192, 1040, 0, "bfloat16"), (64, 512, 67, 0, "bfloat16"), (96, 4352, 96, 1, "float16"),
+                                             (72, 256, 72, 0, "float32")])
+def test_outputs_of_one_matrix_reach_every_window(P, m, n, k, ld, shift, dt):
+    """Stores into the other ranks' windows (here: buffers of the same GPU) of a launch over one matrix: whole and cut groups of eight
+    rows, K of several chunks and split over a cluster, rows of any pitch, windows at odd distances, fp32; nothing beside them."""
+    dev, dtype = torch.device(DEV), getattr(torch, dt)
+    pk, sc, x = _problem(P, n, k, m, 110)
+    step = -(-(m * ld + 8) // 8) * 8
+    for world in (2, 8):
+        flat = torch.full((world * step + 8,), 7.0, dtype=dtype, device=dev)
+        starts = [r * step + (shift if r else 0) for r in range(world)]
+        views = [torch.as_strided(flat, (m, n), (ld, 1), s) for s in starts]
+        P.ops.GroupedGemv([(x, pk, sc, None, views[0])], [(n, k)], peer_delta=[s * flat.element_size() for s in starts])()
+        alone = torch.empty((m, n), dtype=dtype, device=dev)
+        P.ops.GroupedGemv([(x, pk, sc, None, alone)], [(n, k)])()
+        for v in views:
+            assert torch.equal(v, alone)
+            v.fill_(7.0)
+        assert bool((flat == 7.0).all())
