@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(256, 3) gemv_reduce_kernel(const ojx_e8t_gemv_
         const int kc = gemv_kchunks(P.K);
         const int64_t total = (int64_t)M * P.N;
         const int64_t ld = P.ldy > 0 ? P.ldy : P.N;
-        const bool vec = y_dtype != OJX_F32 && (P.N & 7) == 0 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(P.y) & 15) == 0 &&
+        const bool vec = y_dtype != OJX_F32 && peers.wide && (P.N & 7) == 0 && (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(P.y) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(P.partial) & 31) == 0;
         if (vec) {
             const int64_t per_col = P.N / 8;

@@ -509,7 +509,7 @@ gemv_a16_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev, const __grid
                 const int rN = P.N;
                 ld = P.ldy > 0 ? P.ldy : rN;
                 ybase = P.y;
-                vec = P.partial == nullptr && y_dtype != OJX_F32 && tile * kA16Rows + kA16Rows <= rN && (ld & 7) == 0 &&
+                vec = P.partial == nullptr && y_dtype != OJX_F32 && peers.wide && tile * kA16Rows + kA16Rows <= rN && (ld & 7) == 0 &&
                       (reinterpret_cast<uintptr_t>(P.y) & 15) == 0;
                 if (row < rN && col < M) {                           // activation rows beyond M hold zeros: nothing to add up
                     const float* rb = red + (size_t)(n & 1) * Cfg::kRedFloats + tid;

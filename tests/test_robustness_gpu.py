@@ -258,3 +258,24 @@ def test_outputs_of_one_matrix_reach_every_window(P, m, n, k, ld, shift, dt):
             assert torch.equal(v, alone)
             v.fill_(7.0)
         assert bool((flat == 7.0).all())
+
+
+@pytest.mark.parametrize("m", [1, 4, 16])
+@pytest.mark.parametrize("n,k,shift", [(64, 512, 0), (64, 512, 1), (72, 14336, 0), (72, 14336, 1), (40, 4352, 3)])
+def test_outputs_of_several_matrices_reach_windows_at_any_distance(P, m, n, k, shift):
+    """The same of launches over several matrices and of their reduce launch: windows that are no multiple of 16 bytes apart take
+    stores of single outputs."""
+    dev = torch.device(DEV)
+    probs = [_problem(P, n, k, m, 120 + 10 * i) for i in range(2)]
+    step = m * n + 8
+    flat = torch.full((2 * 2 * step + 8,), 7.0, dtype=torch.bfloat16, device=dev)
+    ys = [torch.as_strided(flat, (m, n), (n, 1), i * step) for i in range(2)]
+    far = [torch.as_strided(flat, (m, n), (n, 1), 2 * step + shift + i * step) for i in range(2)]
+    P.ops.GroupedGemv([(x, pk, sc, None, y) for (pk, sc, x), y in zip(probs, ys)], [(n, k)] * 2, peer_delta=[0, (2 * step + shift) * 2])()
+    alone = [torch.empty((m, n), dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    P.ops.GroupedGemv([(x, pk, sc, None, y) for (pk, sc, x), y in zip(probs, alone)], [(n, k)] * 2)()
+    for got, y, want in zip(far, ys, alone):
+        assert torch.equal(got, want) and torch.equal(y, want)
+        got.fill_(7.0)
+        y.fill_(7.0)
+    assert bool((flat == 7.0).all())
