@@ -54,6 +54,12 @@ at::Tensor empty(at::IntArrayRef sizes, at::ScalarType t, c10::Device dev) {
 void* stream_of(c10::Device dev) { return c10::cuda::getCurrentCUDAStream(dev.index()).stream(); }
 void* data(const at::Tensor& t) { return t.data_ptr(); }
 
+// Other Python threads run while this one allocates and launches: a launch waits as long as the launch queue is full.
+struct NoGil {
+    PyThreadState* const state = PyEval_SaveThread();
+    ~NoGil() { PyEval_RestoreThread(state); }
+};
+
 struct Args {
     PyObject* const* v;
     Py_ssize_t n;
@@ -91,29 +97,33 @@ PyObject* py_linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if (args[4] != Py_None &&
         (!plain(bias) || bias->device() != dev || bias->scalar_type() != x->scalar_type() || bias->numel() != n))
         Py_RETURN_NONE;
+    const bool rotate = hadamard && k % 32 == 0;         // rotated weights: the transform of x first
+    if (rotate && (reinterpret_cast<uintptr_t>(data(*x)) & 15) != 0) Py_RETURN_NONE;
     if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
-    const c10::cuda::CUDAGuard guard(dev);
-    void* s = stream_of(dev);
     const int64_t m = x->numel() / k;
     c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = n;
     const int y_code = yd < 0 ? xd : yd;
-    at::Tensor y = empty(sizes, scalar_type(y_code), dev);
-    at::Tensor rot;
-    const void* xp = data(*x);
-    if (hadamard && k % 32 == 0) {                      // rotated weights: the transform of x first
-        if ((reinterpret_cast<uintptr_t>(xp) & 15) != 0) Py_RETURN_NONE;
-        rot = empty({x->numel()}, x->scalar_type(), dev);
-        const int32_t st = ojx_e8t_fwht32(xp, xd, x->numel(), data(rot), s);
-        if (st != OJX_OK) return PyLong_FromLong(st);
-        xp = data(rot);
+    at::Tensor y, rot, ws;
+    int32_t st = OJX_OK;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        void* s = stream_of(dev);
+        y = empty(sizes, scalar_type(y_code), dev);
+        const void* xp = data(*x);
+        if (rotate) {
+            rot = empty({x->numel()}, x->scalar_type(), dev);
+            st = ojx_e8t_fwht32(xp, xd, x->numel(), data(rot), s);
+            xp = data(rot);
+        }
+        const size_t need = ojx_e8t_linear_workspace_bytes(fmt, xd, m, n, k, group, flags);
+        if (need > 0) ws = empty({(int64_t)need}, at::kByte, dev);
+        if (st == OJX_OK)
+            st = ojx_e8t_linear(fmt, xp, xd, m, static_cast<const uint8_t*>(data(*pk)), static_cast<const uint16_t*>(data(*sc)),
+                                bias ? data(*bias) : nullptr, n, k, group, data(y), y_code, need ? data(ws) : nullptr, need, flags, s);
     }
-    const size_t need = ojx_e8t_linear_workspace_bytes(fmt, xd, m, n, k, group, flags);
-    at::Tensor ws;
-    if (need > 0) ws = empty({(int64_t)need}, at::kByte, dev);
-    return status_or(ojx_e8t_linear(fmt, xp, xd, m, static_cast<const uint8_t*>(data(*pk)), static_cast<const uint16_t*>(data(*sc)),
-                                    bias ? data(*bias) : nullptr, n, k, group, data(y), y_code, need ? data(ws) : nullptr, need, flags, s),
-                     std::move(y));
+    return status_or(st, std::move(y));
     END_HANDLE_TH_ERRORS
 }
 
@@ -137,7 +147,6 @@ PyObject* py_linear_adapter(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
         la->dim() != 2 || lb->dim() != 2 || la->size(0) != k || lb->size(1) != n || la->size(1) != lb->size(0))
         Py_RETURN_NONE;
     if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
-    const c10::cuda::CUDAGuard guard(dev);
     const int64_t m = x->numel() / k;
     const int rank = (int)la->size(1);
     const size_t need = ojx_e8t_linear_adapter_workspace_bytes(m, k, rank, hadamard);
@@ -145,10 +154,17 @@ PyObject* py_linear_adapter(PyObject*, PyObject* const* args, Py_ssize_t nargs) 
     c10::SmallVector<int64_t, 6> sizes(x->sizes().begin(), x->sizes().end());
     sizes.back() = n;
     const int y_code = yd < 0 ? xd : yd;
-    at::Tensor y = empty(sizes, scalar_type(y_code), dev), ws = empty({(int64_t)need}, at::kByte, dev);
-    const int32_t st = ojx_e8t_linear_adapter(fmt, data(*x), xd, m, static_cast<const uint8_t*>(data(*pk)), static_cast<const uint16_t*>(data(*sc)),
-                                              bias ? data(*bias) : nullptr, n, k, group, data(*la), data(*lb), rank, (float)scaling, hadamard,
-                                              data(y), y_code, data(ws), need, stream_of(dev));
+    at::Tensor y, ws;
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        y = empty(sizes, scalar_type(y_code), dev);
+        ws = empty({(int64_t)need}, at::kByte, dev);
+        st = ojx_e8t_linear_adapter(fmt, data(*x), xd, m, static_cast<const uint8_t*>(data(*pk)), static_cast<const uint16_t*>(data(*sc)),
+                                    bias ? data(*bias) : nullptr, n, k, group, data(*la), data(*lb), rank, (float)scaling, hadamard,
+                                    data(y), y_code, data(ws), need, stream_of(dev));
+    }
     if (st == OJX_ERR_UNSUPPORTED) Py_RETURN_NONE;
     return status_or(st, std::move(y));
     END_HANDLE_TH_ERRORS
@@ -167,17 +183,22 @@ PyObject* py_linear_dx(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int gd = dtype_code(gy->scalar_type());
     if ((gd != OJX_BF16 && gd != OJX_F16) || !packed_pair(pk, sc, dev) || !holds(fmt, *pk, *sc, n, k, group)) Py_RETURN_NONE;
     if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
-    const c10::cuda::CUDAGuard guard(dev);
     const int64_t m = gy->size(0);
     const int code = od < 0 ? gd : od;
-    at::Tensor dx = empty({m, k}, scalar_type(code), dev);
-    const size_t need = ojx_e8t_gemm_dx_workspace_bytes(m, n, k);
-    at::Tensor ws = empty({(int64_t)need}, at::kByte, dev);
-    const uint8_t* p = static_cast<const uint8_t*>(data(*pk));
-    const uint16_t* q = static_cast<const uint16_t*>(data(*sc));
-    void* s = stream_of(dev);
-    const int32_t st = fmt == 0 ? ojx_e8t_gemm_dx(data(*gy), gd, m, p, q, n, k, group, data(dx), code, data(ws), need, s)
-                                : ojx_e8t_gemm_dx_lowbit(fmt, data(*gy), gd, m, p, q, n, k, group, data(dx), code, data(ws), need, s);
+    at::Tensor dx, ws;
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        dx = empty({m, k}, scalar_type(code), dev);
+        const size_t need = ojx_e8t_gemm_dx_workspace_bytes(m, n, k);
+        ws = empty({(int64_t)need}, at::kByte, dev);
+        const uint8_t* p = static_cast<const uint8_t*>(data(*pk));
+        const uint16_t* q = static_cast<const uint16_t*>(data(*sc));
+        void* s = stream_of(dev);
+        st = fmt == 0 ? ojx_e8t_gemm_dx(data(*gy), gd, m, p, q, n, k, group, data(dx), code, data(ws), need, s)
+                      : ojx_e8t_gemm_dx_lowbit(fmt, data(*gy), gd, m, p, q, n, k, group, data(dx), code, data(ws), need, s);
+    }
     return status_or(st, std::move(dx));
     END_HANDLE_TH_ERRORS
 }
@@ -195,15 +216,21 @@ PyObject* py_encode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int wd = dtype_code(w->scalar_type());
     if (wd < 0) Py_RETURN_NONE;
     const c10::Device dev = w->device();
-    const c10::cuda::CUDAGuard guard(dev);
-    at::Tensor pk = empty({bytes}, at::kByte, dev), sc = empty({count}, at::kHalf, dev);
-    uint8_t* p = static_cast<uint8_t*>(data(pk));
-    uint16_t* q = static_cast<uint16_t*>(data(sc));
-    void* s = stream_of(dev);
-    const int64_t rows = w->size(0), cols = w->size(1);
-    const int32_t st = fmt == 0 ? ojx_e8t_encode_ex(data(*w), wd, rows, cols, group, flags, p, q, s)
-                     : fmt == 2 ? ojx_e8t_encode_2bit(data(*w), wd, rows, cols, group, p, q, s)
-                                : ojx_e8t_encode_1bit(data(*w), wd, rows, cols, group, p, q, s);
+    at::Tensor pk, sc;
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        pk = empty({bytes}, at::kByte, dev);
+        sc = empty({count}, at::kHalf, dev);
+        uint8_t* p = static_cast<uint8_t*>(data(pk));
+        uint16_t* q = static_cast<uint16_t*>(data(sc));
+        void* s = stream_of(dev);
+        const int64_t rows = w->size(0), cols = w->size(1);
+        st = fmt == 0 ? ojx_e8t_encode_ex(data(*w), wd, rows, cols, group, flags, p, q, s)
+           : fmt == 2 ? ojx_e8t_encode_2bit(data(*w), wd, rows, cols, group, p, q, s)
+                      : ojx_e8t_encode_1bit(data(*w), wd, rows, cols, group, p, q, s);
+    }
     if (st != OJX_OK) return PyLong_FromLong(st);
     PyObject* tp = THPVariable_Wrap(std::move(pk));
     PyObject* ts = THPVariable_Wrap(std::move(sc));
@@ -224,14 +251,19 @@ PyObject* py_decode(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int group = (int)a.i(5), od = (int)a.i(6);
     if (!a.ok || !plain(pk) || !packed_pair(pk, sc, pk->device()) || rows <= 0 || cols <= 0) Py_RETURN_NONE;
     const c10::Device dev = pk->device();
-    const c10::cuda::CUDAGuard guard(dev);
-    at::Tensor w = empty({rows, cols}, scalar_type(od), dev);
-    const uint8_t* p = static_cast<const uint8_t*>(data(*pk));
-    const uint16_t* q = static_cast<const uint16_t*>(data(*sc));
-    void* s = stream_of(dev);
-    const int32_t st = fmt == 0 ? ojx_e8t_decode(p, q, rows, cols, group, od, data(w), s)
-                     : fmt == 2 ? ojx_e8t_decode_2bit(p, q, rows, cols, group, od, data(w), s)
-                                : ojx_e8t_decode_1bit(p, q, rows, cols, group, od, data(w), s);
+    at::Tensor w;
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        w = empty({rows, cols}, scalar_type(od), dev);
+        const uint8_t* p = static_cast<const uint8_t*>(data(*pk));
+        const uint16_t* q = static_cast<const uint16_t*>(data(*sc));
+        void* s = stream_of(dev);
+        st = fmt == 0 ? ojx_e8t_decode(p, q, rows, cols, group, od, data(w), s)
+           : fmt == 2 ? ojx_e8t_decode_2bit(p, q, rows, cols, group, od, data(w), s)
+                      : ojx_e8t_decode_1bit(p, q, rows, cols, group, od, data(w), s);
+    }
     return status_or(st, std::move(w));
     END_HANDLE_TH_ERRORS
 }
@@ -246,9 +278,15 @@ PyObject* py_fwht32(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     const int xd = dtype_code(x->scalar_type());
     if (xd < 0) Py_RETURN_NONE;
     const c10::Device dev = x->device();
-    const c10::cuda::CUDAGuard guard(dev);
-    at::Tensor y = empty(x->sizes(), x->scalar_type(), dev);
-    return status_or(ojx_e8t_fwht32(data(*x), xd, x->numel(), data(y), stream_of(dev)), std::move(y));
+    at::Tensor y;
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(dev);
+        y = empty(x->sizes(), x->scalar_type(), dev);
+        st = ojx_e8t_fwht32(data(*x), xd, x->numel(), data(y), stream_of(dev));
+    }
+    return status_or(st, std::move(y));
     END_HANDLE_TH_ERRORS
 }
 
@@ -257,16 +295,20 @@ PyObject* py_grouped(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     HANDLE_TH_ERRORS
     OJX_ARGS(12);
     const c10::DeviceIndex index = (c10::DeviceIndex)a.i(0);
-    const c10::cuda::CUDAGuard guard(index);
     if (ojx_e8t_poll_status() != OJX_OK) return PyLong_FromLong(1);
     const long long table = a.i(1), peers = a.i(8), sync = a.i(10);
     const int count = (int)a.i(2), tiles = (int)a.i(3), m = (int)a.i(4), xd = (int)a.i(5), yd = (int)a.i(6), reduce = (int)a.i(7);
     const int world = (int)a.i(9), flags = (int)a.i(11);
     if (!a.ok) { PyErr_SetString(PyExc_TypeError, "grouped() takes integers"); return nullptr; }
-    return PyLong_FromLong(ojx_e8t_gemv_grouped_ex(reinterpret_cast<const ojx_e8t_gemv_problem*>(table), count, tiles, m, xd, yd, reduce,
-                                                   reinterpret_cast<const int64_t*>(peers), world,
-                                                   reinterpret_cast<ojx_e8t_peer_sync*>(sync), flags,
-                                                   c10::cuda::getCurrentCUDAStream(index).stream()));
+    int32_t st;
+    {
+        const NoGil others;
+        const c10::cuda::CUDAGuard guard(index);
+        st = ojx_e8t_gemv_grouped_ex(reinterpret_cast<const ojx_e8t_gemv_problem*>(table), count, tiles, m, xd, yd, reduce,
+                                     reinterpret_cast<const int64_t*>(peers), world, reinterpret_cast<ojx_e8t_peer_sync*>(sync), flags,
+                                     c10::cuda::getCurrentCUDAStream(index).stream());
+    }
+    return PyLong_FromLong(st);
     END_HANDLE_TH_ERRORS
 }
 

@@ -3,6 +3,7 @@ faulting it: every wait in the kernels is bounded, so the tests make a wait run 
 a copy whose completion is never reported) and check that the kernel returns, that the failure is reported
 through every channel, and that the next normal call is correct."""
 
+import threading
 import time
 
 import numpy as np
@@ -279,3 +280,25 @@ def test_outputs_of_several_matrices_reach_windows_at_any_distance(P, m, n, k, s
         got.fill_(7.0)
         y.fill_(7.0)
     assert bool((flat == 7.0).all())
+
+
+def test_a_full_launch_queue_does_not_stop_other_threads(P):
+    """Launches wait while the GPU's queue is full (here behind a kernel of about half a second); other Python threads go on."""
+    dev = torch.device(DEV)
+    pk, sc, x = _problem(P, 256, 512, 1, 130)
+    y = torch.zeros((1, 256), dtype=torch.bfloat16, device=dev)
+    grp = P.ops.GroupedGemv([(x, pk, sc, None, y)], [(256, 512)])
+    for launch in (grp, lambda: P.ops.linear(x, pk, sc, None, 256, 512, 32), lambda: P.ops.decode(pk, sc, (256, 512))):
+        launch()
+        torch.cuda.synchronize()
+        torch.cuda._sleep(1_000_000_000)
+        worker = threading.Thread(target=lambda: [launch() for _ in range(3000)])
+        longest, last = 0.0, time.perf_counter()
+        worker.start()
+        while worker.is_alive():
+            time.sleep(0.002)
+            now = time.perf_counter()
+            longest, last = max(longest, now - last), now
+        worker.join()
+        torch.cuda.synchronize()
+        assert longest < 0.15, longest
