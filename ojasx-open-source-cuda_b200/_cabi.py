@@ -13,6 +13,7 @@ import importlib.util
 import os
 import shutil
 import subprocess
+import sys
 import threading
 from typing import Optional
 
@@ -20,7 +21,6 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB_DIR = os.path.join(HERE, "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libojx_e8t.so")
-GLUE_PATH = os.path.join(LIB_DIR, "_ojx_torch.so")       # CPython extension: the hot entry points on torch tensors
 
 OJX_F32, OJX_F16, OJX_BF16 = 0, 1, 2
 OJX_GEMV_STATIC_WEIGHTS, OJX_GEMV_SIGNAL_PEERS, OJX_GEMV_WAIT_PEERS, OJX_GEMV_TEST_LOSE_COPY = 1, 2, 4, 8
@@ -60,8 +60,16 @@ def _stale(path: str, srcs) -> bool:
     return not os.path.exists(path) or any(os.path.getmtime(f) > os.path.getmtime(path) for f in srcs)
 
 
+def glue_path() -> str:
+    """The CPython extension with the hot entry points on torch tensors.  It is bound to the torch and the interpreter it was built
+    for, so both are part of its name: under another one there is no such file, instead of a module of the wrong ABI."""
+    import torch
+    return os.path.join(LIB_DIR, f"_ojx_torch.torch-{torch.__version__}.{sys.implementation.cache_tag}.so")
+
+
 def needs_build() -> bool:
-    return _stale(LIB_PATH, sources())
+    header = os.path.join(os.path.dirname(HERE), "include", "ojx_e8t.h")
+    return _stale(LIB_PATH, sources()) or _stale(glue_path(), [os.path.join(CSRC, "torch_glue.cpp"), header])
 
 
 def _compile(cmd, out: str) -> str:
@@ -74,7 +82,7 @@ def _compile(cmd, out: str) -> str:
 
 
 def _build_glue() -> None:
-    """``csrc/torch_glue.cpp`` -> ``lib/_ojx_torch.so`` against the installed torch's headers and libraries."""
+    """``csrc/torch_glue.cpp`` -> :func:`glue_path` against the installed torch's headers and libraries."""
     import sysconfig
 
     import torch
@@ -85,13 +93,13 @@ def _build_glue() -> None:
     _compile(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden",
               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + [f"-I{d}" for d in includes] +
              [os.path.join(CSRC, "torch_glue.cpp"), f"-L{os.path.join(root, 'lib')}", f"-L{LIB_DIR}", "-l:libojx_e8t.so",
-              "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], GLUE_PATH)
+              "-ltorch_python", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"], glue_path())
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile ``csrc/ojx_e8t.cu`` for sm_100a into ``lib/libojx_e8t.so`` (nvcc cross-compiles without a GPU) and the
     torch module beside it.  Returns the library path."""
-    if force or needs_build():
+    if force or _stale(LIB_PATH, sources()):
         nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
         if not os.path.exists(nvcc):
             raise RuntimeError("nvcc not found: cannot build libojx_e8t.so")
@@ -100,7 +108,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             print(log)
     header = os.path.join(os.path.dirname(HERE), "include", "ojx_e8t.h")
-    if force or _stale(GLUE_PATH, [os.path.join(CSRC, "torch_glue.cpp"), header]):
+    if force or _stale(glue_path(), [os.path.join(CSRC, "torch_glue.cpp"), header]):
         _build_glue()
     return LIB_PATH
 
@@ -230,9 +238,10 @@ def glue():
     if _glue is None:
         lib()                                            # the library it links against, with its own error message
         import torch                                     # noqa: F401  (its libraries have to be loaded first)
-        if not os.path.exists(GLUE_PATH):
-            raise RuntimeError(f"{GLUE_PATH} is missing. Build it with this module's build().")
-        loader = importlib.machinery.ExtensionFileLoader("_ojx_torch", GLUE_PATH)
+        path = glue_path()
+        if not os.path.exists(path):
+            raise RuntimeError(f"{path} is missing (no build for this torch). Build it with this module's build().")
+        loader = importlib.machinery.ExtensionFileLoader("_ojx_torch", path)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_ojx_torch", loader))
         loader.exec_module(module)
         _glue = module

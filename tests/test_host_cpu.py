@@ -304,3 +304,13 @@ def test_packed_buffers_have_to_hold_the_whole_weight(P, fmt, group, n, k, codes
             P.ops._check_packed(fmt, a, b, n, k, group)
     with pytest.raises(TypeError):
         P.ops._check_packed(fmt, pk, sc.float(), n, k, group)
+
+
+def test_torch_module_is_built_for_the_torch_that_loads_it(P, monkeypatch):
+    """Under another torch the module on disk is not taken: a build is due, and without one loading it raises."""
+    assert not P._cabi.needs_build() and os.path.exists(P._cabi.glue_path())
+    monkeypatch.setattr(torch, "__version__", "0.0.1+other")
+    monkeypatch.setattr(P._cabi, "_glue", None)
+    assert P._cabi.needs_build()
+    with pytest.raises(RuntimeError, match="no build for this torch"):
+        P._cabi.glue()
