@@ -12,7 +12,11 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/core/GradMode.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/ojx_e8t.h"
 
@@ -25,7 +29,7 @@ at::ScalarType scalar_type(long code) {
     return code == OJX_BF16 ? at::kBFloat16 : (code == OJX_F16 ? at::kHalf : at::kFloat);
 }
 
-const at::Tensor* as_tensor(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+const at::Tensor* as_tensor(PyObject* o) { return o != Py_None && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
 
 // A dense CUDA tensor that holds data (no fake or wrapper tensors).
 bool plain(const at::Tensor* t) {
@@ -79,6 +83,25 @@ struct Args {
 PyObject* status_or(int32_t st, at::Tensor&& y) {
     if (st != OJX_OK) return PyLong_FromLong(st);
     return THPVariable_Wrap(std::move(y));
+}
+
+// direct(x, parameters) -> bool: nothing records, transforms or differentiates operations on these tensors (gradients of either
+// mode, the tracer, a dispatch mode, a function transform), so a call may pass by the dispatcher.
+PyObject* py_direct(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+    HANDLE_TH_ERRORS
+    if (nargs != 2 || !PyDict_Check(args[1])) { PyErr_SetString(PyExc_TypeError, "direct() takes x and a dict of parameters"); return nullptr; }
+    bool ok = !torch::jit::tracer::isTracing() && !c10::impl::TorchDispatchModeTLS::any_modes_set() &&
+              !c10::impl::tls_local_dispatch_key_set().included_.has(c10::DispatchKey::FuncTorchDynamicLayerFrontMode);
+    const bool grad = c10::GradMode::is_enabled();
+    auto look = [&](PyObject* o) {
+        const at::Tensor* t = as_tensor(o);
+        if (t != nullptr && t->defined() && ((grad && t->requires_grad()) || t->_fw_grad(0).defined())) ok = false;
+    };
+    look(args[0]);
+    PyObject *name, *value;
+    for (Py_ssize_t at = 0; ok && PyDict_Next(args[1], &at, &name, &value);) look(value);
+    return PyBool_FromLong(ok);
+    END_HANDLE_TH_ERRORS
 }
 
 // linear(fmt, x, packed, scales, bias, n, k, group, y_dtype, flags, hadamard) -> y [..., n]
@@ -313,7 +336,7 @@ PyObject* py_grouped(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 }
 
 #define OJX_METHOD(name) {#name, (PyCFunction)(void (*)(void))py_##name, METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {OJX_METHOD(linear), OJX_METHOD(linear_adapter), OJX_METHOD(linear_dx), OJX_METHOD(encode), OJX_METHOD(decode), OJX_METHOD(fwht32),
+PyMethodDef methods[] = {OJX_METHOD(direct), OJX_METHOD(linear), OJX_METHOD(linear_adapter), OJX_METHOD(linear_dx), OJX_METHOD(encode), OJX_METHOD(decode), OJX_METHOD(fwht32),
                          OJX_METHOD(grouped), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_ojx_torch", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
 

@@ -30,7 +30,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import ops
+from . import _cabi, ops
 
 _SUPPORTED_BITRATES = (1.0, 1.5, 2.0)
 
@@ -379,9 +379,8 @@ class E8LatticeLinear(nn.Module):
         params = self._parameters
         bias, with_adapter = params["bias"], self.rank > 0 and params["lora_A"] is not None and params["lora_B"] is not None
         out = None
-        if not torch.compiler.is_compiling() and not (
-                torch.is_grad_enabled() and (x.requires_grad or any(p is not None and p.requires_grad for p in params.values()))):
-            # nothing to differentiate: one native call, no autograd node
+        if not torch.compiler.is_compiling() and _cabi.glue().direct(x, params):
+            # nothing to differentiate, record or transform: one native call, no autograd node
             if with_adapter:
                 out = self._forward_decode_with_adapter(x)
                 if out is not None:

@@ -424,3 +424,16 @@ def test_layer_with_adapter_takes_the_fused_epilogue_at_inference(P):
     with pytest.raises(ValueError):
         P.ops.linear_lora(torch.zeros(9, 1024, device=dev, dtype=torch.bfloat16), layer.packed_weight, layer.block_scales,
                           None, 72, 1024, 32, torch.zeros(9, 8, device=dev), torch.zeros(8, 72, device=dev))
+
+
+@pytest.mark.parametrize("rank,m", [(0, 3), (0, 40), (4, 3)])
+def test_traced_layer_computes_with_its_own_input(P, rank, m):
+    """torch.jit.trace of a layer without gradients records an operation, not the result for the traced input."""
+    dev = torch.device(DEV)
+    layer = P.E8LatticeLinear.from_linear(torch.nn.Linear(256, 64).to(dev).bfloat16(), rank=rank, group_size=32, bitrate=1.5).requires_grad_(False)
+    if rank:
+        layer.lora_B.normal_()
+    a, b = torch.randn(m, 256, device=dev).bfloat16(), torch.randn(m, 256, device=dev).bfloat16()
+    traced = torch.jit.trace(layer, a, check_trace=False)
+    want = layer(b)
+    assert float((traced(b).float() - want.float()).norm() / want.float().norm()) <= 1e-2

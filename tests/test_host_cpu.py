@@ -314,3 +314,38 @@ def test_torch_module_is_built_for_the_torch_that_loads_it(P, monkeypatch):
     assert P._cabi.needs_build()
     with pytest.raises(RuntimeError, match="no build for this torch"):
         P._cabi.glue()
+
+
+@pytest.mark.parametrize("rank", [0, 4])
+def test_layer_passes_by_the_dispatcher_only_when_nothing_looks(P, monkeypatch, rank):
+    """Tracing, forward-mode gradients (of x or of a parameter), function transforms and dispatch modes take the autograd node, as
+    before there was a native call: here it refuses CPU tensors, or the transform."""
+    from torch.autograd import forward_ad
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Mode(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            return func(*args, **(kwargs or {}))
+
+    layer, x = P.E8LatticeLinear(64, 8, bias=True, rank=rank).requires_grad_(False), torch.randn(3, 64)
+    taken = torch.zeros(3, 8)
+    monkeypatch.setattr(P.ops, "layer_forward", lambda *a, **k: taken)
+    monkeypatch.setattr(P.lattice.E8LatticeLinear, "_forward_decode_with_adapter", lambda self, x: taken)
+    assert layer(x) is taken
+    with torch.no_grad():
+        assert layer(x.clone().requires_grad_(True)) is taken
+    with pytest.raises(Exception):
+        torch.jit.trace(layer, x)
+    with pytest.raises(Exception):
+        torch.func.vmap(layer)(x)
+    with pytest.raises(Exception):
+        torch.func.jvp(layer, (x,), (x,))
+    with Mode(), pytest.raises(Exception):
+        layer(x)
+    with forward_ad.dual_level():
+        assert layer(x) is taken
+        with pytest.raises(Exception):
+            layer(forward_ad.make_dual(x, x))
+        with pytest.raises(Exception):
+            torch.func.functional_call(layer, {"bias": forward_ad.make_dual(layer.bias.detach(), torch.ones(8))}, (x,))
+    assert layer(x) is taken
