@@ -301,6 +301,7 @@ typedef struct {
 
 int32_t ojx_e8t_gemv_tiles(int64_t N, int64_t K);
 int32_t ojx_e8t_gemv_kchunks(int64_t K);
+int32_t ojx_e8t_gemv_split_flag(int64_t N, int64_t K);
 int32_t ojx_e8t_gemv_grouped(const ojx_e8t_gemv_problem* problems, int32_t count, int32_t total_tiles,
                              int64_t M, int32_t x_dtype, int32_t y_dtype, int32_t needs_reduce, void* stream);
 
@@ -365,8 +366,9 @@ typedef struct {
 #define OJX_GEMV_SIGNAL_PEERS   2
 #define OJX_GEMV_WAIT_PEERS     4
 #define OJX_GEMV_INDEPENDENT    16
-#define OJX_GEMV_SPLIT_K2       32  /* every K is above 4096 (SPLIT_K4: above 12288) and the launch has few rows: clusters of two */
-#define OJX_GEMV_SPLIT_K4       64  /* (four) CTAs share rows and split K; a hint, results do not depend on it beyond summation order */
+#define OJX_GEMV_SPLIT_K2       32  /* a launch over one matrix with few rows and long K: clusters of two (four) CTAs share rows and split */
+#define OJX_GEMV_SPLIT_K4       64  /* K; a hint, results do not depend on it beyond summation order.  ojx_e8t_gemv_split_flag(N, K) gives
+                                       the one that the single-problem entry points would use on the current device, or 0 */
 #define OJX_GEMV_TEST_LOSE_COPY 8   /* tests only: the first work item's copies are never reported complete, so the
                                        wait on them runs into its limit (set a small one) and the error path runs */
 int32_t ojx_e8t_gemv_grouped_ex(const ojx_e8t_gemv_problem* problems, int32_t count, int32_t total_tiles,

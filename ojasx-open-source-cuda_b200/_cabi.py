@@ -31,7 +31,7 @@ PEER_SYNC_BYTES = 48        # sizeof(ojx_e8t_peer_sync): epoch, arrived, status,
 
 EXPORTED_SYMBOLS = (
     "ojx_e8t_version", "ojx_e8t_status_string", "ojx_e8t_encode", "ojx_e8t_encode_ex", "ojx_e8t_fwht32", "ojx_e8t_encode_2bit", "ojx_e8t_decode_2bit", "ojx_e8t_linear_2bit", "ojx_e8t_encode_1bit", "ojx_e8t_decode_1bit", "ojx_e8t_linear_1bit", "ojx_e8t_linear_lowbit_lora", "ojx_e8t_project", "ojx_e8t_ste_quantize", "ojx_e8t_decode",
-    "ojx_e8t_gemv_workspace_bytes", "ojx_e8t_gemv", "ojx_e8t_gemv_lora", "ojx_e8t_gemv_tiles", "ojx_e8t_gemv_kchunks",
+    "ojx_e8t_gemv_workspace_bytes", "ojx_e8t_gemv", "ojx_e8t_gemv_lora", "ojx_e8t_gemv_tiles", "ojx_e8t_gemv_kchunks", "ojx_e8t_gemv_split_flag",
     "ojx_e8t_gemv_grouped", "ojx_e8t_gemv_grouped_peers", "ojx_e8t_gemv_grouped_ex", "ojx_e8t_peer_wait", "ojx_e8t_enable_peer_access", "ojx_e8t_gemm_workspace_bytes", "ojx_e8t_gemm", "ojx_e8t_gemm_lowbit", "ojx_e8t_gemm_status", "ojx_e8t_gemm_dx", "ojx_e8t_gemm_dx_lowbit", "ojx_e8t_gemm_dx_workspace_bytes",
     "ojx_e8t_generate", "ojx_e8t_last_cuda_error", "ojx_e8t_device_status", "ojx_e8t_poll_status", "ojx_e8t_set_wait_limit",
     "ojx_e8t_gemv_static_scratch", "ojx_e8t_gemv_static_scratch_capacity", "ojx_e8t_linear", "ojx_e8t_linear_workspace_bytes",
@@ -173,6 +173,8 @@ def _declare(lib: ctypes.CDLL) -> None:
     lib.ojx_e8t_gemv_tiles.argtypes = [i64, i64]
     lib.ojx_e8t_gemv_kchunks.restype = i32
     lib.ojx_e8t_gemv_kchunks.argtypes = [i64]
+    lib.ojx_e8t_gemv_split_flag.restype = i32
+    lib.ojx_e8t_gemv_split_flag.argtypes = [i64, i64]
     lib.ojx_e8t_gemv_grouped.restype = i32
     lib.ojx_e8t_gemv_grouped.argtypes = [vp, i32, i32, i64, i32, i32, i32, vp]
     lib.ojx_e8t_enable_peer_access.restype = i32

@@ -20,6 +20,13 @@ int32_t gemv_tiles_impl(int64_t N, int64_t K) {
 }
 int32_t gemv_kchunks_impl(int64_t K) { return (K > 0 && K % 256 == 0 && K < (1 << 30)) ? gemv_kchunks((int)K) : 0; }
 
+// The split flag of a grouped launch over this one matrix, by the rule of the single-problem entry points.
+int32_t gemv_split_flag_impl(int64_t N, int64_t K) {
+    if (N <= 0 || K <= 0 || K % 256 != 0 || N >= (1 << 30) || K >= (1 << 30)) return 0;
+    const int cluster = mma_cluster_for((int)((N + 15) / 16), mma_chunks((int)K));
+    return cluster == 4 ? OJX_GEMV_SPLIT_K4 : (cluster == 2 ? OJX_GEMV_SPLIT_K2 : 0);
+}
+
 // Scratch that callers of the single-problem entry point bring for K of several chunks.  The kernels keep their partial sums in
 // shared memory and do not touch it; the size stays part of the interface.
 size_t gemv_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {

@@ -988,7 +988,7 @@ static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_
 // K of several chunks over few tiles: the CTAs of a cluster split the chunks, so that each prepares x for its own chunks only
 // and has more tiles to spread that over.  Beyond four tiles per CTA the preparation no longer shows.
 inline int mma_cluster_for(int tiles, int chunks) {
-    if (chunks < 2 || tiles >= 4 * 148) return 1;
+    if (chunks < 2 || tiles >= 4 * num_sms()) return 1;
     return chunks >= 4 ? 4 : 2;
 }
 

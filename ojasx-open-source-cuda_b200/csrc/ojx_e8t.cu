@@ -203,6 +203,7 @@ int32_t ojx_e8t_gemv_static_scratch(const void* x, int32_t x_dtype, int64_t M, c
 
 int32_t ojx_e8t_gemv_tiles(int64_t N, int64_t K) { return ojx::gemv_tiles_impl(N, K); }
 int32_t ojx_e8t_gemv_kchunks(int64_t K) { return ojx::gemv_kchunks_impl(K); }
+int32_t ojx_e8t_gemv_split_flag(int64_t N, int64_t K) { return ojx::gemv_split_flag_impl(N, K); }
 
 int32_t ojx_e8t_gemv_grouped(const ojx_e8t_gemv_problem* problems, int32_t count, int32_t total_tiles, int64_t M,
                              int32_t x_dtype, int32_t y_dtype, int32_t needs_reduce, void* stream) {

@@ -669,9 +669,9 @@ class GroupedGemv:
         self.flags = ((_cabi.OJX_GEMV_STATIC_WEIGHTS if static_weights else 0) | (_cabi.OJX_GEMV_INDEPENDENT if independent else 0) |
                       (_cabi.OJX_GEMV_WAIT_PEERS if wait_peers else 0) | (_cabi.OJX_GEMV_SIGNAL_PEERS if signal_peers else 0) |
                       int(extra_flags))
-        chunks = min((k + 4095) // 4096 for _, k in shapes)
-        if chunks > 1 and sum((n + 15) // 16 for n, _ in shapes) < 4 * 148:     # few rows, long K: clusters of CTAs split K
-            self.flags |= _cabi.OJX_GEMV_SPLIT_K4 if chunks >= 4 else _cabi.OJX_GEMV_SPLIT_K2
+        if self.count == 1:                                    # few rows, long K: clusters of CTAs split K
+            with torch.cuda.device(self.device):
+                self.flags |= lib.ojx_e8t_gemv_split_flag(*(int(v) for v in shapes[0]))
         self._peers = None
         if peer_delta is not None:
             if not (1 <= len(peer_delta) <= 8):

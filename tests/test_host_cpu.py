@@ -49,6 +49,9 @@ def test_pure_host_entry_points(P):
     assert lib.ojx_e8t_gemv_kchunks(8192) == 2 and lib.ojx_e8t_gemv_kchunks(100) == 0
     assert lib.ojx_e8t_gemv_tiles(4096, 4096) == 128 and lib.ojx_e8t_gemv_tiles(4096, 14336) == 512      # 32-row tiles x K chunks
     assert lib.ojx_e8t_gemv_tiles(17, 256) == 1 and lib.ojx_e8t_gemv_tiles(33, 256) == 2
+    k2, k4 = P._cabi.OJX_GEMV_SPLIT_K2, P._cabi.OJX_GEMV_SPLIT_K4       # one rule: chunks of K, fewer than four tiles per multiprocessor
+    assert [lib.ojx_e8t_gemv_split_flag(4096, k) for k in (256, 4096, 4352, 12288, 12544, 14336, 100)] == [0, 0, k2, k2, k4, k4, 0]
+    assert lib.ojx_e8t_gemv_split_flag(4 * 148 * 16, 14336) == 0 and lib.ojx_e8t_gemv_split_flag(4 * 148 * 16 - 16, 14336) == k4
     assert lib.ojx_e8t_gemv_workspace_bytes(4, 4096, 4096) == 0
     assert lib.ojx_e8t_gemv_workspace_bytes(4, 4096, 14336) == 4 * 4 * 4096 * 4
     assert lib.ojx_e8t_gemm_workspace_bytes(2048, 4096, 4096) >= 16
