@@ -220,7 +220,6 @@ template <bool kBf16> __device__ __forceinline__ float load_act(const void* p, i
 // table walked entry by entry cost the last CTAs ~40 us at the start of every grouped launch).  Every thread of
 // the CTA must call this.
 __device__ __forceinline__ int find_problem(const ojx_e8t_gemv_problem* probs, int count, int item, int scale) {
-    if (count == 1) return 0;                                  // single-problem launches (a layer at a time) skip the pass
     int found = 0;
     for (int base = 0; base < count; base += (int)blockDim.x) {
         const int t = base + (int)threadIdx.x;
@@ -252,10 +251,8 @@ __device__ __noinline__ float lora_term(const ojx_e8t_gemv_problem& P, int64_t c
 // stores - to this rank's buffer and to every peer's window.  16-bit outputs whose rows come in multiples of eight
 // are handled eight rows (one 16-byte vector) per thread.
 template <bool kBf16>
-__global__ void __launch_bounds__(256, 3) gemv_reduce_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev,
-                                                           const __grid_constant__ ojx_e8t_gemv_problem single,
-                                                           int count, int M, int y_dtype, const __grid_constant__ PeerMap peers) {
-    const ojx_e8t_gemv_problem* probs = probs_dev != nullptr ? probs_dev : &single;
+__global__ void __launch_bounds__(256, 3) gemv_reduce_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, int count, int M, int y_dtype,
+                                                           const __grid_constant__ PeerMap peers) {
     for (int p = blockIdx.y; p < count; p += gridDim.y) {
         const ojx_e8t_gemv_problem& P = probs[p];
         if (P.partial == nullptr) continue;

@@ -103,12 +103,11 @@ __device__ __forceinline__ void a16_decode(uint32_t (&a)[4], uint32_t w0, uint32
 
 template <int NB, bool kXF16, bool kI8 = false>
 __global__ void __launch_bounds__(kGemvThreads, 1)
-gemv_a16_kernel(const ojx_e8t_gemv_problem* __restrict__ probs_dev, const __grid_constant__ ojx_e8t_gemv_problem single,
-                int count, int total_items, int M, int y_dtype, int overlap, const __grid_constant__ PeerMap peers) {
+gemv_a16_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, int count, int total_items, int M, int y_dtype, int overlap,
+                const __grid_constant__ PeerMap peers) {
     static_assert(!kI8 || (NB == 1 && !kXF16), "the int8 path serves one bf16 activation row");
     using Cfg = A16Cfg<NB>;
     constexpr int S = Cfg::kStages;
-    const ojx_e8t_gemv_problem* probs = probs_dev != nullptr ? probs_dev : &single;
     extern __shared__ __align__(128) uint8_t smem[];
     const uint32_t lut = smem_u32(smem);
     const uint32_t ring = lut + Cfg::kLutBytes;

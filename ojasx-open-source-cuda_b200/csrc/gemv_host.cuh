@@ -36,8 +36,8 @@ size_t gemv_workspace_bytes_impl(int64_t M, int64_t N, int64_t K) {
 }
 
 template <int NB, bool kXF16, bool kI8 = false>
-static int32_t launch_gemv_a16(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count, int total,
-                               int M, int y_dtype, const PeerMap& peers_in, int overlap, cudaStream_t s) {
+static int32_t launch_gemv_a16(const ojx_e8t_gemv_problem* probs, int count, int total, int M, int y_dtype,
+                               const PeerMap& peers_in, int overlap, cudaStream_t s) {
     PeerMap peers = peers_in;
     peers.host_status = host_status_device_ptr(s);
     peers.wait_limit = wait_limit_override() != 0 ? wait_limit_override() : kSpinLimit;
@@ -49,18 +49,18 @@ static int32_t launch_gemv_a16(const ojx_e8t_gemv_problem* probs, const ojx_e8t_
     const int per = (total + sms - 1) / sms;
     const int grid = (total + per - 1) / per;
     return launch_maybe_overlapped(gemv_a16_kernel<NB, kXF16, kI8>, grid, kGemvThreads, Cfg::kSmem, s, overlap != 0, 1,
-                                   probs, single, count, total, M, y_dtype, overlap, peers);
+                                   probs, count, total, M, y_dtype, overlap, peers);
 }
 
 // One bf16 activation row takes the int8 path; one to eight rows take one block of eight columns per fp16 MMA, nine to
 // sixteen take two.
-static int32_t dispatch_gemv(bool bf16, const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_problem& single, int count,
-                             int total, int M, int y_dtype, const PeerMap& peers, int overlap, cudaStream_t s) {
-    if (bf16 && M == 1) return launch_gemv_a16<1, false, true>(probs, single, count, total, M, y_dtype, peers, overlap, s);
-    if (bf16) return M <= 8 ? launch_gemv_a16<1, false>(probs, single, count, total, M, y_dtype, peers, overlap, s)
-                            : launch_gemv_a16<2, false>(probs, single, count, total, M, y_dtype, peers, overlap, s);
-    return M <= 8 ? launch_gemv_a16<1, true>(probs, single, count, total, M, y_dtype, peers, overlap, s)
-                  : launch_gemv_a16<2, true>(probs, single, count, total, M, y_dtype, peers, overlap, s);
+static int32_t dispatch_gemv(bool bf16, const ojx_e8t_gemv_problem* probs, int count, int total, int M, int y_dtype,
+                             const PeerMap& peers, int overlap, cudaStream_t s) {
+    if (bf16 && M == 1) return launch_gemv_a16<1, false, true>(probs, count, total, M, y_dtype, peers, overlap, s);
+    if (bf16) return M <= 8 ? launch_gemv_a16<1, false>(probs, count, total, M, y_dtype, peers, overlap, s)
+                            : launch_gemv_a16<2, false>(probs, count, total, M, y_dtype, peers, overlap, s);
+    return M <= 8 ? launch_gemv_a16<1, true>(probs, count, total, M, y_dtype, peers, overlap, s)
+                  : launch_gemv_a16<2, true>(probs, count, total, M, y_dtype, peers, overlap, s);
 }
 
 int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int total_tiles, int64_t M,
@@ -102,12 +102,12 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     // table and needs no reduce launch (1024 x 2560: 4.0 and 8.9 us against 4.8 and 12.7, 4096 x 14336: 15.4 against 15.8).
     if (count > 1) {
         if (needs_reduce && peers.sync != nullptr) peers.mode |= 0x100;      // a reduce kernel follows and stores (and signals) in its place
-        const int32_t st = dispatch_gemv(bf, problems, none, count, total_tiles, (int)M, y_dtype, peers, overlap, s);
+        const int32_t st = dispatch_gemv(bf, problems, count, total_tiles, (int)M, y_dtype, peers, overlap, s);
         OJX_RETURN_IF(st != OJX_OK || !needs_reduce, st);
         // Problems whose K spans several chunks carry a partial buffer; the reduce pass skips the rest.
         dim3 grid(64, count > 64 ? 64 : count);
-        if (bf) gemv_reduce_kernel<true><<<grid, 256, 0, s>>>(problems, none, count, (int)M, y_dtype, peers);
-        else gemv_reduce_kernel<false><<<grid, 256, 0, s>>>(problems, none, count, (int)M, y_dtype, peers);
+        if (bf) gemv_reduce_kernel<true><<<grid, 256, 0, s>>>(problems, count, (int)M, y_dtype, peers);
+        else gemv_reduce_kernel<false><<<grid, 256, 0, s>>>(problems, count, (int)M, y_dtype, peers);
         return launch_status();
     }
     peers.host_status = host_status_device_ptr(s);

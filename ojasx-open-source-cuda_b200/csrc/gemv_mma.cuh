@@ -918,7 +918,7 @@ inline bool gemv_mma_ok(int fmt, int64_t M, int64_t N, int64_t K, int group, int
 }
 
 // `max_per`: slices per chunk of the launch's largest item.
-template <int FMT, int G, int NB, bool kRag, bool kI8>
+template <int FMT, int G, int NB, bool kRag>
 inline MmaPlan mma_plan(int M, int max_per, bool chunked, int cluster) {
     using F = MmaFmt<FMT, G>;
     using Sh = MmaShape<FMT, G, NB, kRag>;
@@ -977,7 +977,7 @@ static int32_t mma_launch(const ojx_e8t_gemv_problem* probs, const ojx_e8t_gemv_
         room = f.load(std::memory_order_relaxed) - 1;
         if (room <= 0) { cluster = 1; room = num_sms(); }
     }
-    const MmaPlan plan = mma_plan<FMT, G, NB, kRag, kI8>(M, max_per, chunked, cluster);
+    const MmaPlan plan = mma_plan<FMT, G, NB, kRag>(M, max_per, chunked, cluster);
     const int grid = (units < room ? units : room) * cluster;
     // a launch that waits for its peers reads x after them whatever it may read before the launch ahead has ended
     const bool late_x = peers.sync != nullptr && (peers.mode & OJX_GEMV_WAIT_PEERS) != 0;
