@@ -124,7 +124,8 @@ def test_decode_kernels_keep_non_finite_activations_in_their_row(P, bits, group,
 
 @pytest.mark.parametrize("m", [1, 4, 12])
 def test_grouped_launch_over_many_matrices_of_different_shapes(P, m):
-    """Whole CTAs per matrix (few matrices), an even cut of the cost (many), K of one and of several chunks."""
+    """Work items that run across matrix borders, tables of more entries than a CTA has threads' worth of items, K of one and of
+    several chunks in one launch."""
     dev = torch.device(DEV)
     for count in (2, 40, 300):
         entries, shapes, want = [], [], []
@@ -302,3 +303,16 @@ def test_batches_of_tokens_over_scales_of_every_size(P, bits, group, m, n, k):
         keep = [i for i in range(m) if i not in (3, 9, 10)]
         assert torch.equal(y2[keep], y[keep])
     P.ops.gemm_status(torch.device(DEV))
+
+
+@pytest.mark.parametrize("bits,group", [(1.5, 32), (1.5, 16), (2.0, 8), (1.0, 32)])
+@pytest.mark.parametrize("m,n,k", [(1, 40, 256), (3, 33, 4096), (20, 24, 288)])
+def test_activations_that_are_not_aligned_take_the_fp32_kernels(P, bits, group, m, n, k):
+    """x at an address that is no multiple of 16: the scalar kernel of the format, 16-bit and fp32 activations."""
+    packed, scales, wd = _problem(P, bits, n, k, group)
+    fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    for dt in (torch.bfloat16, torch.float16, torch.float32):
+        x = P.ops.generate(m * k + 1, 8, 1.0, dt, torch.device(DEV))[1:].view(m, k)
+        y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
+        ref, bound = x.double() @ wd.double().t(), x.double().abs() @ wd.double().abs().t()
+        assert float(((y.double() - ref).abs() / bound.clamp_min(1e-30)).max()) <= 2e-6, dt

@@ -159,8 +159,7 @@ def test_gemv_fp16(P, oracle, m):
 
 
 def test_gemv_fp32_out_is_tight(P, oracle):
-    # with fp32 output what is left is the 13-bit fixed-point form of the activations inside the int8
-    # tensor-core kernels (error <= 2^-13 of each 256-wide slice's maximum, exact for large elements)
+    # weights and bf16 activations are exact fp16 operands: with fp32 output what is left is the order of the fp32 sums
     n, k, m = 96, 4096, 4
     w = oracle.gen_normal(5, n * k, 0.02).reshape(n, k)
     packed_np, scales_np, _ = oracle.encode(w, 32)
@@ -176,7 +175,7 @@ def test_gemv_fp32_out_is_tight(P, oracle):
 @pytest.mark.parametrize("n,k,m,xdt", [(7, 13, 3, torch.float32), (5, 19, 2, torch.float32), (4, 48, 2, torch.float32),
                                        (24, 128, 5, torch.bfloat16), (40, 96, 20, torch.float32)])
 def test_generic_path_odd_shapes(P, oracle, n, k, m, xdt):
-    # flat packing whose groups cross row boundaries, fp32 activations, K not a multiple of 256
+    # flat packing whose groups cross row boundaries, fp32 activations; beside them K of four groups and 16-bit activations
     g = 16 if k % 32 else 32
     w = oracle.gen_normal(n * k, n * k, 0.5).reshape(n, k)
     packed_np, scales_np, _ = oracle.encode(w, g)
@@ -229,7 +228,7 @@ def test_gemm_matches_gemv_small_batch(P, oracle):
     y1 = P.ops.linear(x, packed, scales, None, n, k, 32, out_dtype=torch.float32, force="gemv")
     y2 = P.ops.linear(x, packed, scales, None, n, k, 32, out_dtype=torch.float32, force="gemm")
     P.ops.gemm_status(torch.device(DEV))
-    assert float((y1 - y2).norm() / y1.norm()) < 1e-4     # activation fixed-point error of the decode kernel
+    assert float((y1 - y2).norm() / y1.norm()) < 1e-4     # fp32 sums in another order, and the tcgen05 accumulators' rounding
 
 
 def test_grouped_gemv_matches_single(P, oracle):
@@ -592,10 +591,12 @@ def test_low_bit_decode_linear_matches_dense_product(P, oracle, bits, m, k, n, g
 @pytest.mark.parametrize("m,k,n,dt", [(1, 2048, 40, torch.bfloat16), (1, 4096, 4096, torch.bfloat16), (1, 14336, 100, torch.float16),
                                       (1, 8192, 17, torch.float32), (2, 4096, 100, torch.bfloat16), (3, 2048, 33, torch.float16),
                                       (4, 8192, 64, torch.bfloat16), (5, 2048, 48, torch.float32), (8, 4096, 4096, torch.bfloat16),
-                                      (7, 4096, 20, torch.float16)])
+                                      (7, 4096, 20, torch.float16), (2, 2048, 33, torch.float32), (4, 4096, 20, torch.float32),
+                                      (8, 2048, 17, torch.float32)])
 @pytest.mark.parametrize("bits", [2, 1])
 def test_low_bit_tensor_core_kernels(P, oracle, bits, m, k, n, dt):
-    """gemv_b2_kernel / gemv_b1_kernel (one to eight rows, groups of 32, K % 2048 == 0) against the dense fp32 product: within 1e-5 of
+    """gemv_b2_kernel / gemv_b1_kernel (groups of 32, K % 2048 == 0: one to eight rows of fp32 activations, one, in the 1.0-bit format
+    two, of 16-bit ones) and gemv_mma_kernel, which takes the other 16-bit rows, against the dense fp32 product: within 1e-5 of
     sum |x||w| per output (row counts that are not multiples of 16 included), outliers do not hurt their neighbours,
     scaling x by a power of two scales y exactly, Inf / NaN give the dense product's pattern and leave the other rows
     of x within the same bound."""
@@ -717,8 +718,8 @@ def test_low_bit_backward_dx_matches_dense_product(P, oracle, bits, m, k, n, dt,
                                       (8, 2048, 24, torch.bfloat16)])
 def test_ternary_groups_of_16_run_the_tensor_core_kernels(P, oracle, m, k, n, dt):
     """Ternary codes with one scale per 16 weights (what the reference layer's default group size of 8 becomes for this
-    format, ojasx2/math/lattice.py:750-751): forward (the shared-memory fp32 kernel for one or two rows, the tcgen05 kernel
-    beyond) and backward (tcgen05) against the fp32 products with the decoded weights, which are exact in fp16 -
+    format, ojasx2/math/lattice.py:750-751): forward (gemv_mma_kernel up to sixteen rows, the tcgen05 kernel beyond) and
+    backward (tcgen05) against the fp32 products with the decoded weights, which are exact in fp16 -
     within 2e-5 of sum |x||w| per output."""
     dev = torch.device(DEV)
     w = torch.from_numpy(oracle.gen_normal(990 + n, n * k, 0.02).reshape(n, k).copy()).to(dev)
@@ -767,8 +768,8 @@ def test_ternary_fp32_activations_at_decode_shapes(P, oracle, m, k, n, group):
 @pytest.mark.parametrize("bits", [2, 1])
 @pytest.mark.parametrize("m,k,n,r,dt", [(1, 4096, 100, 8, torch.bfloat16), (4, 2048, 48, 16, torch.float16), (8, 4096, 33, 3, torch.float32)])
 def test_low_bit_adapter_epilogue(P, oracle, bits, m, k, n, r, dt):
-    """ojx_e8t_linear_lowbit_lora: the packed product, bias and the low-rank term in one launch of the int8 tensor-core
-    decode kernels, against the fp32 sum of the three - within 1e-5 of sum |x||w| + |bias| + sum |t||B| per output;
+    """ojx_e8t_linear_lowbit_lora: the packed product, bias and the low-rank term in one launch of the tensor-core decode
+    kernels (gemv_b2 / gemv_b1 for one row and for fp32 activations, gemv_mma for the others), against the fp32 sum of the three - within 1e-5 of sum |x||w| + |bias| + sum |t||B| per output;
     then a layer with an adapter at decode shapes against the reference's formula (lattice.py:839-842)."""
     dev = torch.device(DEV)
     w = torch.from_numpy(oracle.gen_normal(1000 + n, n * k, 0.02).reshape(n, k).copy()).to(dev)

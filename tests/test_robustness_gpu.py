@@ -37,9 +37,10 @@ def _problem(P, n, k, m, seed):
 
 
 def test_chain_orders_itself_on_the_device(P):
-    """Two dependent grouped launches - the second reads what the first wrote - ordered by the peer-sync block
-    alone (one rank, so 'every rank' is this one): results equal the unsynchronised path, the epoch counts the
-    signalled launches, and K > 4096 (partial sums + reduce kernel) signals from the reduce kernel."""
+    """Dependent grouped launches - the second reads what the first wrote - ordered by the peer-sync block alone (one
+    rank, so 'every rank' is this one): results equal the unsynchronised path and the epoch counts the signalled
+    launches.  The third splits K over a cluster; the fourth, over two matrices with K > 4096, signals from the reduce
+    kernel, and the fifth, over two matrices, from its main kernel."""
     dev = torch.device(DEV)
     m = 4
     pk1, sc1, x = _problem(P, 512, 4096, m, 10)
@@ -55,15 +56,22 @@ def test_chain_orders_itself_on_the_device(P):
                                wait_peers=True, signal_peers=True, static_weights=True)
     third = P.ops.GroupedGemv([(x3, pk3, sc3, None, out3)], [(128, 14336)], peer_delta=[0], peer_sync=sync.data_ptr(),
                               wait_peers=True, signal_peers=True, static_weights=True)
+    sync4 = dict(peer_delta=[0], peer_sync=sync.data_ptr(), wait_peers=True, signal_peers=True, static_weights=True)
+    out4 = [torch.zeros((m, 128), dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    out5 = [torch.zeros((m, 256), dtype=torch.bfloat16, device=dev) for _ in range(2)]
+    fourth = P.ops.GroupedGemv([(x3, pk3, sc3, None, y) for y in out4], [(128, 14336)] * 2, **sync4)
+    fifth = P.ops.GroupedGemv([(mid, pk2, sc2, None, y) for y in out5], [(256, 512)] * 2, **sync4)
     for _ in range(3):
-        first(); second(); third()
+        first(); second(); third(); fourth(); fifth()
     torch.cuda.synchronize()
     ref_mid = P.ops.linear(x, pk1, sc1, None, 512, 4096, 32)
     ref_out = P.ops.linear(ref_mid, pk2, sc2, None, 256, 512, 32)
     ref3 = P.ops.linear(x3, pk3, sc3, None, 128, 14336, 32)
     assert torch.equal(mid, ref_mid) and torch.equal(out, ref_out) and torch.equal(out3, ref3)
     words = sync.cpu().numpy()
-    assert words[0] == 9 and words[1] == 0 and words[2] == 0 and words[4] == 9      # epoch, arrived, status, flag[0]
+    assert words[0] == 15 and words[1] == 0 and words[2] == 0 and words[4] == 15    # epoch, arrived, status, flag[0]
+    for got, want in [(y, ref3) for y in out4] + [(y, ref_out) for y in out5]:              # another kernel: sums in another order
+        assert float((got.float() - want.float()).norm() / want.float().norm()) <= 4e-3
     assert P._cabi.lib().ojx_e8t_device_status() == 0
 
 
@@ -118,16 +126,18 @@ def test_wait_on_a_rank_that_never_signals_gives_up(P):
     assert lib.ojx_e8t_device_status() == 0
 
 
-def test_copy_that_never_completes_gives_up(P):
-    """The loader withholds one arrival on the first work item's 'copies landed' barrier: every warp's wait on it
-    runs into the (shortened) limit, the CTAs stop touching their inputs, keep their barriers matched, wait for
-    the copies that are in flight, and return."""
+@pytest.mark.parametrize("count", [1, 2])
+def test_copy_that_never_completes_gives_up(P, count):
+    """A wait inside the kernel that nothing ends (several matrices: the loader withholds one arrival on the first work
+    item's 'copies landed' barrier; one matrix: a barrier made for this) runs into the (shortened) limit, the CTAs stop
+    touching their inputs, keep their barriers matched, wait for the copies that are in flight, and return."""
     dev = torch.device(DEV)
     lib = P._cabi.lib()
     pk, sc, x = _problem(P, 4096, 4096, 16, 50)
     y = torch.zeros((16, 4096), dtype=torch.bfloat16, device=dev)
-    good = P.ops.GroupedGemv([(x, pk, sc, None, y)], [(4096, 4096)])
-    bad = P.ops.GroupedGemv([(x, pk, sc, None, y)], [(4096, 4096)], extra_flags=P._cabi.OJX_GEMV_TEST_LOSE_COPY)
+    entries = [(x, pk, sc, None, y)] + [(x, pk, sc, None, torch.zeros_like(y))] * (count - 1)
+    good = P.ops.GroupedGemv(entries, [(4096, 4096)] * count)
+    bad = P.ops.GroupedGemv(entries, [(4096, 4096)] * count, extra_flags=P._cabi.OJX_GEMV_TEST_LOSE_COPY)
     lib.ojx_e8t_set_wait_limit(3000)
     try:
         bad()
