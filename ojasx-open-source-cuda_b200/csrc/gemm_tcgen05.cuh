@@ -76,7 +76,7 @@ struct GemmParams {
 };
 
 // Activation pre-pass: a group of TPR threads (a warp for rows of up to 4096 elements, else the whole CTA)
-// takes one token row, finds its largest magnitude, then writes the row as fp16 scaled by the power of two
+// takes one token row, finds its largest finite magnitude, then writes the row as fp16 scaled by the power of two
 // that brings that magnitude into [2^14, 2^15), and the inverse factor for the epilogue.  Rows of up to
 // TPR * 8 * VECS elements stay in registers between the two steps (one global read); longer rows are read
 // twice.  kSplit (2.0-bit weights in two parts): fp16 rows are not scaled, rows are written twice, each time filled up with zeros
@@ -110,7 +110,10 @@ __global__ void __launch_bounds__(256) normalize_rows_to_f16_kernel(const T* __r
         auto largest = [&](const uint4& v) {
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int q = 0; q < 4; ++q) m = max(m, max((w[q] << 16) & 0x7FFFFFFFu, w[q] & 0x7FFF0000u));
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t a = (w[q] << 16) & 0x7FFFFFFFu, b = w[q] & 0x7FFF0000u;
+                m = max(m, max(a < 0x7F800000u ? a : 0u, b < 0x7F800000u ? b : 0u));
+            }
         };
         if (resident) {
 #pragma unroll
@@ -128,7 +131,7 @@ __global__ void __launch_bounds__(256) normalize_rows_to_f16_kernel(const T* __r
         }
         int e = 0;
         const int ex = (int)((m >> 23) & 0xFFu);
-        if (ex != 0 && ex != 0xFF) e = max(-100, min(100, ex - 127 - 14));
+        if (ex != 0) e = max(-100, min(100, ex - 127 - 14));
         down = __int_as_float((127 - e) << 23);
         if (t == 0 && live) up[row] = __int_as_float((127 + e) << 23);
     }

@@ -316,3 +316,19 @@ def test_activations_that_are_not_aligned_take_the_fp32_kernels(P, bits, group, 
         y = fn(x, packed, scales, None, n, k, group, out_dtype=torch.float32)
         ref, bound = x.double() @ wd.double().t(), x.double().abs() @ wd.double().abs().t()
         assert float(((y.double() - ref).abs() / bound.clamp_min(1e-30)).max()) <= 2e-6, dt
+
+
+@pytest.mark.parametrize("bits", [1.5, 2.0, 1.0])
+@pytest.mark.parametrize("n,k", [(40, 512), (40, 288), (24, 8224)])
+def test_batches_of_tokens_with_large_values_beside_infinities(P, bits, n, k):
+    """A token with an infinity and finite values that fp16 does not have: they stay finite, so that the dense product's Inf is no NaN."""
+    m = 20
+    packed, scales, wd = _problem(P, bits, n, k, 32)
+    fn = {1.0: P.ops.linear_1bit, 1.5: P.ops.linear, 2.0: P.ops.linear_2bit}[bits]
+    x = P.ops.generate(m * k, 8, 1.0, torch.bfloat16, torch.device(DEV)).view(m, k).clone()
+    x[:, 1::7] *= 1e20
+    x[3, 5], x[7, k - 1], x[9, 0] = float("inf"), -float("inf"), float("nan")
+    y, ref = fn(x, packed, scales, None, n, k, 32), x.float() @ wd.t()
+    assert torch.equal(torch.isnan(y), torch.isnan(ref)) and torch.equal(torch.isinf(y), torch.isinf(ref))
+    keep = [i for i in range(m) if i not in (3, 7, 9)]
+    assert float((y[keep].double() - ref[keep].double()).norm() / ref[keep].double().norm()) <= 4e-3
