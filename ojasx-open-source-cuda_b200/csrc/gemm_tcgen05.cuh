@@ -107,20 +107,28 @@ __global__ void __launch_bounds__(256) normalize_rows_to_f16_kernel(const T* __r
     }
     float down = 1.f;
     if constexpr (kBf16) {
-        auto largest = [&](const uint4& v) {
+        // magnitudes as pairs of bf16 bits; with Inf or NaN among them (rare) once more without those
+        auto largest = [&](const uint4& v, bool finite) {
             const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const uint32_t a = (w[q] << 16) & 0x7FFFFFFFu, b = w[q] & 0x7FFF0000u;
-                m = max(m, max(a < 0x7F800000u ? a : 0u, b < 0x7F800000u ? b : 0u));
+                uint32_t mag = w[q] & 0x7FFF7FFFu;
+                if (finite) mag = ((mag & 0xFFFFu) < 0x7F80u ? mag & 0xFFFFu : 0u) | ((mag >> 16) < 0x7F80u ? mag & 0xFFFF0000u : 0u);
+                m = __vmaxu2(m, mag);
             }
         };
-        if (resident) {
+        auto scan = [&](bool finite) {
+            m = 0;
+            if (resident) {
 #pragma unroll
-            for (int j = 0; j < VECS; ++j) largest(keep[j]);
-        } else {
-            for (int64_t i = t; i < vecs; i += TPR) largest(__ldg(src + i));
-        }
+                for (int j = 0; j < VECS; ++j) largest(keep[j], finite);
+            } else {
+                for (int64_t i = t; i < vecs; i += TPR) largest(__ldg(src + i), finite);
+            }
+            m = max(m & 0xFFFFu, m >> 16);
+        };
+        scan(false);
+        if (m >= 0x7F80u) scan(true);
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
         if (TPR > 32) {
@@ -130,7 +138,7 @@ __global__ void __launch_bounds__(256) normalize_rows_to_f16_kernel(const T* __r
             for (int w = 0; w < 8; ++w) m = max(m, warp_max[w]);
         }
         int e = 0;
-        const int ex = (int)((m >> 23) & 0xFFu);
+        const int ex = (int)(m >> 7);
         if (ex != 0) e = max(-100, min(100, ex - 127 - 14));
         down = __int_as_float((127 - e) << 23);
         if (t == 0 && live) up[row] = __int_as_float((127 + e) << 23);
