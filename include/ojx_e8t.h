@@ -121,12 +121,14 @@ int32_t ojx_e8t_fwht32(const void* x, int32_t dtype, int64_t count, void* out, v
  *   ojx_e8t_linear_2bit   y[M, N] = x[M, K] . W^T (+ bias) from the packed codes in one fp32 kernel (any shape,
  *                         any of the three dtypes for x, bias (x's dtype) and y); replaces the 2.0-bit branch of
  *                         _FusedE8GEMMFunction.forward (ojasx2/math/lattice.py:596-624) and the native
- *                         fused_e8_gemm_forward<T> (ojasx2/math/csrc/ojasx_math_core.hpp:444).  One to eight rows
- *                         with group 32, K % 2048 == 0 and 16-byte aligned operands run on int8 tensor cores
- *                         (activations as 28-bit fixed point per scale group, as in ojx_e8t_gemv for one bf16 row;
- *                         Inf / NaN in x give the dense product's pattern); other shapes of up to eight rows with
- *                         K % 16 == 0 and 16-byte aligned x run a shared-memory fp32 kernel (a row of x with Inf
- *                         comes out as NaN there), everything else a scalar fp32 kernel.
+ *                         fused_e8_gemm_forward<T> (ojasx2/math/csrc/ojasx_math_core.hpp:444).  Up to sixteen rows of
+ *                         16-bit x with groups of 8, 16 or 32, K % 32 == 0 and 16-byte aligned operands run on fp16 tensor
+ *                         cores with exact weights; one row of 16-bit x and up to eight of fp32 x with group 32 and
+ *                         K % 2048 == 0 on int8 ones (activations as 28-bit fixed point per scale group, as in
+ *                         ojx_e8t_gemv for one bf16 row); Inf / NaN in x give the dense product's pattern.  Other shapes
+ *                         of up to eight rows with K % 16 == 0 and 16-byte aligned x run a shared-memory fp32 kernel (a
+ *                         row of x with Inf comes out as NaN there), everything else a scalar fp32 kernel.  (Batches
+ *                         of tokens: ojx_e8t_linear.)
  */
 int32_t ojx_e8t_encode_2bit(const void* w, int32_t w_dtype, int64_t rows, int64_t cols, int32_t group,
                             uint8_t* packed_out, uint16_t* scales_out, void* stream);
@@ -145,9 +147,10 @@ int32_t ojx_e8t_linear_2bit(const void* x, int32_t x_dtype, int64_t M, const uin
  *                         torch.sum adds chunks of eight into four vector accumulators in turn; a BLAS that rounds the
  *                         8-term dot products differently may pick the other of two nearly equal candidates.
  *   ojx_e8t_decode_1bit   replaces RootE8LatticePacker.unpack (ojasx2/math/lattice.py:514-537)
- *   ojx_e8t_linear_1bit   y = x . W^T (+ bias) from the codes; the same three kernels as for 2 bits: int8 tensor
- *                         cores for one to eight rows with group 32 and K % 2048 == 0 (a code byte is looked up as
- *                         eight int8 operand bytes), the shared-memory fp32 kernel, the scalar fp32 kernel
+ *   ojx_e8t_linear_1bit   y = x . W^T (+ bias) from the codes; the same kernels as for 2 bits: fp16 tensor cores, int8
+ *                         ones for one or two rows of 16-bit x and up to eight of fp32 x with group 32 and K % 2048 == 0
+ *                         (a code byte is looked up as eight int8 operand bytes), the shared-memory fp32 kernel, the
+ *                         scalar fp32 kernel
  */
 int32_t ojx_e8t_encode_1bit(const void* w, int32_t w_dtype, int64_t rows, int64_t cols, int32_t group,
                             uint8_t* packed_out, uint16_t* scales_out, void* stream);
@@ -160,9 +163,9 @@ int32_t ojx_e8t_linear_1bit(const void* x, int32_t x_dtype, int64_t M, const uin
  * Decode-shape linear of the 2.0-bit (`bits` 2) or 1.0-bit (`bits` 1) format with the adapter term in the epilogue:
  * y = x . W^T (+ bias) + lora_t . lora_b, lora_t fp32 [M, lora_rank] = scaling * (x . A) prepared by the caller,
  * lora_b [lora_rank, N] in x's dtype, accumulated in fp32 before the single rounding (the reference adds the term with
- * three more tensor operations, ojasx2/math/lattice.py:839-842).  Only the shapes of the int8 tensor-core kernels are
- * served (1 <= M <= 8, group 32, K % 2048 == 0, 16-byte aligned operands, 1 <= lora_rank <= 64); anything else returns
- * OJX_ERR_UNSUPPORTED and the caller adds the term itself.
+ * three more tensor operations, ojasx2/math/lattice.py:839-842).  Only the shapes of the tensor-core kernels are served
+ * (16-bit x: 1 <= M <= 16, groups of 8, 16 and 32, K % 32 == 0; fp32 x: M <= 8, group 32, K % 2048 == 0; 16-byte aligned
+ * operands, 1 <= lora_rank <= 64); anything else returns OJX_ERR_UNSUPPORTED and the caller adds the term itself.
  */
 int32_t ojx_e8t_linear_lowbit_lora(int32_t bits, const void* x, int32_t x_dtype, int64_t M, const uint8_t* packed,
                                    const uint16_t* scales, const void* bias, int64_t N, int64_t K, int32_t group,
@@ -200,15 +203,15 @@ int32_t ojx_e8t_decode(const uint8_t* packed, const uint16_t* scales, int64_t ro
  * Replaces _FusedE8GEMMFunction.forward for small batches (ojasx2/math/lattice.py:551-640) and the
  * reference's native fused kernel (ojasx_math_core.hpp:580-634).  fp32 accumulation.
  * Shapes outside the tensor-core path: up to eight rows with K % 64 == 0, a power-of-two group from 16 and 16-byte
- * aligned x (any of the three dtypes) run a shared-memory fp32 kernel with exact products; everything else a scalar
+ * aligned x (fp32 x, or groups above 32) run a shared-memory fp32 kernel with exact products; everything else a scalar
  * fp32 kernel.
- * Numerics of the tensor-core path (M <= 16, K % 256 == 0, group 32, bf16 or fp16 x): the weights enter the
+ * Numerics of the tensor-core path (M <= 16, K % 32 == 0, groups of 32 and 16, bf16 or fp16 x): the weights enter the
  * MMAs as exact fp16 values coord * scale; fp16 activations are used as they are; bf16 activations are
  * multiplied by a power of two per (row, 256-wide slice of K) so that the slice maximum lies in [2^14, 2^15)
  * and converted to fp16 - exact for every element within 2^-29 of its slice maximum, so an activation
  * outlier does not degrade its neighbours; products are exact and accumulate in fp32.  Inf and NaN in x reach
  * every output of that activation row (0 * Inf = NaN, as in a dense product).
- * One bf16 activation row (M == 1, the decode case) runs on int8 tensor cores instead: the 32 activations of a
+ * One bf16 activation row (M == 1, the decode case) with K % 256 == 0 and group 32 runs on int8 tensor cores instead: the 32 activations of a
  * scale group share the exponent of their largest finite magnitude and become 28-bit integers (four signed
  * base-128 digits, one int8 MMA operand each), the ternary coordinates are int8, the integer dot product of a
  * group is exact and is scaled once by weight scale * 2^exponent in fp32.  Every activation within 2^-19 of
@@ -219,9 +222,10 @@ int32_t ojx_e8t_decode(const uint8_t* packed, const uint16_t* scales, int64_t ro
  * Other shapes and fp32 activations run a plain fp32 kernel.
  *   x, y       row-major, dtypes x_dtype / y_dtype (bf16, fp16 or fp32)
  *   bias       [N] in x_dtype, or null
- *   group      must be 32 and K % 32 == 0 (every row owns whole groups)
+ *   group      as in the encoder: anything that is not a positive multiple of 16 means 16
  *   workspace  scratch of at least ojx_e8t_gemv_workspace_bytes(M, N, K) bytes (may be null when
- *              that function returns 0); contents need not be initialised
+ *              that function returns 0).  The kernels keep their partial sums in shared memory and do not touch it; a
+ *              missing or short one is still refused
  */
 size_t  ojx_e8t_gemv_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int32_t ojx_e8t_gemv(const void* x, int32_t x_dtype, int64_t M,
@@ -248,19 +252,13 @@ int32_t ojx_e8t_gemv_lora(const void* x, int32_t x_dtype, int64_t M,
  * ojx_e8t_gemv for callers that cannot hand over scratch memory (no counterpart in the reference).
  * Meant for hosts where a plug-in only ever sees its input and output buffers: a serving process whose
  * device memory is pre-carved by its own arena, a callback that runs where cudaMalloc is not allowed
- * (it synchronises the device), a worker without allocation rights.  The fp32 partial sums that
- * K > 4096 needs are kept in a 4 MiB array that is part of the library image on every GPU that loads
- * it; the call allocates nothing and frees nothing.
+ * (it synchronises the device), a worker without allocation rights.  The kernels keep the partial sums of
+ * K > 4096 in shared memory, so the call needs no scratch, allocates nothing and frees nothing.
  *   - Same arguments and results as ojx_e8t_gemv, minus the workspace.
- *   - Limit: ojx_e8t_gemv_workspace_bytes(M, N, K) must not exceed
- *     ojx_e8t_gemv_static_scratch_capacity() (4 MiB; e.g. K = 14336, N = 4096, M = 16 needs 1 MiB);
- *     larger problems return OJX_ERR_WORKSPACE and must use ojx_e8t_gemv with caller scratch.
- *   - The first call on each device looks up the array's device address (a driver query, done once
- *     per device with that device current); make that first call before starting a stream capture.
- *   - All calls share the one array.  It keeps whatever the last call left; nothing needs clearing
- *     because every element is written before it is read.  Two calls that run on the GPU at the same
- *     time (different streams, or different threads) would overwrite each other's partial sums:
- *     serialise them.
+ *   - Limit, part of the interface: ojx_e8t_gemv_workspace_bytes(M, N, K) must not exceed
+ *     ojx_e8t_gemv_static_scratch_capacity() (4 MiB; e.g. K = 14336, N = 4096, M = 16 is 1 MiB);
+ *     larger problems return OJX_ERR_WORKSPACE and must use ojx_e8t_gemv.
+ *   - Calls share nothing: they may run at the same time, from any stream or thread, and inside a capture.
  */
 size_t  ojx_e8t_gemv_static_scratch_capacity(void);
 int32_t ojx_e8t_gemv_static_scratch(const void* x, int32_t x_dtype, int64_t M,
@@ -291,7 +289,7 @@ typedef struct {
      *   y[m, n] += sum_r lora_t[m, r] * lora_b[r, n]
      * lora_t = scaling * (x . A) as fp32 [M, lora_rank] (computed by the caller; it is read after the product, so it may
      * be produced by work queued just ahead of the launch), lora_b [lora_rank, N] in x's dtype.  lora_rank == 0: none;
-     * honoured for M <= 8.
+     * honoured for M <= 8 (in launches over one matrix for M <= 16).
      * This is the adapter term of E8LatticeLinear.forward_fused (ojasx2/math/lattice.py:839-842). */
     const float*    lora_t;
     const void*     lora_b;

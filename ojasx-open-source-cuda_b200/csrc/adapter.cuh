@@ -3,7 +3,7 @@
 // as two launches: adapter_prologue_kernel (t = scaling * (x . A) in fp32, and H(x)) and the decode kernel, whose epilogue adds
 // t . B.  Through the tensor library the same layer took a product of A (6.7 us at 4 x 4096 x 16), a conversion, a scaling, the
 // transform and the decode kernel one after the other (23 us on the GPU and 77 us of host time per call); the two launches take
-// 12.5 us, since the decode kernel starts beside the first and only waits for it before it reads x.
+// 14.4 us, since the decode kernel starts beside the first and only waits for it before it reads x.
 #pragma once
 
 #include <cooperative_groups.h>

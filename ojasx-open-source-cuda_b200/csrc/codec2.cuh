@@ -132,8 +132,9 @@ int32_t encode2_impl(const void* w, int w_dtype, int64_t rows, int64_t cols, int
 
 // Decoder.  Bound by the write of the output.  A thread's step is the 16 bytes that one store writes (four fp32 or eight 16-bit weights,
 // one scale), neighbouring lanes take neighbouring ones, so every store of a warp fills whole sectors; with eight fp32 weights per thread
-// each store left half of its sectors to the next one (4001 x 3003: 13.2 -> 12.3 us, 28672 x 8192: 247 -> 201; four steps at a time per
-// thread were no faster for fp32 and cost the 16-bit types 30%).
+// each store left half of its sectors to the next one (28672 x 8192: 247 -> 201 us, fp16 127 -> 115; 4001 x 3003: 14.4 -> 12.4 with the
+// output in L2 and 14.8 -> 14.4 without, where a plain fill of the output takes 10.3; four steps at a time per thread were no faster
+// for fp32 and cost the 16-bit types 30%).
 template <typename T>
 __global__ void __launch_bounds__(256) decode2_kernel(const uint8_t* __restrict__ packed, const uint16_t* __restrict__ scales,
                                                        int64_t total, int per_scale, int shift, T* __restrict__ out) {

@@ -16,8 +16,7 @@ Same names, argument meaning and error behaviour as the reference module
 
 Differences, all deliberate: tensors must live on a CUDA device (the kernels are the only
 implementation; nothing falls back to CPU or to PyTorch ops), and no dense weight matrix is ever
-materialised in the forward pass (the 2.0- and 1.0-bit formats run one fused fp32 kernel instead of the
-tensor-core kernels; their backward decodes the weights).
+materialised in the forward pass or, for 16-bit gradients, in the backward pass.
 """
 
 from __future__ import annotations

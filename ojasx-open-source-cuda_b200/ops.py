@@ -57,8 +57,8 @@ def _result(r, what: str):
 
 def scratch(device: torch.device, nbytes: int, tag: str = "ws") -> torch.Tensor:
     """Grow-only scratch buffer per (device, stream, tag) - the counterpart of the reference's
-    ``_get_ephemeral_workspace`` (ojasx2/math/lattice.py:62-84), but only a few KB..MB of fp32
-    partial sums instead of a full decoded weight matrix."""
+    ``_get_ephemeral_workspace`` (ojasx2/math/lattice.py:62-84), but only a few KB..MB of scratch instead of a full
+    decoded weight matrix."""
     key = (device.index if device.index is not None else torch.cuda.current_device(),
            int(torch.cuda.current_stream(device).cuda_stream), tag)
     buf = _scratch.get(key)
@@ -277,10 +277,10 @@ def decode_2bit(packed: torch.Tensor, scales: torch.Tensor, shape: Tuple[int, in
 
 def linear_2bit(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor], n: int, k: int,
                 group_size: int, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``y = x . W^T (+ bias)`` from 2-bit codes: up to eight rows of x run the decode kernels (int8 tensor cores for
-    groups of 32 and K % 2048 == 0), more rows with 16-bit activations, groups of 8, 16 or 32 and K % 256 == 0 the tcgen05
-    prefill kernel (weights rounded to fp16 once, as ``decode_2bit(..., torch.float16)`` gives them), anything else
-    a scalar fp32 kernel."""
+    """``y = x . W^T (+ bias)`` from 2-bit codes, routed by the library (``csrc/linear_host.cuh``).  16-bit activations, groups of
+    8, 16 or 32 and K % 32 == 0 run on tensor cores: up to sixteen rows with exact weights, more rows on the tcgen05 kernel
+    (K % 256 == 0: weights rounded to fp16 once, as ``decode_2bit(..., torch.float16)`` gives them; other K: exact).
+    Anything else runs an fp32 kernel."""
     return _linear(2, x.reshape(-1, k), packed, scales, bias, int(n), int(k), int(group_size), out_dtype)
 
 
@@ -299,8 +299,8 @@ def decode_1bit(packed: torch.Tensor, scales: torch.Tensor, shape: Tuple[int, in
 
 def linear_1bit(x: torch.Tensor, packed: torch.Tensor, scales: torch.Tensor, bias: Optional[torch.Tensor], n: int, k: int,
                 group_size: int, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """``y = x . W^T (+ bias)`` from root codes; routed as :func:`linear_2bit` (here the fp16 weights of the
-    prefill kernel are exact)."""
+    """``y = x . W^T (+ bias)`` from root codes; routed as :func:`linear_2bit` (here the fp16 weights are exact for every
+    batch)."""
     return _linear(1, x.reshape(-1, k), packed, scales, bias, int(n), int(k), int(group_size), out_dtype)
 
 
