@@ -100,7 +100,10 @@ int32_t gemv_grouped_impl(const ojx_e8t_gemv_problem* problems, int count, int t
     // gemv_mma_kernel starts each matrix anew (two of 14336 x 4096, one and sixteen rows: 19.9 and 39 us against 20.5 and 42.4,
     // eight of them 59.5 and 119 against 65 and 138).  One matrix, the dependent steps of a chain, is the other's: it fills a smaller
     // table and needs no reduce launch (1024 x 2560: 4.0 and 8.9 us against 4.8 and 12.7, 4096 x 14336: 15.4 against 15.8).
-    if (count > 1) {
+    // Its copies take 32-bit byte offsets, so a matrix of more than 4 GB of codes (a tile unit has at most 32 x 4096 weights, 24 KB) is
+    // the first one's.
+    constexpr int kOneMatrixTiles = (int)(((int64_t)1 << 32) / (32 * 4096 * 3 / 16));
+    if (count > 1 || total_tiles >= kOneMatrixTiles) {
         if (needs_reduce && peers.sync != nullptr) peers.mode |= 0x100;      // a reduce kernel follows and stores (and signals) in its place
         const int32_t st = dispatch_gemv(bf, problems, count, total_tiles, (int)M, y_dtype, peers, overlap, s);
         OJX_RETURN_IF(st != OJX_OK || !needs_reduce, st);

@@ -312,3 +312,17 @@ def test_a_full_launch_queue_does_not_stop_other_threads(P):
         worker.join()
         torch.cuda.synchronize()
         assert longest < 0.15, longest
+
+
+def test_one_matrix_of_more_than_4_gb(P):
+    """Rows whose codes lie beyond 4 GB: a weight of 256 rows over and over, so every 256 outputs are the same."""
+    n, k, m, dev = 256 * 5469, 16384, 2, torch.device(DEV)              # 4.3 GB of codes
+    if torch.cuda.mem_get_info(dev)[0] < 16 << 30:
+        pytest.skip("needs 16 GB")
+    pk, sc, x = _problem(P, 256, k, m, 140)
+    want = P.ops.linear(x, pk, sc, None, 256, k, 32)
+    y = torch.empty((m, n), dtype=torch.bfloat16, device=dev)
+    P.ops.GroupedGemv([(x, pk.repeat(n // 256), sc.repeat(n // 256), None, y)], [(n, k)])()
+    got = y.view(m, n // 256, 256)
+    assert bool((got == got[:, :1]).all())
+    assert float((got[:, 0].float() - want.float()).norm() / want.float().norm()) <= 4e-3
