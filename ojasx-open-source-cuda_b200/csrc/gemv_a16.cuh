@@ -101,9 +101,11 @@ __device__ __forceinline__ void a16_decode(uint32_t (&a)[4], uint32_t w0, uint32
     a[2] = prmt(pa, pb, sel.y); a[3] = prmt(pa, pb, sel.y >> 16);
 }
 
+// `probs` is not declared __restrict__ by measurement: with it the benchmark's sweep takes 4.063 instead of 4.034 ms, its launch over 64
+// matrices of 14336 x 4096 at four rows 0.527 instead of 0.514.
 template <int NB, bool kXF16, bool kI8 = false>
 __global__ void __launch_bounds__(kGemvThreads, 1)
-gemv_a16_kernel(const ojx_e8t_gemv_problem* __restrict__ probs, int count, int total_items, int M, int y_dtype, int overlap,
+gemv_a16_kernel(const ojx_e8t_gemv_problem* probs, int count, int total_items, int M, int y_dtype, int overlap,
                 const __grid_constant__ PeerMap peers) {
     static_assert(!kI8 || (NB == 1 && !kXF16), "the int8 path serves one bf16 activation row");
     using Cfg = A16Cfg<NB>;
